@@ -133,8 +133,7 @@ struct Counters {
   uint32_t big_used;      // large-cavity slots used
   uint32_t n_inserted;    // winners this round
   uint32_t huge_used;     // huge-cavity slots used
-  uint32_t btab_used;     // k_write's large edge tables handed out this round
-  uint32_t bface_used;    // boundary-face list entries this round
+  uint32_t nbigw;         // winners whose star a whole block writes
   uint32_t work[4];       // dynamic work cursors of k_bfs, k_shared, k_write (one spare)
   uint32_t sbc[kOrderBuckets + 1];  // starts per order bucket (the last: overflow region)
   uint32_t err;           // error flags
@@ -171,21 +170,35 @@ struct alignas(16) State {
   uint32_t last_starts, last_cand, last_inserted, last_alloc;
 };
 
-// One tet slot: its vertex ids (retired: {DEAD, forward}) and its links,
-// (neighbour << 2) | face, NONE on the super tetrahedron's hull -- one 32-byte
-// sector, so that a visit reads both with one memory transaction.
-struct __align__(32) Tet {
+// One tet slot, one 128-byte line: its vertex ids (retired: {DEAD, forward})
+// and links ((neighbour << 2) | face, NONE on the super tetrahedron's hull);
+// the round's words -- the cavity claim (64-bit key, smallest wins), the
+// neighbourhood pre-claim and the vote (score | ~point); the coordinates of its
+// vertices by axis; and, on faces that two cavities of a round share, the new
+// tets of its cavity's star.
+//
+// The cavity search and the walks are chains of dependent loads, so what they
+// pay for is round trips, not bytes: with the coordinates in the record a
+// visited tet costs one trip (claim, links and coordinates together) instead
+// of two (ids, then four points), and its words share one DRAM page and one
+// address translation.
+struct __align__(128) Tet {
   uint4 v;
   uint4 n;
-};
-// The per-round words of one tet slot, likewise one sector: the cavity claim
-// (64-bit key, smallest wins), the "tested outside" memo of the cavity search,
-// the neighbourhood pre-claim and the vote (score | ~point).
-struct __align__(32) Claim {
   unsigned long long cav;
-  unsigned long long ring;
   unsigned long long pre;
   unsigned long long vote;
+  unsigned long long pad;
+  float4 X, Y, Z;  // .x/.y/.z/.w: vertices 0..3
+  uint4 slot;
+};
+static_assert(sizeof(Tet) == 128, "one tet slot is one 128-byte line");
+
+// The last round (16 bits; the run stops before they repeat) in which a point's
+// completed cavity lost a tet to a better claim, its cavity was completed, and
+// it inserted.  Stamps need no clearing between rounds, and one load gives all.
+struct __align__(8) Stat {
+  uint16_t lost, done, ins, pad;
 };
 
 // Everything a kernel needs, passed by value.
@@ -206,32 +219,27 @@ struct Dev {
   uint8_t* bigflag;  // point needs the large-cavity path
   // tets
   Tet* T;
-  Claim* C;
-  uint4* nslot;
   uint32_t* bface;  // boundary faces of this round's winners, (tet << 2) | face, per winner contiguous
   uint32_t cap;
   uint32_t nv;  // vertices (range guard)
   // clouds
   uint32_t* centry;  // a live tet of each cloud
   // lists (act / freed above are the double-buffered ones)
-  uint32_t* cand;
-  uint32_t* cand_off;  // pool offset, or BIG flag | big slot
-  uint32_t* cand_len;
-  uint32_t* cand_base;
-  uint32_t* cand_nf;   // boundary faces of each winning candidate (k_shared)
-  uint8_t* st1;  // candidate owns its whole cavity
-  uint8_t* st2;  // ... and no shared face with a better winner is violated
-  uint32_t* bigcand;  // points taking the huge-cavity path this round
-  uint32_t* starts;   // vote winners expanding their cavity this round, in order-bucket regions
+  uint4* cand;         // completed cavities: point, cavity list (pool offset or big slot), tets, boundary faces
+  uint32_t* cand_bf;   // boundary-face list of each (pool offset, even)
+  uint4* cwin;         // winners (k_shared): first new slot, flags, contested faces of the first 32
+  Stat* stat;          // the last round in which each point ... (see Stat)
+  uint32_t* bigw;      // winners whose star a whole block writes
+  uint32_t* bigcand;   // points taking the huge-cavity path this round
+  uint2* starts;       // vote winners (point, tet) expanding their cavity this round, in order-bucket regions
   uint32_t start_rc;  // capacity of one order bucket's region
   uint32_t start_ovf; // offset of the overflow region
   uint32_t prefilter;
-  uint32_t* wscratch; // one BIG_CAP cavity queue per lane group of k_bfs
-  unsigned long long* etab_key;  // k_write's global edge tables, kEdgeSlotsG per warp
-  uint32_t* etab_val;            // two values per slot
+  uint32_t* wscratch; // kScratchWords per lane group of k_bfs: its cavity queue and boundary faces beyond shared memory
+  uint32_t wgroups;   // lane groups it was sized for
+  uint32_t* etab;     // k_write's edge tables in global memory, kEdgeWordsG words per warp
   uint32_t etab_warps;
-  unsigned long long* btab_key;  // kBigTables tables of kBigTableSlots for larger cavities
-  uint32_t* btab_val;
+  uint32_t* btab;     // kBigTables edge tables of kBigEdgeWords words for the largest stars
   uint32_t* pool;
   uint32_t pool_cap;
   uint32_t* big;
@@ -304,6 +312,44 @@ __device__ __forceinline__ void load_pt(const float4* pts, uint32_t v, double* o
   o[2] = q.z;
 }
 
+// Coordinates of vertex i of a record (w = 0), and replacing them.
+__device__ __forceinline__ float fcomp(const float4& v, int i) {
+  return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w));
+}
+__device__ __forceinline__ void set_fcomp(float4& v, int i, float x) {
+  if (i == 0) v.x = x;
+  else if (i == 1) v.y = x;
+  else if (i == 2) v.z = x;
+  else v.w = x;
+}
+
+struct Coords {
+  float4 X, Y, Z;
+};
+__device__ __forceinline__ float4 corner(const float4& X, const float4& Y, const float4& Z, int i) {
+  return make_float4(fcomp(X, i), fcomp(Y, i), fcomp(Z, i), 0.f);
+}
+
+// Loads issued as written (volatile asm is neither sunk into the branch that
+// uses the value nor merged with later loads), so that a visit issues its
+// loads of one record together.
+__device__ __forceinline__ uint4 ld_u4(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 ld_f4(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+// Claim words change during the kernel: read from L2.
+__device__ __forceinline__ ulonglong2 ld_cg_u64x2(const unsigned long long* p) {
+  ulonglong2 v;
+  asm volatile("ld.global.cg.v2.u64 {%0,%1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p));
+  return v;
+}
+
 // Bijective 32-bit mixer (murmur3 finaliser) -> distinct priorities per round.
 __device__ __forceinline__ uint32_t mix32(uint32_t h) {
   h ^= h >> 16;
@@ -323,6 +369,12 @@ __device__ __forceinline__ uint32_t mix32(uint32_t h) {
 // network gave it this round (1..1023).
 __device__ __forceinline__ unsigned long long make_key(const Dev& D, const RoundArgs& R, uint32_t p) {
   const unsigned long long prio = D.bigflag[p] == 2 ? 0u : (D.prio ? D.prio[p] : 1u);
+  return R.stamp | (prio << 32) | mix32(p ^ (R.round * 0x9E3779B9u));
+}
+
+// The key of a vote winner that is not on the huge path.
+__device__ __forceinline__ unsigned long long start_key(const Dev& D, const RoundArgs& R, uint32_t p) {
+  const unsigned long long prio = D.prio ? D.prio[p] : 1u;
   return R.stamp | (prio << 32) | mix32(p ^ (R.round * 0x9E3779B9u));
 }
 
@@ -416,6 +468,22 @@ __device__ __noinline__ int o4d_sos_call(float4 a, float4 b, float4 c, float4 d,
   return o4d_sos_f(a, b, c, d, e, va, vb, vc, vd, ve, sos, err);
 }
 
+// Insphere test of p (coordinates pq) against tet T, whose coordinates were
+// loaded with the record; its vertex ids are read only when the FP32 stage
+// cannot decide.
+__device__ __forceinline__ int in_sphere(const Dev& D, const Tet* T, const float4& X, const float4& Y,
+                                         const float4& Z, const float4& pq, uint32_t p) {
+  const int s = ex::insphere_f32(corner(X, Y, Z, 0), corner(X, Y, Z, 1), corner(X, Y, Z, 2), corner(X, Y, Z, 3), pq);
+  if (s != 0) return s;
+  const uint4 V = ld_u4(&T->v);
+  if (V.x >= D.nv || V.y >= D.nv || V.z >= D.nv || V.w >= D.nv) {
+    atomicOr(&D.ctr->err, kErrGuard);
+    return 1;
+  }
+  return o4d_sos_slow(corner(X, Y, Z, 0), corner(X, Y, Z, 1), corner(X, Y, Z, 2), corner(X, Y, Z, 3), pq, V.x, V.y,
+                      V.z, V.w, p, D.sos, &D.ctr->err);
+}
+
 // Visibility walk with exact orient3d + SoS from tet t to the tet containing p.
 __device__ __forceinline__ uint32_t walk_to(const Dev& D, uint32_t t, uint32_t p, const float4& pq, uint32_t& steps) {
   int entry = -1;
@@ -424,12 +492,13 @@ __device__ __forceinline__ uint32_t walk_to(const Dev& D, uint32_t t, uint32_t p
       atomicOr(&D.ctr->err, kErrGuard);
       return 0;
     }
-    const uint4 V = D.T[t].v;
+    const uint4 V = ld_u4(&D.T[t].v), N = ld_u4(&D.T[t].n);
+    const float4 X = ld_f4(&D.T[t].X), Y = ld_f4(&D.T[t].Y), Z = ld_f4(&D.T[t].Z);
     if (V.x >= D.nv || V.y >= D.nv || V.z >= D.nv || V.w >= D.nv) {
       atomicOr(&D.ctr->err, kErrGuard);
       return t;
     }
-    const float4 P0 = D.pts[V.x], P1 = D.pts[V.y], P2 = D.pts[V.z], P3 = D.pts[V.w];
+    const float4 P0 = corner(X, Y, Z, 0), P1 = corner(X, Y, Z, 1), P2 = corner(X, Y, Z, 2), P3 = corner(X, Y, Z, 3);
     int moved = -1;
     for (int i = 0; i < 4; ++i) {
       const int f = (i + int(s)) & 3;
@@ -445,7 +514,7 @@ __device__ __forceinline__ uint32_t walk_to(const Dev& D, uint32_t t, uint32_t p
       steps += s + 1;
       return t;
     }
-    const uint32_t n = comp(D.T[t].n, moved);
+    const uint32_t n = comp(N, moved);
     if (n == NONE) {
       atomicOr(&D.ctr->err, kErrWalk);
       return t;
@@ -628,12 +697,13 @@ __global__ void k_scatter_points(const uint64_t* off, const CloudInfo* ci, uint3
 
 // Unused tet slots: dead, no links; claims and pre-claims at the largest key
 // (any claim beats them), no vote.
-__global__ void k_init_slots(Tet* T, Claim* C, uint64_t from, uint64_t to) {
+__global__ void k_init_slots(Tet* T, uint64_t from, uint64_t to) {
   for (uint64_t i = from + uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < to;
        i += uint64_t(gridDim.x) * blockDim.x) {
     T[i].v = make_uint4(DEAD, DEAD, DEAD, DEAD);
     T[i].n = make_uint4(NONE, NONE, NONE, NONE);
-    C[i] = Claim{~0ull, ~0ull, ~0ull, 0ull};
+    T[i].cav = T[i].pre = ~0ull;
+    T[i].vote = 0ull;
   }
 }
 
@@ -658,6 +728,12 @@ __global__ void k_init_clouds(const CloudInfo* ci, uint32_t nc, Dev D) {
   int o = o3d_sos(P[0], P[1], P[2], P[3], s0, s0 + 1, s0 + 2, s0 + 3, D.sos, &D.ctr->err);
   D.T[c].v = (o > 0) ? make_uint4(s0, s0 + 1, s0 + 2, s0 + 3) : make_uint4(s0 + 1, s0, s0 + 2, s0 + 3);
   D.T[c].n = make_uint4(NONE, NONE, NONE, NONE);
+  float4 q[4];
+  const uint4 V0 = D.T[c].v;
+  for (int k = 0; k < 4; ++k) q[k] = D.pts[comp(V0, k)];
+  D.T[c].X = make_float4(q[0].x, q[1].x, q[2].x, q[3].x);
+  D.T[c].Y = make_float4(q[0].y, q[1].y, q[2].y, q[3].y);
+  D.T[c].Z = make_float4(q[0].z, q[1].z, q[2].z, q[3].z);
   D.centry[c] = c;
 }
 
@@ -666,8 +742,9 @@ __global__ void k_init_clouds(const CloudInfo* ci, uint32_t nc, Dev D) {
 // Vote score: larger = inserted first.  Circumcenter rule: depth of p inside
 // the circumsphere (f32 insphere, src/shaders/vote.wgsl:401-494 semantics);
 // centroid rule: inverse squared distance to the centroid.
-__device__ __forceinline__ float vote_score(const float4* pts, uint4 V, float4 q, int rule) {
-  float4 a = pts[V.x], b = pts[V.y], c = pts[V.z], d = pts[V.w];
+__device__ __forceinline__ float vote_score(const Tet& t, float4 q, int rule) {
+  const float4 X = t.X, Y = t.Y, Z = t.Z;
+  const float4 a = corner(X, Y, Z, 0), b = corner(X, Y, Z, 1), c = corner(X, Y, Z, 2), d = corner(X, Y, Z, 3);
   if (rule == 1) {
     float cx = 0.25f * (a.x + b.x + c.x + d.x) - q.x;
     float cy = 0.25f * (a.y + b.y + c.y + d.y) - q.y;
@@ -700,13 +777,8 @@ __device__ __forceinline__ void cast_vote(const Dev& D, uint32_t p, uint32_t t) 
     atomicOr(&D.ctr->err, kErrGuard);
     return;
   }
-  const uint4 V = D.T[t].v;
-  if (V.x >= D.nv || V.y >= D.nv || V.z >= D.nv || V.w >= D.nv) {
-    atomicOr(&D.ctr->err, kErrGuard);
-    return;
-  }
-  const float sc = vote_score(D.pts, V, D.pts[p], D.rule);
-  atomicMax(&D.C[t].vote, ((unsigned long long)__float_as_uint(sc) << 32) | (unsigned long long)(~p));
+  const float sc = vote_score(D.T[t], D.pts[p], D.rule);
+  atomicMax(&D.T[t].vote, ((unsigned long long)__float_as_uint(sc) << 32) | (unsigned long long)(~p));
 }
 
 // Locates the points of one stratum: walk from the tet of the point one
@@ -774,7 +846,7 @@ __device__ __forceinline__ void load_start_prefix(const Dev& D, uint32_t* sp) {
 }
 
 // Start i of the round in bucket order.
-__device__ __forceinline__ uint32_t start_at(const Dev& D, const uint32_t* sp, uint32_t i) {
+__device__ __forceinline__ uint2 start_at(const Dev& D, const uint32_t* sp, uint32_t i) {
   uint32_t b = 0;
 #pragma unroll
   for (uint32_t k = 1; k <= kOrderBuckets; ++k) b += i >= sp[k] ? 1u : 0u;
@@ -800,36 +872,15 @@ __device__ __forceinline__ bool this_round(const RoundArgs& R, unsigned long lon
 }
 
 // Pre-claims of vote winner p in tet t with its key: t and its face
-// neighbours, and with `two` also the other neighbours of those (up to 17
-// tets).  A candidate whose pre-claimed tets are not all its own would lose its
-// cavity to a better one, so it skips cavity growth (k_bfs checks them).
-__device__ __forceinline__ void pre_claim(const Dev& D, uint32_t t, unsigned long long key, bool two) {
-  atomicMin(&D.C[t].pre, key);
+// neighbours.  A candidate whose pre-claimed tets are not all its own would
+// lose its cavity to a better one, so it skips cavity growth (k_bfs checks them).
+__device__ __forceinline__ void pre_claim(const Dev& D, uint32_t t, unsigned long long key) {
+  atomicMin(&D.T[t].pre, key);
   const uint4 N = D.T[t].n;
   for (int f = 0; f < 4; ++f) {
     const uint32_t nb = comp(N, f);
-    if (nb == NONE || (nb >> 2) >= D.cap) continue;
-    atomicMin(&D.C[nb >> 2].pre, key);
-    if (!two) continue;
-    const uint4 N2 = D.T[nb >> 2].n;
-    for (int g = 1; g < 4; ++g) {  // the three faces other than the one back to t
-      const uint32_t nb2 = comp(N2, (int(nb & 3) + g) & 3);
-      if (nb2 != NONE && (nb2 >> 2) < D.cap) atomicMin(&D.C[nb2 >> 2].pre, key);
-    }
+    if (nb != NONE && (nb >> 2) < D.cap) atomicMin(&D.T[nb >> 2].pre, key);
   }
-}
-
-// Tet k of p's pre-claim set (k = 0: t; k = 1 + 4i: face neighbour i;
-// k = 1 + 4i + j, j = 1..3: the j-th other neighbour of face neighbour i), or
-// NONE.
-__device__ __forceinline__ uint32_t pre_claim_tet(const Dev& D, uint32_t t, uint32_t k) {
-  if (k == 0) return t;
-  const uint32_t i = (k - 1) / 4, j = (k - 1) % 4;
-  const uint32_t nb = comp(D.T[t].n, int(i));
-  if (nb == NONE || (nb >> 2) >= D.cap) return NONE;
-  if (j == 0) return nb >> 2;
-  const uint32_t nb2 = comp(D.T[nb >> 2].n, (int(nb & 3) + int(j)) & 3);
-  return (nb2 == NONE || (nb2 >> 2) >= D.cap) ? NONE : nb2 >> 2;
 }
 
 // Features of vote winner p in its tet t (vote = the tet's vote word): the
@@ -840,21 +891,21 @@ __device__ __forceinline__ uint32_t pre_claim_tet(const Dev& D, uint32_t t, uint
 // scale.  k_cands has already counted this win in losses[p].
 __device__ __forceinline__ void winner_features(const Dev& D, const RoundArgs& R, uint32_t p, uint32_t t,
                                                 unsigned long long vote, float* f) {
-  const uint4 V = D.T[t].v;
+  const float4 X = D.T[t].X, Y = D.T[t].Y, Z = D.T[t].Z;
   const uint4 N = D.T[t].n;
   uint32_t r1 = 0, r2 = 0;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const uint32_t nb = comp(N, i);
     if (nb == NONE || (nb >> 2) >= D.cap) continue;
-    const unsigned long long nv = __ldcg(&D.C[nb >> 2].vote);
+    const unsigned long long nv = __ldcg(&D.T[nb >> 2].vote);
     if (nv != 0ull) ++r1;
     if ((nv >> 32) > (vote >> 32)) ++r2;  // a rival with a larger vote score
   }
   const uint32_t lost = D.losses[p] ? D.losses[p] - 1u : 0u;
   const uint32_t stratum = __ldcg(&D.st->stratum_size);
-  mlp::features(D.pts[V.x], D.pts[V.y], D.pts[V.z], D.pts[V.w], D.pts[p], __uint_as_float(uint32_t(vote >> 32)),
-                r1, r2, R.round, lost, R.n_active, stratum, f);
+  mlp::features(corner(X, Y, Z, 0), corner(X, Y, Z, 1), corner(X, Y, Z, 2), corner(X, Y, Z, 3), D.pts[p],
+                __uint_as_float(uint32_t(vote >> 32)), r1, r2, R.round, lost, R.n_active, stratum, f);
 }
 
 // Scheduler log (training data), after k_cands: in the rounds the learned
@@ -868,7 +919,7 @@ __global__ void k_log_features(Dev D) {
   load_start_prefix(D, sp);
   const uint32_t nstart = sp[kOrderBuckets + 1];
   for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < nstart; s += gridDim.x * blockDim.x) {
-    const uint32_t p = start_at(D, sp, s);
+    const uint32_t p = start_at(D, sp, s).x;
     D.log_pslot[p] = NONE;
     if ((mix32(p ^ (R.round * 0x27D4EB2Fu)) & ((1u << D.log_shift) - 1u)) != 0u) continue;
     const uint32_t slot = atomicAdd(&D.st->log_used, 1u);
@@ -877,7 +928,7 @@ __global__ void k_log_features(Dev D) {
     D.log_y[slot] = 0;
     const uint32_t t = D.loc[p];
     float f[mlp::kIn];
-    winner_features(D, R, p, t, __ldcg(&D.C[t].vote), f);
+    winner_features(D, R, p, t, __ldcg(&D.T[t].vote), f);
 #pragma unroll
     for (int k = 0; k < mlp::kIn; ++k) D.log_x[size_t(slot) * mlp::kIn + k] = f[k];
   }
@@ -910,7 +961,7 @@ __device__ __forceinline__ void cands_body(const Dev& D, const RoundArgs& R, Can
       p = R.active[i];
       const uint8_t tier = D.bigflag[p];
       t = D.loc[p];
-      if (!(tier & kDup) && t < D.cap) vote = D.C[t].vote;
+      if (!(tier & kDup) && t < D.cap) vote = D.T[t].vote;
       if (!(tier & kDup) && t < D.cap && uint32_t(vote) == ~p) {
         if (D.losses && D.losses[p] < 255u) D.losses[p] += 1u;
         if (tier == 2) {
@@ -918,8 +969,6 @@ __device__ __forceinline__ void cands_body(const Dev& D, const RoundArgs& R, Can
           if (b < HUGE_SLOTS) D.bigcand[b] = p;
         } else if (!tier) {
           start = true;
-          D.st1[p] = 0;
-          D.st2[p] = 0;
         }
       }
     }
@@ -951,7 +1000,7 @@ __device__ __forceinline__ void cands_body(const Dev& D, const RoundArgs& R, Can
       if (start && D.prio) D.prio[p] = 1;
       b = start ? (mix32(p ^ (R.round * 0x9E3779B9u)) >> 28) : 0u;
     }
-    if (start && D.prefilter) pre_claim(D, t, make_key(D, R, p), false);
+    if (start && D.prefilter) pre_claim(D, t, start_key(D, R, p));
     warp_append(&D.ctr->big_used, start);  // total count
     const unsigned grp = __match_any_sync(0xFFFFFFFFu, start ? b : 0xFFFFFFFFu);
     const uint32_t leader = uint32_t(__ffs(grp) - 1);
@@ -961,9 +1010,9 @@ __device__ __forceinline__ void cands_body(const Dev& D, const RoundArgs& R, Can
     if (start) {
       const uint32_t slot = base + uint32_t(__popc(grp & ((1u << lane) - 1u)));
       if (slot < D.start_rc) {
-        D.starts[b * D.start_rc + slot] = p;
+        D.starts[b * D.start_rc + slot] = make_uint2(p, t);
       } else {  // a bucket beyond its region (never expected): the overflow region
-        D.starts[D.start_ovf + atomicAdd(&D.ctr->sbc[kOrderBuckets], 1u)] = p;
+        D.starts[D.start_ovf + atomicAdd(&D.ctr->sbc[kOrderBuckets], 1u)] = make_uint2(p, t);
       }
     }
   }
@@ -985,258 +1034,92 @@ __global__ void __launch_bounds__(256) k_cands_learned(Dev D) {
   cands_body<true>(D, R, &sm);
 }
 
-// Cavity growth by groups of kBfsLanes lanes, kWarpGroups candidates per
-// warp: a group tests kBfsLanes (queued tet, face) pairs per pass, so a small
-// cavity costs one dependent load chain (tet -> neighbour -> claim ->
-// vertices -> coordinates -> insphere -> claim) per pass, and a warp keeps
-// several such chains in flight.  The queue starts in shared memory and
-// continues in the group's global region; cavities beyond BIG_CAP move to the
-// huge path next round.
+// Cavity growth by groups of kBfsLanes lanes, kWarpGroups at a time per warp:
+// a group tests kBfsLanes (queued tet, face) pairs per pass, so a pass costs
+// one dependent chain (record -> insphere -> claim), and a warp keeps several
+// such chains in flight.  A warp takes up to 32 starts per fetch: each lane
+// checks one start's pre-claims (the four neighbours' words in one trip for
+// the whole warp), the survivors -- about half of them -- are handed to the
+// lane groups one by one, and a group that finishes takes the next survivor
+// without waiting for the other group.  Every (cavity tet, face) pair is
+// tested exactly once, so the search also writes the list of boundary faces
+// that the later passes work from, and a claim that displaces another one of
+// the same round marks its owner as lost: a completed cavity that nobody
+// marked holds the minimum claim on all its tets.  The queue and the list
+// start in shared memory and continue in the group's global region; cavities
+// beyond BIG_CAP tets move to the huge path next round.
 #ifndef WTET_BFS_LANES
 #define WTET_BFS_LANES 16
 #endif
 constexpr uint32_t kBfsLanes = WTET_BFS_LANES;
 constexpr uint32_t kWarpGroups = 32 / kBfsLanes;
-constexpr uint32_t kBfsShared = 4 * kBfsLanes;  // queue entries (tet + neighbour words) per group in shared memory
+constexpr uint32_t kBfsShared = 48;  // queue entries (tet + neighbour words) per group in shared memory
+constexpr uint32_t kBfsFaces = 48;   // boundary faces per group in shared memory
+// A cavity of K tets joined through at least K - 1 faces has at most 2K + 2 boundary faces.
+constexpr uint32_t kMaxFaces = 2 * BIG_CAP + 2;
+constexpr uint32_t kScratchWords = BIG_CAP + 2 * kMaxFaces;
+constexpr uint32_t kPoolChunk = 512;  // pool words a lane group reserves at a time
 
-// Loads issued as written (volatile asm is neither sunk into the branch that
-// uses the value nor merged with later loads), so that a pass of the cavity
-// search issues its claim, memo, vertex and neighbour loads together.
-__device__ __forceinline__ uint4 ld_nc_u4(const uint4* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p));
-  return v;
-}
-__device__ __forceinline__ unsigned long long ld_cg_u64(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.global.cg.u64 %0, [%1];" : "=l"(v) : "l"(p));
-  return v;
-}
-
-__global__ void __launch_bounds__(128, WTET_BFS_MINB) k_bfs(Dev D) {
-  const RoundArgs R = load_round(D);
-  if (!R.live) return;
-  constexpr uint32_t FULL = 0xFFFFFFFFu, GM = (kBfsLanes == 32) ? 0xFFFFFFFFu : ((1u << kBfsLanes) - 1u);
-  // queue of each lane group: cavity tets and their four neighbour words
-  __shared__ uint32_t sq_all[4 * kWarpGroups][kBfsShared];
-  __shared__ uint4 sn_all[4 * kWarpGroups][kBfsShared];
-  const uint32_t lane = threadIdx.x & 31, gl = lane % kBfsLanes, shift = lane - gl;
-  const uint32_t lt = (1u << gl) - 1u;
-  const uint32_t gid = (blockIdx.x * blockDim.x + threadIdx.x) / kBfsLanes;  // global group index
-  uint32_t* sq = sq_all[threadIdx.x / kBfsLanes];
-  uint4* sn = sn_all[threadIdx.x / kBfsLanes];
-  uint32_t* cav = D.wscratch + size_t(gid) * BIG_CAP;
-  __shared__ uint32_t sp[kOrderBuckets + 2];
-  __shared__ unsigned long long block_searches;
-  if (threadIdx.x == 0) block_searches = 0;
-  load_start_prefix(D, sp);
-  const uint32_t nstart = sp[kOrderBuckets + 1];
-  unsigned long long searches = 0;
-  // Work is taken dynamically, one start per lane group (kWarpGroups per
-  // warp) per fetch: cavities differ in size by orders of magnitude, and a
-  // static grid-stride split leaves warps idle behind the slowest ones.
-  const uint32_t bchunk = kWarpGroups;
-  for (uint32_t chunk0 = warp_next(&D.ctr->work[0], bchunk); chunk0 < nstart;
-       chunk0 = warp_next(&D.ctr->work[0], bchunk))
-  for (uint32_t base = chunk0; base < min(chunk0 + bchunk, nstart); base += kWarpGroups) {
-    const uint32_t si = base + lane / kBfsLanes;
-    bool active = si < nstart;
-    uint32_t p = 0, t0 = 0;
-    if (active) {
-      p = start_at(D, sp, si);
-      t0 = D.loc[p];
-    }
-    unsigned long long key = 0;
-    float4 pq = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (active) {
-      key = make_key(D, R, p);
-      pq = D.pts[p];
-    }
-    int pre_lost = 0;
-    if (active && D.prefilter) {
-      // the winner's own pre-claims (t0 and its face neighbours) must all hold
-      for (uint32_t k = gl; k < 5; k += kBfsLanes) {
-        const uint32_t t = pre_claim_tet(D, t0, k == 0 ? 0u : 4u * (k - 1u) + 1u);
-        if (t != NONE && __ldcg(&D.C[t].pre) != key) pre_lost = 1;
-      }
-    }
-    // warp collectives first, outside any short-circuit: every lane must reach them
-    const uint32_t g_pre = (__ballot_sync(FULL, pre_lost) >> shift) & GM;
-    const bool searched = active && !g_pre;
-    int claim_lost = 0;
-    if (searched && gl == 0) {
-      const unsigned long long old = atomicMin(&D.C[t0].cav, key);
-      claim_lost = old < key;
-      sq[0] = t0;
-      sn[0] = D.T[t0].n;
-    }
-    const int g_claim = __shfl_sync(FULL, claim_lost, shift);
-    bool lost = !searched || g_claim;
-    uint32_t K = 1, head = 0;
-    bool overflow = false;
-    bool running = !lost;
-    __syncwarp();
-    while (__any_sync(FULL, running)) {
-      bool add = false, my_lost = false, my_guard = false;
-      uint32_t nt = 0;
-      uint4 nn = make_uint4(NONE, NONE, NONE, NONE);
-      const uint32_t idx = head + gl / 4u;
-      const uint32_t f = gl & 3u;
-      if (running && idx < K) {
-        // the neighbour word comes from the queue (loaded when the tet was
-        // added), or from global memory for entries beyond the shared part
-        const uint32_t nb = idx < kBfsShared ? comp(sn[idx], int(f))
-                                             : reinterpret_cast<const uint32_t*>(&D.T[cav[idx]].n)[f];
-        if (nb != NONE) {
-          nt = nb >> 2;
-          if (nt >= D.cap) {
-            my_guard = true;
-          } else {
-            // one round trip: claim, memo, vertices and neighbours together
-            const unsigned long long cc = ld_cg_u64(&D.C[nt].cav);
-            const unsigned long long cr = ld_cg_u64(&D.C[nt].ring);
-            const uint4 W = ld_nc_u4(&D.T[nt].v);
-            nn = ld_nc_u4(&D.T[nt].n);
-            if (cc != key && cr != key) {
-              if (W.x >= D.nv || W.y >= D.nv || W.z >= D.nv || W.w >= D.nv) {
-                my_guard = true;
-              } else {
-                const int sg = o4d_sos_f(D.pts[W.x], D.pts[W.y], D.pts[W.z], D.pts[W.w], pq, W.x, W.y, W.z, W.w, p,
-                                         D.sos, &D.ctr->err);
-                if (sg < 0) {
-                  const unsigned long long old = atomicMin(&D.C[nt].cav, key);
-                  if (old < key) my_lost = true;
-                  else if (old != key) add = true;
-                } else {
-                  D.C[nt].ring = key;  // memo for this candidate only
-                }
-              }
-            }
-          }
-        }
-      }
-      const uint32_t gball = (__ballot_sync(FULL, add) >> shift) & GM;
-      const uint32_t pos = K + __popc(gball & lt);
-      bool my_over = false;
-      if (add) {
-        if (pos < kBfsShared) {
-          sq[pos] = nt;
-          sn[pos] = nn;
-        } else if (pos < BIG_CAP) {
-          cav[pos] = nt;
-        } else {
-          my_over = true;
-        }
-      }
-      const bool g_guard = (__ballot_sync(FULL, my_guard) >> shift) & GM;
-      const bool g_lost = (__ballot_sync(FULL, my_lost) >> shift) & GM;
-      const bool g_over = (__ballot_sync(FULL, my_over) >> shift) & GM;
-      if (running) {
-        if (g_guard) {
-          if (gl == 0) atomicOr(&D.ctr->err, kErrGuard);
-          lost = true;
-        }
-        lost = lost || g_lost;
-        overflow = overflow || g_over;
-        head = min(head + kBfsLanes / 4u, K);
-        K += __popc(gball);
-        running = !lost && !overflow && head < K;
-      }
-      __syncwarp();
-    }
-    if (searched && gl == 0) ++searches;
-    // Partial claims carry this round's key: the huge path takes it next round.
-    if (searched && overflow && gl == 0) D.bigflag[p] = kPending | 2;
-    bool ok = searched && !lost && !overflow;
-    // One reservation for the warp's completed cavities (pool entries and
-    // candidate slots are shared counters of the whole grid).
-    const uint32_t kk = ok ? K : 0u;
-    uint32_t tot = 0, n_ok = 0, my_off = 0, my_ci = 0;  // each group follows the earlier groups' entries
-#pragma unroll
-    for (uint32_t g = 0; g < kWarpGroups; ++g) {
-      const uint32_t kg = __shfl_sync(FULL, kk, int(g * kBfsLanes));
-      if (g * kBfsLanes == shift) {
-        my_off = tot;
-        my_ci = n_ok;
-      }
-      tot += kg;
-      n_ok += kg ? 1u : 0u;
-    }
-    uint32_t off = 0, ci = 0;
-    if (lane == 0 && n_ok) {
-      off = atomicAdd(&D.ctr->pool_used, tot);
-      ci = atomicAdd(&D.ctr->n_cand, n_ok);
-    }
-    off = __shfl_sync(FULL, off, 0) + my_off;
-    ci = __shfl_sync(FULL, ci, 0) + my_ci;
-    ok = ok && off + K <= D.pool_cap;  // pool full: retry next round
-    if (ok) {
-      for (uint32_t k = gl; k < K; k += kBfsLanes) D.pool[off + k] = k < kBfsShared ? sq[k] : cav[k];
-      if (gl == 0) {
-        D.cand[ci] = p;
-        D.cand_off[ci] = off;
-        D.cand_len[ci] = K;
-      }
-    } else if (kk && gl == 0) {
-      // a reserved candidate slot whose cavity did not fit the pool: it holds
-      // no cavity, and k_resolve rejects it
-      D.cand[ci] = p;
-      D.cand_off[ci] = 0;
-      D.cand_len[ci] = 0;
-    }
-    __syncwarp();
-  }
-  // per-block statistics, one atomic per block
-  if (searches) atomicAdd(&block_searches, searches);
-  __syncthreads();
-  if (threadIdx.x == 0 && block_searches) atomicAdd(&D.ctr->n_expanded, block_searches);
-}
+template <uint32_t kWarps>
+struct BfsSmem {
+  uint4 n[kWarps * kWarpGroups][kBfsShared];
+  uint2 b[kWarps * kWarpGroups][kBfsFaces];
+  uint32_t q[kWarps * kWarpGroups][kBfsShared];
+  uint32_t sp[kOrderBuckets + 2];
+  uint32_t huge[6];
+  unsigned long long searches;
+};
 
 // Global cavity slot bi of the huge path (HUGE_CAP tets each).
 __device__ __forceinline__ uint32_t* big_slot(const Dev& D, uint32_t bi) {
   return D.big + size_t(bi) * HUGE_CAP;
 }
-
 __device__ __forceinline__ const uint32_t* cand_cavity(const Dev& D, uint32_t off) {
   return (off & 0x80000000u) ? big_slot(D, off & 0x7FFFFFFFu) : D.pool + off;
 }
 
+// Claims tet t for `key`; true when a better claim holds it.  A displaced
+// owner of this round is marked: it has lost a tet of its cavity.
+__device__ __forceinline__ bool claim(const Dev& D, const RoundArgs& R, uint32_t t, unsigned long long key,
+                                      unsigned long long& old) {
+  old = atomicMin(&D.T[t].cav, key);
+  if (old > key && this_round(R, old)) {
+    const uint32_t q = key_owner(R, old);
+    if (q < D.nv) D.stat[q].lost = uint16_t(R.round);
+  }
+  return old < key;
+}
 
 // Huge cavities: one block per candidate; each pass tests blockDim/4 queued
-// tets x 4 faces, appending to the slot's list through a shared counter.
-__global__ void __launch_bounds__(256) k_expand_big(Dev D) {
-  const RoundArgs R = load_round(D);
-  if (!R.live) return;
-  const uint32_t nhuge = min(__ldcg(&D.ctr->huge_used), HUGE_SLOTS);
-  const uint32_t bi = blockIdx.x;
-  if (bi >= nhuge) return;  // block-uniform
-  __shared__ uint32_t sK, sNew, sHead, sLost, sOver, sGuard;
+// tets x 4 faces, appending to the slot's list through a shared counter.  The
+// boundary faces are listed in two more passes over the finished cavity
+// (count, reserve, write).  h: six shared words.
+__device__ __forceinline__ void expand_big(const Dev& D, const RoundArgs& R, uint32_t bi, uint32_t* h) {
+  enum { kK, kNew, kHead, kBad, kF, kOff };  // kBad: 1 lost, 2 list overflow, 4 range guard
   const uint32_t tid = threadIdx.x;
   const uint32_t p = D.bigcand[bi];
   const uint32_t t0 = D.loc[p];
   uint32_t* cav = big_slot(D, bi);
   const unsigned long long key = make_key(D, R, p);
   const float4 pq = D.pts[p];
+  __syncthreads();
   if (tid == 0) {
-    D.st1[p] = 0;
-    D.st2[p] = 0;
-    const unsigned long long old = t0 < D.cap ? atomicMin(&D.C[t0].cav, key) : 0ull;
-    sLost = old < key ? 1u : 0u;
-    sOver = 0u;
-    sGuard = t0 < D.cap ? 0u : 1u;
+    unsigned long long old = 0;
+    h[kBad] = 0u;
+    if (t0 >= D.cap) h[kBad] = 4u;
+    else if (claim(D, R, t0, key, old)) h[kBad] = 1u;
     cav[0] = t0;
-    sK = 1u;
-    sNew = 1u;
-    sHead = 0u;
+    h[kK] = 1u;
+    h[kNew] = 1u;
+    h[kHead] = 0u;
+    h[kF] = 0u;
   }
   __syncthreads();
   for (;;) {
-    const uint32_t K = sK, head = sHead;
-    const bool stop = sLost || sOver || sGuard || head >= K;
+    const uint32_t K = h[kK], head = h[kHead];
+    const bool stop = h[kBad] || head >= K;
     __syncthreads();  // every thread has read the pass state
-    if (stop) break;   // block-uniform
+    if (stop) break;  // block-uniform
     const uint32_t idx = head + tid / 4u, f = tid & 3u;
     if (idx < K) {
       const uint32_t c = cav[idx];
@@ -1244,25 +1127,17 @@ __global__ void __launch_bounds__(256) k_expand_big(Dev D) {
       if (nb != NONE) {
         const uint32_t nt = nb >> 2;
         if (nt >= D.cap) {
-          sGuard = 1u;
-        } else if (__ldcg(&D.C[nt].cav) != key && __ldcg(&D.C[nt].ring) != key) {
-          const uint4 W = D.T[nt].v;
-          if (W.x >= D.nv || W.y >= D.nv || W.z >= D.nv || W.w >= D.nv) {
-            sGuard = 1u;
-          } else {
-            const int sg = o4d_sos_f(D.pts[W.x], D.pts[W.y], D.pts[W.z], D.pts[W.w], pq, W.x, W.y, W.z, W.w, p,
-                                     D.sos, &D.ctr->err);
-            if (sg < 0) {
-              const unsigned long long old = atomicMin(&D.C[nt].cav, key);
-              if (old < key) {
-                sLost = 1u;
-              } else if (old != key) {
-                const uint32_t pos = atomicAdd(&sNew, 1u);
-                if (pos < HUGE_CAP) cav[pos] = nt;
-                else sOver = 1u;
-              }
-            } else {
-              D.C[nt].ring = key;
+          atomicOr(&h[kBad], 4u);
+        } else if (__ldcg(&D.T[nt].cav) != key) {
+          const Tet* T = D.T + nt;
+          if (in_sphere(D, T, ld_f4(&T->X), ld_f4(&T->Y), ld_f4(&T->Z), pq, p) < 0) {
+            unsigned long long old = 0;
+            if (claim(D, R, nt, key, old)) {
+              atomicOr(&h[kBad], 1u);
+            } else if (old != key) {
+              const uint32_t pos = atomicAdd(&h[kNew], 1u);
+              if (pos < HUGE_CAP) cav[pos] = nt;
+              else atomicOr(&h[kBad], 2u);
             }
           }
         }
@@ -1270,50 +1145,284 @@ __global__ void __launch_bounds__(256) k_expand_big(Dev D) {
     }
     __syncthreads();
     if (tid == 0) {
-      sHead = min(head + blockDim.x / 4u, K);
-      sK = min(sNew, HUGE_CAP);
+      h[kHead] = min(head + blockDim.x / 4u, K);
+      h[kK] = min(h[kNew], HUGE_CAP);
     }
     __syncthreads();
   }
-  if (tid == 0) {
-    atomicAdd(&D.ctr->n_big, 1ull);
-    if (sGuard) atomicOr(&D.ctr->err, kErrGuard);
-    if (sOver) atomicOr(&D.ctr->err, kErrBig);
-    if (!sLost && !sOver && !sGuard) {
-      const uint32_t ci = atomicAdd(&D.ctr->n_cand, 1u);
-      D.cand[ci] = p;
-      D.cand_off[ci] = 0x80000000u | bi;
-      D.cand_len[ci] = sK;
+  const uint32_t K = h[kK];
+  if (h[kBad] == 0u) {
+    // A claim displaced meanwhile only means that p has lost (it is marked).
+    for (uint32_t pass = 0; pass < 2; ++pass) {
+      const uint32_t F = h[kF], off = h[kOff];
+      __syncthreads();
+      if (pass == 1 && tid == 0) h[kNew] = 0u;
+      __syncthreads();
+      if (pass == 1 && off + 2u * F > D.pool_cap) break;  // pool full: retry next round (block-uniform)
+      for (uint32_t e = tid; e < 4 * K; e += blockDim.x) {
+        const uint32_t c = cav[e >> 2];
+        const uint32_t nb = reinterpret_cast<const uint32_t*>(&D.T[c].n)[e & 3u];
+        if (nb != NONE && __ldcg(&D.T[nb >> 2].cav) == key) continue;
+        if (pass == 0) {
+          atomicAdd(&h[kF], 1u);
+        } else {
+          const uint32_t pos = atomicAdd(&h[kNew], 1u);
+          if (pos < F)
+            reinterpret_cast<uint2*>(D.pool + off)[pos] = make_uint2((c << 2) | (e & 3u), nb);
+        }
+      }
+      __syncthreads();
+      if (pass == 0 && tid == 0) h[kOff] = atomicAdd(&D.ctr->pool_used, 2u * h[kF]);
+      __syncthreads();
     }
   }
+  if (tid == 0) {
+    atomicAdd(&D.ctr->n_big, 1ull);
+    if (h[kBad] & 4u) atomicOr(&D.ctr->err, kErrGuard);
+    if (h[kBad] & 2u) atomicOr(&D.ctr->err, kErrBig);
+    if (h[kBad] == 0u && h[kOff] + 2u * h[kF] <= D.pool_cap && h[kNew] == h[kF]) {
+      const uint32_t ci = atomicAdd(&D.ctr->n_cand, 1u);
+      D.cand[ci] = make_uint4(p, 0x80000000u | bi, K, h[kF]);
+      D.cand_bf[ci] = h[kOff];
+      D.stat[p].done = uint16_t(R.round);
+    }
+  }
+  __syncthreads();
 }
 
-// A candidate wins its cavity when it holds the minimum claim on every tet.
-__global__ void k_resolve(Dev D) {
+template <uint32_t kWarps>
+__device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSmem<kWarps>& sm) {
+  constexpr uint32_t FULL = 0xFFFFFFFFu, GM = (kBfsLanes == 32) ? 0xFFFFFFFFu : ((1u << kBfsLanes) - 1u);
+  // one block per huge candidate, before the block's share of the starts
+  const uint32_t nhuge = min(__ldcg(&D.ctr->huge_used), HUGE_SLOTS);
+  for (uint32_t bi = blockIdx.x; bi < nhuge; bi += gridDim.x) expand_big(D, R, bi, sm.huge);
+  const uint32_t lane = threadIdx.x & 31, gl = lane % kBfsLanes, shift = lane - gl;
+  const uint32_t lt = (1u << gl) - 1u;
+  const uint32_t warp = threadIdx.x >> 5;
+  const uint32_t gid = (blockIdx.x * blockDim.x + threadIdx.x) / kBfsLanes;  // global group index
+  uint32_t* sq = sm.q[threadIdx.x / kBfsLanes];
+  uint4* sn = sm.n[threadIdx.x / kBfsLanes];
+  uint2* sb = sm.b[threadIdx.x / kBfsLanes];
+  uint32_t* gq = D.wscratch + size_t(gid < D.wgroups ? gid : 0) * kScratchWords;
+  uint2* gb = reinterpret_cast<uint2*>(gq + BIG_CAP);
+  if (threadIdx.x == 0) sm.searches = 0;
+  load_start_prefix(D, sm.sp);
+  const uint32_t nstart = sm.sp[kOrderBuckets + 1];
+  const uint32_t nwarps = gridDim.x * kWarps;
+  // About four fetches per warp, between one start per lane group and one per lane.
+  const uint32_t chunk = min(32u, max(kWarpGroups, nstart / (4u * nwarps)));
+  // Same-address atomics serialise, so in large rounds a group reserves several
+  // cavities' worth of pool at a time (small ones would run out of pool).
+  const uint32_t pool_chunk = chunk == 32u ? kPoolChunk : 0u;
+  unsigned long long searches = 0;
+  uint32_t pool_at = 0, pool_end = 0;  // the group's reserved pool words
+  const uint32_t lgrp = lane / kBfsLanes;
+  for (uint32_t base = (blockIdx.x * kWarps + warp) * chunk; base < nstart;
+       base = nwarps * chunk + warp_next(&D.ctr->work[0], chunk)) {
+    // ---- one start per lane: its pre-claims (its tet and the four face neighbours) must all hold
+    const uint32_t si = base + lane;
+    bool ok = lane < chunk && si < nstart;
+    uint32_t p_l = 0, t_l = 0;
+    unsigned long long key_l = 0;
+    float4 pq_l = make_float4(0.f, 0.f, 0.f, 0.f);
+    uint4 n_l = make_uint4(NONE, NONE, NONE, NONE);
+    if (ok) {
+      const uint2 st = start_at(D, sm.sp, si);
+      p_l = st.x;
+      t_l = st.y;
+      n_l = ld_u4(&D.T[t_l].n);
+      const unsigned long long own = __ldcg(&D.T[t_l].pre);
+      pq_l = ld_f4(&D.pts[p_l]);
+      key_l = start_key(D, R, p_l);
+      if (D.prefilter) {
+        const uint32_t i0 = n_l.x >> 2, i1 = n_l.y >> 2, i2 = n_l.z >> 2, i3 = n_l.w >> 2;
+        const unsigned long long a0 = i0 < D.cap ? __ldcg(&D.T[i0].pre) : key_l;
+        const unsigned long long a1 = i1 < D.cap ? __ldcg(&D.T[i1].pre) : key_l;
+        const unsigned long long a2 = i2 < D.cap ? __ldcg(&D.T[i2].pre) : key_l;
+        const unsigned long long a3 = i3 < D.cap ? __ldcg(&D.T[i3].pre) : key_l;
+        ok = own == key_l && a0 == key_l && a1 == key_l && a2 == key_l && a3 == key_l;
+      }
+    }
+    uint32_t todo = __ballot_sync(FULL, ok);  // survivors not yet handed out
+    if (ok) ++searches;
+    // finished cavities of this lane's start
+    uint32_t rec_off = 0, rec_k = 0, rec_f = 0, rec_bf = 0;
+    // ---- the groups' searches
+    uint32_t cur = 0;  // the lane whose start this group works on
+    bool running = false, lost = false, overflow = false;
+    uint32_t p = 0, K = 0, F = 0, head = 0;
+    unsigned long long key = 0;
+    float4 pq = pq_l;
+    for (;;) {
+      const uint32_t busy = __ballot_sync(FULL, running);
+      bool fresh = false;
+      if (todo && busy != FULL) {
+        // idle groups take the next survivors, in order
+#pragma unroll
+        for (uint32_t g = 0; g < kWarpGroups; ++g) {
+          if (((busy >> (g * kBfsLanes)) & 1u) == 0u && todo) {
+            const uint32_t j = uint32_t(__ffs(int(todo))) - 1u;
+            todo &= todo - 1u;
+            if (lgrp == g) {
+              cur = j;
+              fresh = true;
+            }
+          }
+        }
+        const uint32_t p_s = __shfl_sync(FULL, p_l, int(cur)), t_s = __shfl_sync(FULL, t_l, int(cur));
+        const unsigned long long k_s = __shfl_sync(FULL, key_l, int(cur));
+        const float x_s = __shfl_sync(FULL, pq_l.x, int(cur)), y_s = __shfl_sync(FULL, pq_l.y, int(cur)),
+                    z_s = __shfl_sync(FULL, pq_l.z, int(cur));
+        const uint32_t n0 = __shfl_sync(FULL, n_l.x, int(cur)), n1 = __shfl_sync(FULL, n_l.y, int(cur)),
+                       n2 = __shfl_sync(FULL, n_l.z, int(cur)), n3 = __shfl_sync(FULL, n_l.w, int(cur));
+        if (fresh) {
+          p = p_s;
+          key = k_s;
+          pq = make_float4(x_s, y_s, z_s, 0.f);
+          K = 1;
+          F = 0;
+          head = 0;
+          lost = overflow = false;
+          running = true;
+          if (gl == 0) {
+            sq[0] = t_s;
+            sn[0] = make_uint4(n0, n1, n2, n3);
+          }
+        }
+        __syncwarp();
+      } else if (!busy) {
+        break;  // nothing left to hand out
+      }
+      // ---- one pass: kBfsLanes (queued tet, face) pairs of each group
+      bool add = false, bnd = false, my_lost = false, my_guard = false;
+      uint32_t nt = 0, code = 0, outer = NONE;
+      uint4 nn = make_uint4(NONE, NONE, NONE, NONE);
+      unsigned long long old0 = ~0ull;
+      if (fresh && gl == 0) my_lost = claim(D, R, sq[0], key, old0);
+      const uint32_t idx = head + gl / 4u;
+      const uint32_t f = gl & 3u;
+      if (running && idx < K) {
+        const uint32_t c = idx < kBfsShared ? sq[idx] : gq[idx];
+        outer = idx < kBfsShared ? comp(sn[idx], int(f)) : reinterpret_cast<const uint32_t*>(&D.T[c].n)[f];
+        code = (c << 2) | f;
+        nt = outer >> 2;
+        if (outer == NONE) {
+          bnd = true;
+        } else if (nt >= D.cap) {
+          my_guard = true;
+        } else {
+          // one round trip: claim, neighbours and coordinates together
+          const Tet* T = D.T + nt;
+          const unsigned long long cc = __ldcg(&T->cav);
+          nn = ld_u4(&T->n);
+          const float4 X = ld_f4(&T->X), Y = ld_f4(&T->Y), Z = ld_f4(&T->Z);
+          if (cc != key) {
+            if (in_sphere(D, T, X, Y, Z, pq, p) < 0) {
+              unsigned long long old;
+              if (claim(D, R, nt, key, old)) my_lost = true;
+              else add = old != key;
+            } else {
+              bnd = true;
+            }
+          }
+        }
+      }
+      const uint32_t aball = (__ballot_sync(FULL, add) >> shift) & GM;
+      const uint32_t bball = (__ballot_sync(FULL, bnd) >> shift) & GM;
+      const uint32_t pos = K + __popc(aball & lt), posb = F + __popc(bball & lt);
+      bool my_over = false;
+      if (add) {
+        if (pos < kBfsShared) {
+          sq[pos] = nt;
+          sn[pos] = nn;
+        } else if (pos < BIG_CAP) {
+          gq[pos] = nt;
+        } else {
+          my_over = true;
+        }
+      }
+      if (bnd) {
+        if (posb < kBfsFaces) sb[posb] = make_uint2(code, outer);
+        else if (posb < kMaxFaces) gb[posb] = make_uint2(code, outer);
+        else my_over = true;
+      }
+      const uint32_t g_guard = (__ballot_sync(FULL, my_guard) >> shift) & GM;
+      const uint32_t g_lost = (__ballot_sync(FULL, my_lost) >> shift) & GM;
+      const uint32_t g_over = (__ballot_sync(FULL, my_over) >> shift) & GM;
+      bool fin = false;
+      if (running) {
+        if (g_guard && gl == 0) atomicOr(&D.ctr->err, kErrGuard);
+        lost = lost || g_lost || g_guard;
+        overflow = overflow || g_over;
+        head = min(head + kBfsLanes / 4u, K);
+        K += __popc(aball);
+        F += __popc(bball);
+        running = !lost && !overflow && head < K;
+        fin = !running;
+      }
+      __syncwarp();
+      if (!__any_sync(FULL, fin)) continue;
+      // ---- finished searches: the cavity and its boundary go to the pool
+      // Partial claims carry this round's key: the huge path takes it next round.
+      if (fin && !lost && overflow && gl == 0) D.bigflag[p] = kPending | 2;
+      bool keep = fin && !lost && !overflow;
+      if (keep) {
+        const uint32_t need = ((K + 1u) & ~1u) + 2u * F;
+        if (pool_at + need > pool_end) {
+          const uint32_t want = max(need, pool_chunk);  // even
+          uint32_t got = 0;
+          if (gl == 0) got = atomicAdd(&D.ctr->pool_used, want);
+          got = __shfl_sync(GM << shift, got, int(shift));
+          pool_at = got;
+          pool_end = got + want;
+        }
+        keep = pool_at + need <= D.pool_cap && pool_at + need > pool_at;  // pool full: retry next round
+        if (keep) {
+          for (uint32_t k = gl; k < K; k += kBfsLanes) D.pool[pool_at + k] = k < kBfsShared ? sq[k] : gq[k];
+          uint2* pb = reinterpret_cast<uint2*>(D.pool + pool_at + ((K + 1u) & ~1u));
+          for (uint32_t k = gl; k < F; k += kBfsLanes) pb[k] = k < kBfsFaces ? sb[k] : gb[k];
+        }
+      }
+#pragma unroll
+      for (uint32_t g = 0; g < kWarpGroups; ++g) {
+        const int src = int(g * kBfsLanes);
+        const uint32_t kg = __shfl_sync(FULL, keep ? K : 0u, src);
+        const uint32_t fg = __shfl_sync(FULL, F, src), og = __shfl_sync(FULL, pool_at, src);
+        const uint32_t cg = __shfl_sync(FULL, cur, src);
+        if (kg && lane == cg) {
+          rec_k = kg;
+          rec_f = fg;
+          rec_off = og;
+          rec_bf = og + ((kg + 1u) & ~1u);
+        }
+      }
+      if (keep) pool_at += ((K + 1u) & ~1u) + 2u * F;
+      __syncwarp();
+    }
+    // ---- one reservation for the batch's completed cavities
+    const uint32_t ci = warp_append(&D.ctr->n_cand, rec_k != 0u);
+    if (rec_k) {
+      D.cand[ci] = make_uint4(p_l, rec_off, rec_k, rec_f);
+      D.cand_bf[ci] = rec_bf;
+      D.stat[p_l].done = uint16_t(R.round);
+    }
+    __syncwarp();
+  }
+  // per-block statistics, one atomic per block
+  if (searches) atomicAdd(&sm.searches, searches);
+  __syncthreads();
+  if (threadIdx.x == 0 && sm.searches) atomicAdd(&D.ctr->n_expanded, sm.searches);
+}
+
+__global__ void __launch_bounds__(128, WTET_BFS_MINB) k_bfs(Dev D) {
   const RoundArgs R = load_round(D);
   if (!R.live) return;
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t ncand = __ldcg(&D.ctr->n_cand);
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t ci = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; ci < ncand; ci += nwarps) {
-    uint32_t p = D.cand[ci];
-    uint32_t K = D.cand_len[ci];
-    const uint32_t* cav = cand_cavity(D, D.cand_off[ci]);
-    unsigned long long key = make_key(D, R, p);
-    bool ok = K > 0;  // a slot whose cavity did not fit the pool holds none
-    for (uint32_t i = lane; i < K; i += 32)
-      if (__ldcg(&D.C[cav[i]].cav) != key) ok = false;
-    bool win = __all_sync(0xFFFFFFFFu, ok);
-    if (lane == 0) D.st1[p] = win ? 1 : 0;
-  }
+  __shared__ BfsSmem<4> sm;
+  bfs_body<4>(D, R, sm);
 }
 
 __device__ __forceinline__ uint32_t slot_of(const Dev& D, const RoundArgs& R, uint32_t v) {
   return v < R.n_freed_prev ? R.freed_prev[v] : R.tet_top + (v - R.n_freed_prev);
-}
-
-__device__ __forceinline__ bool boundary_face(const Dev& D, uint32_t nb, unsigned long long key) {
-  return nb == NONE || __ldcg(&D.C[nb >> 2].cav) != key;
 }
 
 // The edge of face f of tet V opposite corner k (k != f): its two vertex ids,
@@ -1333,407 +1442,579 @@ __device__ __forceinline__ uint32_t edge_hi(const uint4& V, int f, int k) {
 // Delaunay: the better winner q must lie outside the circumsphere of the
 // worse winner p's new tet on f (then either insertion order gives the same
 // tets).  The worse one of a violating pair steps back.  A winner that stays
-// is handed one slot per boundary face (recycled slots first, then fresh
-// ones) in the same pass over its cavity.
-__global__ void __launch_bounds__(128, WTET_SHARED_MINB) k_shared(Dev D) {
-  const RoundArgs R = load_round(D);
-  if (!R.live) return;
+// is handed its slots in the same pass.  One lane per boundary face of the
+// list that the search wrote; the loads of up to kChunk winners are issued
+// together (records, then faces, then the outer tets' claims), because each
+// of them is one random trip.  cwin: first new slot (virtual), flags, the
+// faces of the first 32 that another cavity of this round touches.
+constexpr uint32_t kWinInPlace = 1u;  // the star takes the cavity's own slots
+constexpr uint32_t kWinBlock = 2u;    // a whole block writes the star
+constexpr uint32_t kBigWinners = 4096;
+constexpr uint32_t kBlockFaces = 340;  // larger stars are written by a whole block
+
+template <uint32_t kWarps>
+__device__ __forceinline__ void shared_body(const Dev& D, const RoundArgs& R) {
   constexpr uint32_t FULL = 0xFFFFFFFFu;
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t ncand = __ldcg(&D.ctr->n_cand);
   const uint32_t ch = chunk_for(ncand);
-  for (uint32_t c0 = warp_next(&D.ctr->work[1], ch); c0 < ncand; c0 = warp_next(&D.ctr->work[1], ch)) {
-    // Phase 1, per winner of the chunk: the shared-face test and the count of
-    // boundary faces.  Phase 2: one allocation for the whole chunk (the slot
-    // and list counters are shared by every warp of the grid).  Phase 3: the
-    // slots of each winner's boundary faces.
-    uint32_t need_fresh[kChunk], need_total[kChunk], bmask[kChunk];
-    bool keep[kChunk], inpl[kChunk];
+  const uint32_t nwarps = gridDim.x * kWarps;
+  const uint16_t stamp = uint16_t(R.round);
+  for (uint32_t c0 = (blockIdx.x * kWarps + (threadIdx.x >> 5)) * ch; c0 < ncand;
+       c0 = nwarps * ch + warp_next(&D.ctr->work[1], ch)) {
+    // the chunk's records, one per lane; a cavity that lost a tet is out
+    uint4 rec_l = make_uint4(0, 0, 0, 0);
+    uint32_t bf_l = 0;
+    unsigned long long key_l = 0;
+    bool alive = false;
+    if (lane < ch && c0 + lane < ncand) {
+      rec_l = ld_u4(&D.cand[c0 + lane]);
+      bf_l = D.cand_bf[c0 + lane];
+      key_l = make_key(D, R, rec_l.x);
+      alive = D.stat[rec_l.x].lost != stamp;
+    }
+    const uint32_t live = __ballot_sync(FULL, alive);
+    if (!live) continue;
+    // faces, then the claims of the tets beyond them (first 32 of each winner)
+    uint2 e[kChunk];
+    unsigned long long key[kChunk], cc[kChunk];
+    uint32_t F[kChunk];
 #pragma unroll
     for (uint32_t j = 0; j < kChunk; ++j) {
-      const uint32_t ci = c0 + j;
-      keep[j] = false;
-      inpl[j] = false;
-      need_fresh[j] = need_total[j] = bmask[j] = 0;
-      if (j >= ch || ci >= ncand) continue;
-      const uint32_t p = D.cand[ci];
-      if (!D.st1[p]) {
-        if (lane == 0) D.st2[p] = 0;
-        continue;
+      F[j] = (live >> j) & 1u ? __shfl_sync(FULL, rec_l.w, int(j)) : 0u;
+      key[j] = __shfl_sync(FULL, key_l, int(j));
+      const uint32_t bfo = __shfl_sync(FULL, bf_l, int(j));
+      e[j] = make_uint2(0u, NONE);
+      if (lane < F[j]) e[j] = reinterpret_cast<const uint2*>(D.pool + bfo)[lane];
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < kChunk; ++j) cc[j] = e[j].y != NONE ? __ldcg(&D.T[e[j].y >> 2].cav) : ~0ull;
+    uint32_t touch[kChunk], base[kChunk], fresh[kChunk];
+    uint32_t sum = 0;
+    bool keep_l = false;  // this lane's winner stays
+#pragma unroll
+    for (uint32_t j = 0; j < kChunk; ++j) {
+      const uint32_t p = __shfl_sync(FULL, rec_l.x, int(j)), K = __shfl_sync(FULL, rec_l.z, int(j));
+      const uint32_t off = __shfl_sync(FULL, rec_l.y, int(j)), bfo = __shfl_sync(FULL, bf_l, int(j));
+      bool bad = false, mine = false;
+      for (uint32_t i = lane; i < F[j]; i += 32) {
+        const uint2 ej = i < 32 ? e[j] : reinterpret_cast<const uint2*>(D.pool + bfo)[i];
+        const unsigned long long cj = i < 32 ? cc[j] : ej.y != NONE ? __ldcg(&D.T[ej.y >> 2].cav) : ~0ull;
+        if (!this_round(R, cj) || cj == key[j]) continue;
+        if (i < 32) mine = true;
+        if (cj > key[j] || bad) continue;
+        const uint32_t q = key_owner(R, cj);
+        if (q >= D.nv) continue;
+        const Stat sq = D.stat[q];
+        if (sq.done != stamp || sq.lost == stamp) continue;
+        // the new tet on the face: p replaces the opposite vertex
+        const uint32_t c = ej.x >> 2;
+        const int f = int(ej.x & 3u);
+        uint4 V = D.T[c].v;
+        float4 X = D.T[c].X, Y = D.T[c].Y, Z = D.T[c].Z;
+        const float4 pq = D.pts[p];
+        set_comp(V, f, p);
+        set_fcomp(X, f, pq.x);
+        set_fcomp(Y, f, pq.y);
+        set_fcomp(Z, f, pq.z);
+        if (o4d_sos_call(corner(X, Y, Z, 0), corner(X, Y, Z, 1), corner(X, Y, Z, 2), corner(X, Y, Z, 3), D.pts[q], V.x,
+                         V.y, V.z, V.w, q, D.sos, &D.ctr->err) < 0)
+          bad = true;
       }
-      const uint32_t K = D.cand_len[ci];
-      const uint32_t* cav = cand_cavity(D, D.cand_off[ci]);
-      const unsigned long long key = make_key(D, R, p);
-      // one lane per (cavity tet, face): boundary faces are counted (their
-      // flags kept in a register for cavities of up to 64 tets), faces shared
-      // with a better winner are tested
-      bool bad = false;
-      uint32_t total = 0, bm = 0;
-      for (uint32_t e0 = 0; e0 < 4 * K; e0 += 32) {
-        const uint32_t e = e0 + lane;
-        bool bnd = false;
-        if (e < 4 * K) {
-          const uint32_t c = cav[e >> 2];
-          const int f = int(e & 3u);
-          const uint32_t nb = reinterpret_cast<const uint32_t*>(&D.T[c].n)[f];
-          const unsigned long long cc = nb == NONE ? 0ull : __ldcg(&D.C[nb >> 2].cav);
-          bnd = nb == NONE || cc != key;
-          if (bnd && nb != NONE && !bad && cc < key && this_round(R, cc)) {
-            const uint32_t q = key_owner(R, cc);
-            if (q < D.nv && D.st1[q]) {
-              // the new tet on face f: p replaces vertex f
-              const uint4 V = D.T[c].v;
-              const uint32_t w0 = f == 0 ? p : V.x, w1 = f == 1 ? p : V.y, w2 = f == 2 ? p : V.z,
-                             w3 = f == 3 ? p : V.w;
-              if (o4d_sos_call(D.pts[w0], D.pts[w1], D.pts[w2], D.pts[w3], D.pts[q], w0, w1, w2, w3, q, D.sos,
-                            &D.ctr->err) < 0)
-                bad = true;
-            }
-          }
-        }
-        const uint32_t ball = __ballot_sync(FULL, bnd);
-        total += __popc(ball);
-        if (e0 < 256 && bnd) bm |= 1u << (e0 >> 5);
-      }
-      if (__any_sync(FULL, bad)) {
-        if (lane == 0) D.st2[p] = 0;
-        continue;
-      }
+      bad = __any_sync(FULL, bad);
+      touch[j] = __ballot_sync(FULL, mine);
+      if (bad) F[j] = 0;
       // A small star goes into the cavity's own slots (boundary face r < K
       // takes the slot of cavity tet r), plus fresh slots for the faces
       // beyond K: tets that are neighbours in space stay neighbours in memory.
       // Larger stars take recycled / fresh slots for every face.
-      inpl[j] = total <= kInPlaceFaces && !(D.cand_off[ci] & 0x80000000u);
-      keep[j] = true;
-      need_total[j] = total;
-      need_fresh[j] = total - (inpl[j] ? min(K, total) : 0u);
-      bmask[j] = bm;
+      const bool inpl = F[j] <= kInPlaceFaces && !(off & 0x80000000u);
+      fresh[j] = F[j] - (inpl ? min(K, F[j]) : 0u);
+      base[j] = sum;
+      sum += fresh[j];
+      if (lane == j && F[j]) keep_l = true;
     }
-    uint32_t sum_fresh = 0, sum_total = 0;
+    // one reservation for the chunk (the counter is shared by the whole grid)
+    uint32_t b0 = 0;
+    if (lane == 0 && sum) b0 = atomicAdd(&D.ctr->alloc_used, sum);
+    b0 = __shfl_sync(FULL, b0, 0);
+    uint32_t flags_l = 0, base_l = 0, touch_l = 0;
 #pragma unroll
     for (uint32_t j = 0; j < kChunk; ++j) {
-      sum_fresh += need_fresh[j];
-      sum_total += need_total[j];
-    }
-    if (sum_total == 0) continue;  // warp-uniform
-    uint32_t base = 0, bfo = 0;
-    if (lane == 0) {
-      base = atomicAdd(&D.ctr->alloc_used, sum_fresh);
-      bfo = atomicAdd(&D.ctr->bface_used, sum_total);
-    }
-    base = __shfl_sync(FULL, base, 0);
-    bfo = __shfl_sync(FULL, bfo, 0);
-#pragma unroll
-    for (uint32_t j = 0; j < kChunk; ++j) {
-      const uint32_t mybase = base, mybfo = bfo;
-      base += need_fresh[j];
-      bfo += need_total[j];
-      if (!keep[j]) continue;
-      const uint32_t ci = c0 + j;
-      const uint32_t p = D.cand[ci];
-      const uint32_t K = D.cand_len[ci];
-      const uint32_t* cav = cand_cavity(D, D.cand_off[ci]);
-      const unsigned long long key = make_key(D, R, p);
-      const uint32_t total = need_total[j], fresh = need_fresh[j];
-      const uint32_t reuse = total - fresh;
-      const uint32_t last = mybase + fresh;
-      if ((last > R.n_freed_prev && R.tet_top + (last - R.n_freed_prev) > D.cap) || mybfo + total > D.cap) {
-        if (lane == 0) {
-          atomicOr(&D.ctr->err, kErrCapacity);
-          D.st2[p] = 0;
-        }
+      if (!F[j]) continue;  // warp-uniform
+      const uint32_t K = __shfl_sync(FULL, rec_l.z, int(j)), off = __shfl_sync(FULL, rec_l.y, int(j));
+      const uint32_t bfo = __shfl_sync(FULL, bf_l, int(j));
+      const uint32_t mybase = b0 + base[j], last = mybase + fresh[j];
+      if (last > R.n_freed_prev && R.tet_top + (last - R.n_freed_prev) > D.cap) {
+        if (lane == 0) atomicOr(&D.ctr->err, kErrCapacity);
+        if (lane == j) keep_l = false;
         continue;
       }
-      // slots in (tet, face) order; inner faces get NONE
-      uint32_t run = 0;
-      for (uint32_t e0 = 0; e0 < 4 * K; e0 += 32) {
-        const uint32_t e = e0 + lane;
-        bool bnd = false;
-        uint32_t c = 0;
-        int f = 0;
-        if (e < 4 * K) {
-          c = cav[e >> 2];
-          f = int(e & 3u);
-          if (4 * K <= 256) {
-            bnd = (bmask[j] >> (e0 >> 5)) & 1u;
-          } else {
-            const uint32_t nb = reinterpret_cast<const uint32_t*>(&D.T[c].n)[f];
-            bnd = boundary_face(D, nb, key);
+      const uint32_t* cav = cand_cavity(D, off);
+      const uint32_t reuse = F[j] - fresh[j];
+      // the new tets on faces that other cavities touch, for their links (of a
+      // larger star: on every face, for the rotation too)
+      if (F[j] <= kInPlaceFaces) {
+        if ((touch[j] >> lane) & 1u)
+          reinterpret_cast<uint32_t*>(&D.T[e[j].x >> 2].slot)[e[j].x & 3u] =
+              lane < reuse ? cav[lane] : slot_of(D, R, mybase + (lane - reuse));
+      } else {
+        for (uint32_t i = lane; i < F[j]; i += 32) {
+          const uint2 ej = reinterpret_cast<const uint2*>(D.pool + bfo)[i];
+          reinterpret_cast<uint32_t*>(&D.T[ej.x >> 2].slot)[ej.x & 3u] =
+              i < reuse ? cav[i] : slot_of(D, R, mybase + (i - reuse));
+        }
+      }
+      if (lane == j) {
+        base_l = mybase;
+        touch_l = touch[j];
+        flags_l = F[j] <= kInPlaceFaces && !(off & 0x80000000u) ? kWinInPlace : 0u;
+        if (F[j] > kBlockFaces) {
+          const uint32_t i = atomicAdd(&D.ctr->nbigw, 1u);
+          if (i < kBigWinners) {
+            D.bigw[i] = c0 + j;
+            flags_l |= kWinBlock;
           }
         }
-        const uint32_t ball = __ballot_sync(FULL, bnd);
-        const uint32_t r = run + __popc(ball & ((1u << lane) - 1u));  // rank of this boundary face
-        if (e < 4 * K)
-          reinterpret_cast<uint32_t*>(D.nslot + c)[f] =
-              !bnd ? NONE : (r < reuse ? cav[r] : slot_of(D, R, mybase + (r - reuse)));
-        if (bnd) D.bface[mybfo + r] = (c << 2) | uint32_t(f);
-        run += __popc(ball);
-      }
-      if (lane == 0) {
-        D.cand_base[ci] = mybfo;
-        D.cand_nf[ci] = total | (inpl[j] ? 0x80000000u : 0u);
-        D.st2[p] = 1;
       }
     }
+    if (keep_l) {
+      D.cwin[c0 + lane] = make_uint4(base_l, flags_l, touch_l, 0u);
+      D.stat[rec_l.x].ins = stamp;
+    }
+    __syncwarp();
   }
+}
+
+__global__ void __launch_bounds__(128, WTET_SHARED_MINB) k_shared(Dev D) {
+  const RoundArgs R = load_round(D);
+  if (!R.live) return;
+  shared_body<4>(D, R);
 }
 
 // Writes the new tets of every winner.  The three faces through p of a new
 // tet pair up across the boundary edges of the cavity (each boundary edge is
-// shared by exactly two new tets): the pairs are matched in an open-addressing
-// edge table of at least 3 slots per boundary face (load <= 1/2) -- in shared
-// memory for up to kEdgeFaces faces, in the warp's region of a global table
-// for up to kEdgeFacesG faces, in one of kBigTables large tables (taken per
-// round, first come) for up to kBigTableFaces -- and the rest rotate around
-// each edge inside the cavity.  A boundary face shared with another winner's cavity
-// links to that winner's new tet.
-constexpr uint32_t kEdgeSlots = 256;    // shared-memory slots per warp
-constexpr uint32_t kEdgeFaces = 80;
-constexpr uint32_t kEdgeSlotsG = 1024;  // global slots per warp
-constexpr uint32_t kEdgeFacesG = 340;
-constexpr uint32_t kBigTables = 16;         // large tables per round, taken first come
+// shared by exactly two new tets).  Every new tet publishes its three edges;
+// an open-addressing table of edge numbers brings the two ends of an edge
+// together: the first to come leaves its number, the second finds it and
+// writes both links, so each edge costs one compare-and-swap and no second
+// lookup.  The tables are in shared memory for up to kEdgeFaces faces and in
+// the warp's region of a global table for up to kEdgeFacesG; larger stars are
+// written by a whole block, with one of kBigTables large tables for up to
+// kBigTableFaces faces and rotation around each boundary edge beyond.  A
+// boundary face shared with another winner's cavity links to that winner's
+// new tet.
+constexpr uint32_t kEdgeFaces = 64;
+constexpr uint32_t kEdgeSlots = 256;     // table entries: at most 3/2 edges per face, load 3/8
+constexpr uint32_t kEdgeFacesG = kBlockFaces;
+constexpr uint32_t kEdgeSlotsG = 1024;   // load 1/2
+constexpr uint32_t kBigTables = 16;
 constexpr uint32_t kBigTableSlots = 1u << 14;
 constexpr uint32_t kBigTableFaces = kBigTableSlots / 3;
+// words of one table: slots, then per edge a 64-bit key, a value and a link
+constexpr uint32_t kEdgeWordsG = kEdgeSlotsG + 3 * kEdgeFacesG * 4;
+constexpr uint32_t kBigEdgeWords = kBigTableSlots + 3 * kBigTableFaces * 4;
+constexpr uint32_t kNoEdge = 0xFFFFFFFFu;
+
+struct EdgeTable {
+  uint32_t* tab;             // edge number or kNoEdge
+  unsigned long long* key;   // (larger vertex, smaller vertex)
+  uint32_t* val;             // (new tet << 2) | face: what the other end links to
+  uint32_t* link;            // what this end links to
+  uint32_t mask;
+};
+
+template <uint32_t kWarps>
+struct WriteSmem {
+  unsigned long long key[kWarps][3 * kEdgeFaces];
+  uint32_t val[kWarps][3 * kEdgeFaces], link[kWarps][3 * kEdgeFaces];
+  uint32_t tab[kWarps][kEdgeSlots];
+  uint32_t inserted, bad, s0, fbase;
+  unsigned long long created;
+};
 
 __device__ __forceinline__ uint32_t edge_hash(uint32_t a, uint32_t b, uint32_t mask) {
   return mix32(a * 0x9E3779B9u ^ b) & mask;
 }
 
-__global__ void __launch_bounds__(128, WTET_WRITE_MINB) k_write(Dev D) {
-  const RoundArgs R = load_round(D);
-  if (!R.live) return;
-  __shared__ unsigned long long ekey[4][kEdgeSlots];
-  __shared__ uint32_t ev0[4][kEdgeSlots], ev1[4][kEdgeSlots];
+// The threads that write one star together: a warp or a whole block.
+struct WarpTeam {
+  __device__ __forceinline__ uint32_t id() const { return threadIdx.x & 31u; }
+  __device__ __forceinline__ uint32_t size() const { return 32u; }
+  __device__ __forceinline__ void sync() const { __syncwarp(); }
+};
+struct BlockTeam {
+  __device__ __forceinline__ uint32_t id() const { return threadIdx.x; }
+  __device__ __forceinline__ uint32_t size() const { return blockDim.x; }
+  __device__ __forceinline__ void sync() const { __syncthreads(); }
+};
+
+// One new tet while its star is written.
+struct NewTet {
+  uint4 v, n;
+  Coords q;
+  uint32_t sl, outer;
+  bool shared;
+};
+
+// Slot of boundary face j of a winner.
+__device__ __forceinline__ uint32_t star_slot(const Dev& D, const RoundArgs& R, const uint32_t* cav, uint32_t reuse,
+                                              uint32_t base, uint32_t j) {
+  return j < reuse ? cav[j] : slot_of(D, R, base + (j - reuse));
+}
+
+// Publishes the edges of boundary face j (clears the table first: table()).
+template <class Team>
+__device__ __forceinline__ void table_clear(const Team& tm, const EdgeTable& E) {
+  for (uint32_t j = tm.id(); j <= E.mask; j += tm.size()) E.tab[j] = kNoEdge;
+}
+__device__ __forceinline__ void table_publish(const EdgeTable& E, uint32_t j, const uint4& V, int f, uint32_t sl) {
+  uint32_t e = 3 * j;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (k == f) continue;
+    E.key[e] = (static_cast<unsigned long long>(edge_lo(V, f, k)) << 32) | edge_hi(V, f, k);
+    E.val[e] = (sl << 2) | uint32_t(k);
+    E.link[e] = NONE;
+    ++e;
+  }
+}
+__device__ __forceinline__ void table_match(const EdgeTable& E, uint32_t j) {
+#pragma unroll
+  for (uint32_t i = 0; i < 3; ++i) {
+    const uint32_t e = 3 * j + i;
+    const unsigned long long k = E.key[e];
+    uint32_t h = edge_hash(uint32_t(k >> 32), uint32_t(k), E.mask);
+    for (uint32_t probe = 0; probe <= E.mask; ++probe) {
+      const uint32_t o = atomicCAS(&E.tab[h], kNoEdge, e);
+      if (o == kNoEdge) break;
+      if (E.key[o] == k) {
+        E.link[e] = E.val[o];
+        E.link[o] = E.val[e];
+        break;
+      }
+      h = (h + 1) & E.mask;
+    }
+  }
+}
+
+// The links of a new tet through p when its star has no table: rotation
+// around each boundary edge inside the cavity.
+__device__ __forceinline__ uint32_t rotate_link(const Dev& D, unsigned long long key, uint32_t c, int f, int k) {
+  uint32_t cur = c;
+  uint4 Vc = D.T[c].v;
+  int kc = k, ms = f;
+  for (int it = 0; it < ROT_LIMIT; ++it) {
+    const uint32_t nb = comp(D.T[cur].n, kc);
+    if (nb == NONE || __ldcg(&D.T[nb >> 2].cav) != key) return (comp(D.T[cur].slot, kc) << 2) | uint32_t(ms);
+    const uint32_t nt = nb >> 2;
+    if (nt >= D.cap) break;
+    const int entry = int(nb & 3);
+    const uint32_t x = comp(Vc, ms);
+    const uint4 Wt = D.T[nt].v;
+    int kx = -1;
+    for (int q = 0; q < 4; ++q)
+      if (comp(Wt, q) == x) kx = q;
+    if (kx < 0) break;
+    cur = nt;
+    Vc = Wt;
+    kc = kx;
+    ms = entry;
+  }
+  return NONE;
+}
+
+// Loads boundary face j of p's star: the cavity tet with the face's opposite
+// vertex replaced by p, linked to the outer tet (or to another winner's new
+// tet on a shared face).
+__device__ __forceinline__ void star_face(const Dev& D, const RoundArgs& R, uint2 e, uint32_t sl, bool contested,
+                                          uint32_t p, const float4& pq, NewTet& t, uint4& V) {
+  const uint32_t c = e.x >> 2;
+  const int f = int(e.x & 3u);
+  V = ld_u4(&D.T[c].v);
+  t.q.X = ld_f4(&D.T[c].X);
+  t.q.Y = ld_f4(&D.T[c].Y);
+  t.q.Z = ld_f4(&D.T[c].Z);
+  t.sl = sl;
+  t.outer = e.y;
+  t.shared = false;
+  uint32_t link_out = e.y;
+  if (contested && e.y != NONE) {
+    const uint32_t o = e.y >> 2;
+    const unsigned long long cc = __ldcg(&D.T[o].cav);
+    if (this_round(R, cc)) {
+      const uint32_t q = key_owner(R, cc);
+      if (q != p && q < D.nv && D.stat[q].ins == uint16_t(R.round)) {
+        t.shared = true;
+        link_out = (comp(D.T[o].slot, int(e.y & 3u)) << 2) | (e.y & 3u);
+      }
+    }
+  }
+  t.v = V;
+  set_comp(t.v, f, p);
+  set_fcomp(t.q.X, f, pq.x);
+  set_fcomp(t.q.Y, f, pq.y);
+  set_fcomp(t.q.Z, f, pq.z);
+  t.n = make_uint4(NONE, NONE, NONE, NONE);
+  set_comp(t.n, f, link_out);
+}
+
+// Writes one new tet and what points at it.
+__device__ __forceinline__ void star_commit(const Dev& D, const NewTet& t, int f) {
+  Tet* T = D.T + t.sl;
+  T->v = t.v;
+  T->n = t.n;
+  T->X = t.q.X;
+  T->Y = t.q.Y;
+  T->Z = t.q.Z;
+  T->vote = 0ull;  // the new tet's points vote in k_relocate
+  // Every vertex on the cavity boundary gets a live incident tet, so a
+  // vertex's hint tet is alive whenever it is read (strata activation).
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (k != f) D.vtet[comp(t.v, k)] = t.sl;
+  if (t.outer != NONE && !t.shared && (t.outer >> 2) < D.cap)
+    reinterpret_cast<uint32_t*>(&D.T[t.outer >> 2].n)[t.outer & 3u] = (t.sl << 2) | uint32_t(f);
+}
+
+// Writes the star of one winner whose faces do not fit one per lane, or by a
+// whole block.  `E.tab` null: links by rotation.  Returns whether every face
+// through p found its partner.
+template <class Team>
+__device__ __forceinline__ bool write_star(const Dev& D, const RoundArgs& R, const Team& tm, const uint4& rec,
+                                           const uint32_t* cav, const uint2* bf, uint32_t base, bool use_table,
+                                           const EdgeTable& E, unsigned long long key, const float4& pq) {
+  const uint32_t p = rec.x, F = rec.w;
+  bool bad = false;
+  if (use_table) {
+    table_clear(tm, E);
+    for (uint32_t j = tm.id(); j < F; j += tm.size()) {
+      const uint2 e = bf[j];
+      table_publish(E, j, ld_u4(&D.T[e.x >> 2].v), int(e.x & 3u), star_slot(D, R, cav, 0u, base, j));
+    }
+    tm.sync();
+    for (uint32_t j = tm.id(); j < F; j += tm.size()) table_match(E, j);
+    tm.sync();
+  }
+  for (uint32_t j = tm.id(); j < F; j += tm.size()) {
+    const uint2 e = bf[j];
+    const int f = int(e.x & 3u);
+    NewTet t;
+    uint4 V;
+    star_face(D, R, e, star_slot(D, R, cav, 0u, base, j), true, p, pq, t, V);
+    uint32_t i = 3 * j;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (k == f) continue;
+      const uint32_t link = use_table ? E.link[i] : rotate_link(D, key, e.x >> 2, f, k);
+      if (link == NONE) bad = true;
+      set_comp(t.n, k, link);
+      ++i;
+    }
+    star_commit(D, t, f);
+  }
+  return !bad;
+}
+
+// Retires the cavity tets from `reused` on (the star took the slots of the
+// earlier ones): they go to the recycled list at fbase, and forward the points
+// inside to a new tet on one of their own faces where they have one, else to s0.
+template <class Team>
+__device__ __forceinline__ void retire(const Dev& D, const RoundArgs& R, const Team& tm, const uint4& rec,
+                                       const uint32_t* cav, const uint2* bf, uint32_t reused, uint32_t base,
+                                       uint32_t s0, uint32_t fbase) {
+  for (uint32_t i = reused + tm.id(); i < rec.z; i += tm.size()) {
+    const uint32_t c = cav[i];
+    D.T[c].v = make_uint4(DEAD, s0, 0u, 0u);
+    R.freed_next[fbase + (i - reused)] = c;
+  }
+  tm.sync();
+  for (uint32_t j = tm.id(); j < rec.w; j += tm.size()) {
+    const uint32_t c = bf[j].x >> 2;
+    if (D.T[c].v.x == DEAD) D.T[c].v.y = star_slot(D, R, cav, reused, base, j);
+  }
+}
+
+// What one thread does for a point that has inserted.
+__device__ __forceinline__ void mark_inserted(const Dev& D, uint32_t p, uint32_t s0) {
+  if (D.log_pslot && D.log_pslot[p] != NONE) D.log_y[D.log_pslot[p]] = 1;  // scheduler log: inserted
+  D.vtet[p] = s0;
+  D.loc[p] |= INS_BIT;
+  D.centry[D.vcloud[p]] = s0;
+  D.bigflag[p] = 0;
+}
+
+template <uint32_t kWarps>
+__device__ __forceinline__ void write_body(const Dev& D, const RoundArgs& R, WriteSmem<kWarps>& sm) {
+  constexpr uint32_t FULL = 0xFFFFFFFFu;
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t w = threadIdx.x >> 5;
-  const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t gwarp = blockIdx.x * kWarps + w;
   const uint32_t ncand = __ldcg(&D.ctr->n_cand);
-  __shared__ uint32_t block_inserted;
-  __shared__ unsigned long long block_created;
   if (threadIdx.x == 0) {
-    block_inserted = 0;
-    block_created = 0;
+    sm.inserted = 0;
+    sm.created = 0;
   }
   __syncthreads();
+  // ---- the largest stars, one block each
+  const uint32_t nbig = min(__ldcg(&D.ctr->nbigw), kBigWinners);
+  const uint32_t big_blocks = min(gridDim.x, kBigTables);
+  for (uint32_t i = blockIdx.x; blockIdx.x < big_blocks && i < nbig; i += big_blocks) {
+    const BlockTeam tm;
+    const uint32_t ci = D.bigw[i];
+    const uint4 rec = D.cand[ci];
+    const uint4 win = D.cwin[ci];
+    const uint32_t* cav = cand_cavity(D, rec.y);
+    const uint2* bf = reinterpret_cast<const uint2*>(D.pool + D.cand_bf[ci]);
+    uint32_t* words = D.btab + size_t(blockIdx.x) * kBigEdgeWords;
+    EdgeTable E;
+    E.key = reinterpret_cast<unsigned long long*>(words);
+    E.val = words + 6 * kBigTableFaces;
+    E.link = E.val + 3 * kBigTableFaces;
+    E.tab = E.link + 3 * kBigTableFaces;
+    E.mask = 1023;
+    while (E.mask + 1 < 3 * rec.w) E.mask = 2 * E.mask + 1;
+    if (threadIdx.x == 0) sm.bad = 0;
+    __syncthreads();
+    if (!write_star(D, R, tm, rec, cav, bf, win.x, rec.w <= kBigTableFaces, E, make_key(D, R, rec.x), D.pts[rec.x]))
+      sm.bad = 1;
+    if (threadIdx.x == 0) sm.fbase = atomicAdd(&D.ctr->n_freed_next, rec.z);
+    __syncthreads();  // every thread is done reading the cavity before it is retired
+    const uint32_t s0 = star_slot(D, R, cav, 0u, win.x, 0u);
+    retire(D, R, tm, rec, cav, bf, 0u, win.x, s0, sm.fbase);
+    if (threadIdx.x == 0) {
+      if (sm.bad) atomicOr(&D.ctr->err, kErrRotate);
+      mark_inserted(D, rec.x, s0);
+      sm.inserted += 1;
+      sm.created += rec.w;
+    }
+    __syncthreads();
+  }
+  // ---- one warp per star
+  const WarpTeam tm;
   uint32_t inserted = 0;
   unsigned long long created = 0;
   const uint32_t ch = chunk_for(ncand);
-  for (uint32_t c0 = warp_next(&D.ctr->work[2], ch); c0 < ncand; c0 = warp_next(&D.ctr->work[2], ch))
-  for (uint32_t ci = c0; ci < min(c0 + ch, ncand); ++ci) {
-    uint32_t p = D.cand[ci];
-    if (!D.st2[p]) continue;
-    uint32_t K = D.cand_len[ci];
-    const uint32_t* cav = cand_cavity(D, D.cand_off[ci]);
-    unsigned long long key = make_key(D, R, p);
-    const uint32_t nfw = D.cand_nf[ci];
-    const uint32_t F = nfw & 0x7FFFFFFFu;    // boundary faces, counted by k_shared
-    const bool inplace = (nfw >> 31) != 0u;  // the star takes the cavity's own slots
-    const uint32_t bfo = D.cand_base[ci];    // first entry of its boundary-face list
-    unsigned long long* tk = nullptr;
-    uint32_t *t0 = nullptr, *t1 = nullptr;
-    uint32_t mask = 31;
-    while (mask + 1 < 3 * F) mask = 2 * mask + 1;
-    if (F <= kEdgeFaces) {
-      tk = ekey[w];
-      t0 = ev0[w];
-      t1 = ev1[w];
-    } else if (F <= kEdgeFacesG && gwarp < D.etab_warps) {
-      tk = D.etab_key + size_t(gwarp) * kEdgeSlotsG;
-      t0 = D.etab_val + size_t(gwarp) * 2 * kEdgeSlotsG;
-      t1 = t0 + kEdgeSlotsG;
-    } else if (F <= kBigTableFaces) {
-      uint32_t bt = 0;
-      if (lane == 0) bt = atomicAdd(&D.ctr->btab_used, 1u);
-      bt = __shfl_sync(0xFFFFFFFFu, bt, 0);
-      if (bt < kBigTables) {
-        tk = D.btab_key + size_t(bt) * kBigTableSlots;
-        t0 = D.btab_val + size_t(bt) * 2 * kBigTableSlots;
-        t1 = t0 + kBigTableSlots;
-      }
+  const uint32_t nwarps = gridDim.x * kWarps;
+  for (uint32_t c0 = gwarp * ch; c0 < ncand; c0 = nwarps * ch + warp_next(&D.ctr->work[2], ch)) {
+    // the chunk's records, one per lane
+    uint4 rec_l = make_uint4(0, 0, 0, 0), win_l = make_uint4(0, 0, 0, 0);
+    uint32_t bf_l = 0;
+    float4 pq_l = make_float4(0.f, 0.f, 0.f, 0.f);
+    bool mine = false;
+    if (lane < ch && c0 + lane < ncand) {
+      rec_l = ld_u4(&D.cand[c0 + lane]);
+      win_l = ld_u4(&D.cwin[c0 + lane]);
+      bf_l = D.cand_bf[c0 + lane];
+      pq_l = ld_f4(&D.pts[rec_l.x]);
+      mine = D.stat[rec_l.x].ins == uint16_t(R.round) && !(win_l.y & kWinBlock);
     }
-    const bool use_table = tk != nullptr;
-    if (use_table) {
-      for (uint32_t j = lane; j <= mask; j += 32) {
-        tk[j] = ~0ull;
-        t0[j] = NONE;
-        t1[j] = NONE;
-      }
-      __syncwarp();
-      for (uint32_t j = lane; j < F; j += 32) {
-        const uint32_t bf = D.bface[bfo + j];
-        const uint32_t c = bf >> 2;
-        const int f = int(bf & 3u);
-        const uint32_t sl = reinterpret_cast<const uint32_t*>(D.nslot + c)[f];
-        const uint4 V = D.T[c].v;
-        {
+    uint32_t todo = __ballot_sync(FULL, mine);
+    while (todo) {
+      const int j = __ffs(int(todo)) - 1;
+      todo &= todo - 1;
+      uint4 rec;
+      rec.x = __shfl_sync(FULL, rec_l.x, j);
+      rec.y = __shfl_sync(FULL, rec_l.y, j);
+      rec.z = __shfl_sync(FULL, rec_l.z, j);
+      rec.w = __shfl_sync(FULL, rec_l.w, j);
+      const uint32_t base = __shfl_sync(FULL, win_l.x, j), flags = __shfl_sync(FULL, win_l.y, j);
+      const uint32_t contested = __shfl_sync(FULL, win_l.z, j);
+      const uint32_t bfo = __shfl_sync(FULL, bf_l, j);
+      const float4 pq = make_float4(__shfl_sync(FULL, pq_l.x, j), __shfl_sync(FULL, pq_l.y, j),
+                                    __shfl_sync(FULL, pq_l.z, j), 0.f);
+      const uint32_t p = rec.x, K = rec.z, F = rec.w;
+      const uint32_t* cav = cand_cavity(D, rec.y);
+      const uint2* bf = reinterpret_cast<const uint2*>(D.pool + bfo);
+      const bool inplace = (flags & kWinInPlace) != 0u;
+      const uint32_t reused = inplace ? min(K, F) : 0u;
+      uint32_t s0 = 0;
+      bool bad = false;
+      EdgeTable E;
+      E.key = sm.key[w];
+      E.val = sm.val[w];
+      E.link = sm.link[w];
+      E.tab = sm.tab[w];
+      if (inplace) {
+        // One face per lane (F <= 32).  The star overwrites the cavity's own
+        // slots: every lane reads first, the warp synchronises, then writes.
+        E.mask = 127;  // at most 48 edges
+        table_clear(tm, E);
+        NewTet t;
+        uint4 V = make_uint4(0, 0, 0, 0);
+        uint2 e = make_uint2(0, NONE);
+        t.sl = 0;
+        if (lane < F) {
+          e = bf[lane];
+          const uint32_t sl = star_slot(D, R, cav, reused, base, lane);
+          star_face(D, R, e, sl, (contested >> lane) & 1u, p, pq, t, V);
+          table_publish(E, lane, V, int(e.x & 3u), t.sl);
+        }
+        __syncwarp();
+        if (lane < F) table_match(E, lane);
+        __syncwarp();
+        if (lane < F) {
+          const int f = int(e.x & 3u);
+          uint32_t i = 3 * lane;
+#pragma unroll
           for (int k = 0; k < 4; ++k) {
             if (k == f) continue;
-            const uint32_t a = edge_lo(V, f, k), b = edge_hi(V, f, k);
-            const unsigned long long ek = (static_cast<unsigned long long>(a) << 32) | b;
-            const uint32_t val = (sl << 2) | uint32_t(k);
-            uint32_t h = edge_hash(a, b, mask);
-            for (uint32_t probe = 0; probe <= mask; ++probe) {
-              const unsigned long long old = atomicCAS(&tk[h], ~0ull, ek);
-              if (old == ~0ull || old == ek) {
-                if (atomicCAS(&t0[h], NONE, val) != NONE) t1[h] = val;
-                break;
-              }
-              h = (h + 1) & mask;
-            }
+            const uint32_t link = E.link[i];
+            if (link == NONE) bad = true;
+            set_comp(t.n, k, link);
+            ++i;
           }
+          star_commit(D, t, f);
         }
+        s0 = __shfl_sync(FULL, t.sl, 0);
+      } else {
+        E.mask = kEdgeSlots - 1;
+        bool use_table = true;
+        if (F > kEdgeFaces) {
+          use_table = F <= kEdgeFacesG && gwarp < D.etab_warps;
+          uint32_t* words = D.etab + size_t(use_table ? gwarp : 0) * kEdgeWordsG;
+          E.key = reinterpret_cast<unsigned long long*>(words);
+          E.val = words + 6 * kEdgeFacesG;
+          E.link = E.val + 3 * kEdgeFacesG;
+          E.tab = E.link + 3 * kEdgeFacesG;
+          E.mask = kEdgeSlotsG - 1;
+        }
+        bad = !write_star(D, R, tm, rec, cav, bf, base, use_table, E, make_key(D, R, p), pq);
+        s0 = star_slot(D, R, cav, 0u, base, 0u);
+      }
+      if (__any_sync(FULL, bad) && lane == 0) atomicOr(&D.ctr->err, kErrRotate);
+      __syncwarp();  // every lane is done with the cavity before it is retired
+      if (K > reused) {
+        uint32_t fbase = 0;
+        if (lane == 0) fbase = atomicAdd(&D.ctr->n_freed_next, K - reused);
+        fbase = __shfl_sync(FULL, fbase, 0);
+        retire(D, R, tm, rec, cav, bf, reused, base, s0, fbase);
+      }
+      if (lane == 0) {
+        mark_inserted(D, p, s0);
+        ++inserted;
+        created += F;
       }
       __syncwarp();
     }
-    bool bad = false;
-    // The new tet of boundary face j (the compact list k_shared wrote): the
-    // cavity tet with the face's opposite vertex replaced by p, linked to the
-    // outer tet (or to another winner's new tet on a shared face) and, across
-    // its three faces through p, to its neighbours in the star.
-    auto build = [&](uint32_t j, uint4& nv, uint4& nn, uint32_t& sl, uint32_t& outer, bool& shared) {
-      const uint32_t bf = D.bface[bfo + j];
-      const uint32_t c = bf >> 2;
-      const int f = int(bf & 3u);
-      sl = reinterpret_cast<const uint32_t*>(D.nslot + c)[f];
-      const uint4 V = D.T[c].v;
-      outer = reinterpret_cast<const uint32_t*>(&D.T[c].n)[f];
-      shared = false;
-      uint32_t link_out = outer;
-      if (outer != NONE) {
-        const uint32_t o = outer >> 2;
-        const unsigned long long cc = __ldcg(&D.C[o].cav);
-        if (cc != key && this_round(R, cc)) {
-          const uint32_t q = key_owner(R, cc);
-          if (q < D.nv && D.st2[q]) {
-            shared = true;
-            link_out = (comp(D.nslot[o], outer & 3) << 2) | (outer & 3);
-          }
-        }
-      }
-      nv = V;
-      set_comp(nv, f, p);
-      nn = make_uint4(NONE, NONE, NONE, NONE);
-      set_comp(nn, f, link_out);
-      for (int k = 0; k < 4; ++k) {
-        if (k == f) continue;
-        uint32_t link = NONE;
-        if (use_table) {
-          const uint32_t a = edge_lo(V, f, k), b = edge_hi(V, f, k);
-          const unsigned long long ek = (static_cast<unsigned long long>(a) << 32) | b;
-          const uint32_t mine = (sl << 2) | uint32_t(k);
-          uint32_t h = edge_hash(a, b, mask);
-          for (uint32_t probe = 0; probe <= mask; ++probe) {
-            const unsigned long long kk = tk[h];
-            if (kk == ek) {
-              link = t0[h] == mine ? t1[h] : t0[h];
-              break;
-            }
-            if (kk == ~0ull) break;
-            h = (h + 1) & mask;
-          }
-        } else {
-          uint32_t cur = c;
-          uint4 Vc = V;
-          int kc = k, ms = f;
-          for (int it = 0; it < ROT_LIMIT; ++it) {
-            const uint32_t nb = comp(D.T[cur].n, kc);
-            if (boundary_face(D, nb, key)) {
-              link = (comp(D.nslot[cur], kc) << 2) | uint32_t(ms);
-              break;
-            }
-            const uint32_t nt = nb >> 2;
-            if (nt >= D.cap) break;
-            const int entry = int(nb & 3);
-            const uint32_t x = comp(Vc, ms);
-            const uint4 Wt = D.T[nt].v;
-            int kx = -1;
-            for (int q = 0; q < 4; ++q)
-              if (comp(Wt, q) == x) kx = q;
-            if (kx < 0) break;
-            cur = nt;
-            Vc = Wt;
-            kc = kx;
-            ms = entry;
-          }
-        }
-        if (link == NONE) bad = true;
-        set_comp(nn, k, link);
-      }
-    };
-    auto commit = [&](const uint4& nv, const uint4& nn, uint32_t sl, uint32_t outer, bool shared) {
-      D.T[sl].v = nv;
-      D.T[sl].n = nn;
-      D.C[sl].vote = 0ull;  // the new tet's points vote in k_relocate
-      // Every vertex on the cavity boundary gets a live incident tet, so a
-      // vertex's hint tet is alive whenever it is read (strata activation).
-      for (int q = 0; q < 4; ++q)
-        if (comp(nv, q) != p) D.vtet[comp(nv, q)] = sl;
-      if (outer != NONE && !shared && (outer >> 2) < D.cap) {
-        uint32_t* wp = reinterpret_cast<uint32_t*>(&D.T[outer >> 2].n) + (outer & 3);
-        const int f = comp(nv, 0) == p ? 0 : comp(nv, 1) == p ? 1 : comp(nv, 2) == p ? 2 : 3;
-        *wp = (sl << 2) | uint32_t(f);
-      }
-    };
-    if (inplace) {
-      // The star overwrites the cavity's own slots: every lane reads first,
-      // the warp synchronises, then every lane writes (F <= 32: one face each).
-      uint4 nv = make_uint4(0, 0, 0, 0), nn = make_uint4(0, 0, 0, 0);
-      uint32_t sl = 0, outer = NONE;
-      bool shared = false;
-      if (lane < F) build(lane, nv, nn, sl, outer, shared);
-      __syncwarp();
-      if (lane < F) commit(nv, nn, sl, outer, shared);
-    } else {
-      for (uint32_t j = lane; j < F; j += 32) {
-        uint4 nv, nn;
-        uint32_t sl, outer;
-        bool shared;
-        build(j, nv, nn, sl, outer, shared);
-        commit(nv, nn, sl, outer, shared);
-      }
-    }
-    if (__any_sync(0xFFFFFFFFu, bad) && lane == 0) atomicOr(&D.ctr->err, kErrRotate);
-    __syncwarp();  // every lane is done reading the cavity before it is retired
-    uint32_t s0 = 0;
-    if (lane == 0) {
-      const uint32_t bf0 = D.bface[bfo];
-      s0 = reinterpret_cast<const uint32_t*>(D.nslot + (bf0 >> 2))[bf0 & 3u];
-    }
-    s0 = __shfl_sync(0xFFFFFFFFu, s0, 0);
-    // cavity tets whose slots the star did not take are retired
-    const uint32_t reused = inplace ? min(K, F) : 0u;
-    uint32_t fbase = 0;
-    if (lane == 0 && K > reused) fbase = atomicAdd(&D.ctr->n_freed_next, K - reused);
-    fbase = __shfl_sync(0xFFFFFFFFu, fbase, 0);
-    for (uint32_t i = reused + lane; i < K; i += 32) {
-      const uint32_t c = cav[i];
-      // Points inside c relocate from a new tet on one of c's own faces.
-      const uint4 S = D.nslot[c];
-      const uint32_t fwd = S.x != NONE ? S.x : S.y != NONE ? S.y : S.z != NONE ? S.z : S.w != NONE ? S.w : s0;
-      D.T[c].v = make_uint4(DEAD, fwd, 0u, 0u);
-      R.freed_next[fbase + (i - reused)] = c;
-    }
-    if (lane == 0) {
-      if (D.log_pslot && D.log_pslot[p] != NONE) D.log_y[D.log_pslot[p]] = 1;  // scheduler log: inserted
-      D.vtet[p] = s0;
-      D.loc[p] |= INS_BIT;
-      D.centry[D.vcloud[p]] = s0;
-      D.bigflag[p] = 0;
-      ++inserted;
-      created += F;
-    }
-    __syncwarp();
   }
   // per-block statistics, one atomic each per block
   if (inserted) {
-    atomicAdd(&block_inserted, inserted);
-    atomicAdd(&block_created, created);
+    atomicAdd(&sm.inserted, inserted);
+    atomicAdd(&sm.created, created);
   }
   __syncthreads();
-  if (threadIdx.x == 0 && block_inserted) {
-    atomicAdd(&D.ctr->n_inserted, block_inserted);
-    atomicAdd(&D.ctr->created, block_created);
+  if (threadIdx.x == 0 && sm.inserted) {
+    atomicAdd(&D.ctr->n_inserted, sm.inserted);
+    atomicAdd(&D.ctr->created, sm.created);
   }
+}
+
+__global__ void __launch_bounds__(128, WTET_WRITE_MINB) k_write(Dev D) {
+  const RoundArgs R = load_round(D);
+  if (!R.live) return;
+  __shared__ WriteSmem<4> sm;
+  write_body<4>(D, R, sm);
 }
 
 // Clears the votes, relocates points whose tet was retired, compacts the
@@ -1769,10 +2050,10 @@ __global__ void __launch_bounds__(512, WTET_RELOC_MINB) k_relocate(Dev D) {
           // retired and overwritten by a star in place: t held a cavity tet
           // of a winner that inserted (its claim is this round's), and now
           // holds a tet of that winner's star, which covers the point
-          const unsigned long long cc = __ldcg(&D.C[t].cav);
+          const unsigned long long cc = __ldcg(&D.T[t].cav);
           if (this_round(R, cc)) {
             const uint32_t q = key_owner(R, cc);
-            if (q < D.nv && D.st2[q]) from = t;
+            if (q < D.nv && D.stat[q].ins == uint16_t(R.round)) from = t;
           }
         }
         if (from != NONE) {
@@ -1835,8 +2116,7 @@ __device__ void begin_round(const Dev& D) {
   C->big_used = 0;
   C->n_inserted = 0;
   C->huge_used = 0;
-  C->btab_used = 0;
-  C->bface_used = 0;
+  C->nbigw = 0;
   C->work[0] = C->work[1] = C->work[2] = C->work[3] = 0;
   for (uint32_t b = 0; b <= kOrderBuckets; ++b) C->sbc[b] = 0;
 }
@@ -2072,14 +2352,11 @@ struct Workspace {
   DBuf<uint32_t> sos, vcloud, vtet, loc;
   DBuf<uint8_t> bigflag;
   DBuf<Tet> T;
-  DBuf<Claim> C;
-  DBuf<uint4> nslot;
-  DBuf<uint32_t> bface;
-  DBuf<uint32_t> centry, active, active_next, cand, cand_off, cand_len, cand_base, cand_nf, pool, big, freed_a, freed_b;
-  DBuf<uint8_t> st1, st2;
-  DBuf<uint32_t> bigcand, starts, wscratch, etab_val;
-  DBuf<unsigned long long> etab_key, btab_key;
-  DBuf<uint32_t> btab_val;
+  DBuf<uint32_t> centry, active, active_next, cand_bf, bigw, pool, big, freed_a, freed_b;
+  DBuf<uint4> cand, cwin;
+  DBuf<Stat> stat;
+  DBuf<uint2> starts;
+  DBuf<uint32_t> bigcand, wscratch, etab, btab;
   DBuf<uint64_t> lvl_off;
   DBuf<uint32_t> lvl_total;
   DBuf<State> state;
@@ -2162,14 +2439,14 @@ void release_thread_workspace() {
   Workspace& w = *tl_ws;
   w.xyz.release(); w.off.release(); w.ci.release(); w.mn.release(); w.mx.release();
   w.bucket.release(); w.hist.release(); w.tmp.release(); w.pts.release(); w.sos.release();
-  w.vcloud.release(); w.vtet.release(); w.loc.release(); w.bigflag.release(); w.T.release(); w.C.release();
-  w.nslot.release(); w.bface.release();
+  w.vcloud.release(); w.vtet.release(); w.loc.release(); w.bigflag.release(); w.T.release();
+  
   w.centry.release(); w.active.release(); w.active_next.release(); w.cand.release();
-  w.cand_off.release(); w.cand_len.release(); w.cand_base.release(); w.cand_nf.release(); w.st1.release(); w.st2.release(); w.bigcand.release(); w.starts.release(); w.wscratch.release(); w.pool.release(); w.big.release();
+  w.cand_bf.release(); w.cwin.release(); w.stat.release(); w.bigw.release(); w.bigcand.release(); w.starts.release(); w.wscratch.release(); w.pool.release(); w.big.release();
   w.freed_a.release(); w.freed_b.release(); w.lvl_off.release(); w.lvl_total.release(); w.state.release(); w.ctr.release();
   w.ccount.release(); w.hullcnt.release(); w.cfill.release(); w.newid.release();
   w.hull.release(); w.coff.release(); w.out_t.release(); w.out_a.release(); w.dtab.release(); w.dup.release();
-  w.etab_key.release(); w.etab_val.release(); w.btab_key.release(); w.btab_val.release();
+  w.etab.release(); w.btab.release();
   w.log_pslot.release(); w.losses.release(); w.prio.release();
   for (auto& b : w.scan_tmp) b.release();
   if (w.h_ctr) cudaFreeHost(w.h_ctr);
@@ -2320,7 +2597,7 @@ void reserve_stack_once() {
   std::lock_guard<std::mutex> g(mu);
   if (dev < 0 || dev >= 64 || done[dev]) return;
   size_t need = 0;
-  const void* ks[] = {(const void*)k_bfs, (const void*)k_expand_big, (const void*)k_shared,
+  const void* ks[] = {(const void*)k_bfs, (const void*)k_shared,
                       (const void*)k_relocate, (const void*)k_activate, (const void*)k_init_clouds};
   for (const void* k : ks) {
     cudaFuncAttributes a{};
@@ -2391,27 +2668,28 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
   W.active.reserve(n, "active");
   W.active_next.reserve(n, "active");
   W.cand.reserve(n, "cand");
-  W.cand_off.reserve(n, "cand");
-  W.cand_len.reserve(n, "cand");
-  W.cand_base.reserve(n, "cand");
-  W.cand_nf.reserve(n, "cand");
-  W.st1.reserve(nv, "status");
+  W.cand_bf.reserve(n, "cand");
+  W.cwin.reserve(n, "cand");
+  W.stat.reserve(nv, "status");
+  W.bigw.reserve(kBigWinners, "large stars");
   W.bigcand.reserve(HUGE_SLOTS, "bigcand");
   // order-bucket regions: the expected n / kOrderBuckets starts per bucket
   // plus a 25% margin; anything beyond goes to the overflow region
   const uint64_t start_rc = n / kOrderBuckets + n / 64 + 1024;
   const uint64_t start_ovf = start_rc * kOrderBuckets;
   W.starts.reserve(start_ovf + n, "starts");
-  // one overflow queue per lane group of a k_bfs wave
-  W.wscratch.reserve(size_t(wave(k_bfs, 128)) * (128 / kBfsLanes) * BIG_CAP, "cavity queues");
-  const uint32_t etab_warps = wave(k_write, 128) * 4;  // one edge table per warp of a k_write wave
-  W.etab_key.reserve(size_t(etab_warps) * kEdgeSlotsG, "edge tables");
-  W.etab_val.reserve(size_t(etab_warps) * 2 * kEdgeSlotsG, "edge tables");
-  W.btab_key.reserve(size_t(kBigTables) * kBigTableSlots, "edge tables");
-  W.btab_val.reserve(size_t(kBigTables) * 2 * kBigTableSlots, "edge tables");
-  W.st2.reserve(nv, "status");
+  // one overflow region per lane group of a k_bfs wave, one edge table per
+  // warp of a k_write wave
+  const uint32_t wgroups = wave(k_bfs, 128) * 4 * kWarpGroups;
+  W.wscratch.reserve(size_t(wgroups) * kScratchWords, "cavity queues");
+  const uint32_t etab_warps = wave(k_write, 128) * 4;
+  W.etab.reserve(size_t(etab_warps) * kEdgeWordsG, "edge tables");
+  W.btab.reserve(size_t(kBigTables) * kBigEdgeWords, "edge tables");
+  // A round's cavity and boundary lists; the last term holds the largest
+  // boundary one cavity can have (a triangulated sphere over all vertices).
   const uint64_t pool_factor = std::min<uint32_t>(std::max<uint32_t>(cfg.pool_factor, 4u), 64u);
-  const uint32_t pool_cap = uint32_t(std::min<uint64_t>(std::max<uint64_t>(n * pool_factor, 1 << 16), 1ull << 30));
+  const uint32_t pool_cap = uint32_t(
+      std::min<uint64_t>(std::max<uint64_t>(n * pool_factor, 1 << 16) + 4 * n + 4096, 1ull << 30));
   W.pool.reserve(pool_cap, "pool");
   W.big.reserve(size_t(HUGE_SLOTS) * HUGE_CAP, "big");
   W.ctr.reserve(1, "counters");
@@ -2425,9 +2703,6 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
   W.coff.reserve(nc + 1, "coff");
   auto reserve_tets = [&](uint64_t cap) {
     W.T.reserve(cap, "tets");
-    W.nslot.reserve(cap, "nslot");
-    W.bface.reserve(cap, "boundary faces");
-    W.C.reserve(cap, "claims");
     W.freed_a.reserve(cap, "freed");
     W.freed_b.reserve(cap, "freed");
     W.newid.reserve(cap, "newid");
@@ -2440,8 +2715,9 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
   ck(cudaMemsetAsync(W.mn.p, 0xFF, 3ull * nc * 4, s), "memset");
   ck(cudaMemsetAsync(W.mx.p, 0x00, 3ull * nc * 4, s), "memset");
   ck(cudaMemsetAsync(W.hist.p, 0, (buckets + 1) * 4, s), "memset");
+  ck(cudaMemsetAsync(W.stat.p, 0, nv * sizeof(Stat), s), "memset");
   ck(cudaMemsetAsync(W.ctr.p, 0, sizeof(Counters), s), "memset");
-  k_init_slots<<<blocks_for(cap, 256, 148 * 16), 256, 0, s>>>(W.T.p, W.C.p, 0, cap);
+  k_init_slots<<<blocks_for(cap, 256, 148 * 16), 256, 0, s>>>(W.T.p, 0, cap);
   if (vmode) {
     W.losses.reserve(nv, "losses");
     ck(cudaMemsetAsync(W.losses.p, 0, nv, s), "memset");
@@ -2458,14 +2734,13 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
   Dev D{};
   auto refresh = [&]() {
     D.pts = W.pts.p; D.sos = W.sos.p; D.vcloud = W.vcloud.p; D.vtet = W.vtet.p; D.loc = W.loc.p;
-    D.bigflag = W.bigflag.p; D.T = W.T.p; D.C = W.C.p;
-    D.nslot = W.nslot.p; D.bface = W.bface.p; D.cap = uint32_t(cap); D.nv = uint32_t(nv); D.centry = W.centry.p;
-    D.cand = W.cand.p; D.cand_off = W.cand_off.p;
-    D.cand_len = W.cand_len.p; D.cand_base = W.cand_base.p; D.cand_nf = W.cand_nf.p; D.st1 = W.st1.p; D.st2 = W.st2.p; D.bigcand = W.bigcand.p;
+    D.bigflag = W.bigflag.p; D.T = W.T.p;
+    D.cap = uint32_t(cap); D.nv = uint32_t(nv); D.centry = W.centry.p;
+    D.cand = W.cand.p; D.cand_bf = W.cand_bf.p; D.cwin = W.cwin.p; D.stat = W.stat.p;
+    D.bigw = W.bigw.p; D.bigcand = W.bigcand.p; D.wgroups = wgroups;
     D.starts = W.starts.p; D.wscratch = W.wscratch.p;
     D.start_rc = uint32_t(start_rc); D.start_ovf = uint32_t(start_ovf);
-    D.etab_key = W.etab_key.p; D.etab_val = W.etab_val.p; D.etab_warps = etab_warps;
-    D.btab_key = W.btab_key.p; D.btab_val = W.btab_val.p;
+    D.etab = W.etab.p; D.etab_warps = etab_warps; D.btab = W.btab.p;
     D.prefilter = cfg.candidate_filter == 2 ? 0u : 1u; D.pool = W.pool.p; D.pool_cap = pool_cap; D.big = W.big.p;
     D.ctr = W.ctr.p;
     D.st = W.state.p; D.act[0] = W.active.p; D.act[1] = W.active_next.p;
@@ -2552,21 +2827,20 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
   // Every round kernel loops grid-stride over its work, so each gets exactly
   // one full wave of resident blocks: an idle round then costs one short
   // wave per kernel.
-  const uint32_t GB = HUGE_SLOTS;  // one block per huge-cavity slot
   struct Grids {
-    uint32_t act, vote, cand, candl, logf, bfs, res, sh, wr, rel;
+    uint32_t act, vote, cand, candl, logf, bfs, sh, wr, rel;
   };
   const Grids big{wave(k_activate, TB), 0u,      wave(k_cands, TB),
                   vmode == 1 ? wave(k_cands_learned, 256) : 0u,
-                  wave(k_log_features, TB), wave(k_bfs, 128), wave(k_resolve, 128), wave(k_shared, 128),
+                  wave(k_log_features, TB), wave(k_bfs, 128), wave(k_shared, 128),
                   wave(k_write, 128),  wave(k_relocate, TB)};
   // Rounds of the first strata have a few thousand points: a full wave of
   // blocks that exit at once costs more than their work, so those rounds
   // replay a graph with one block per SM.
   auto shrink = [](uint32_t g) { return std::min<uint32_t>(g, 148u); };
   const Grids small{shrink(big.act), 0u, shrink(big.cand), shrink(big.candl), shrink(big.logf),
-                    shrink(big.bfs), shrink(big.res),  shrink(big.sh),   shrink(big.wr),    shrink(big.rel)};
-  const uint64_t kernels_per_round = 9 + (vmode == 2 ? 1 : 0);
+                    shrink(big.bfs), shrink(big.sh),   shrink(big.wr),    shrink(big.rel)};
+  const uint64_t kernels_per_round = 7 + (vmode == 2 ? 1 : 0);
 
   // One round: k_end also starts the next round (k_begin starts the first).
   // `learned`: the learned scheduler's candidate kernel.
@@ -2576,8 +2850,6 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
     else k_cands<<<G.cand, TB, 0, s>>>(D);
     if (vmode == 2) k_log_features<<<G.logf, TB, 0, s>>>(D);
     k_bfs<<<G.bfs, 128, 0, s>>>(D);
-    k_expand_big<<<GB, 256, 0, s>>>(D);
-    k_resolve<<<G.res, 128, 0, s>>>(D);
     k_shared<<<G.sh, 128, 0, s>>>(D);
     k_write<<<G.wr, 128, 0, s>>>(D);
     k_relocate<<<G.rel, TB, 0, s>>>(D);
@@ -2666,10 +2938,7 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
       if (ncap <= cap) throw Error{WTET_ERR_CAPACITY, "tet capacity exhausted"};
       const uint32_t top = hs.tet_top;
       W.T.grow_keep(ncap, top, s, "grow tets");
-      W.C.grow_keep(ncap, top, s, "grow claims");
-      k_init_slots<<<blocks_for(ncap - top, 256, 148 * 16), 256, 0, s>>>(W.T.p, W.C.p, top, ncap);
-      W.nslot.grow_keep(ncap, 0, s, "grow nslot");
-      W.bface.grow_keep(ncap, 0, s, "grow boundary faces");
+      k_init_slots<<<blocks_for(ncap - top, 256, 148 * 16), 256, 0, s>>>(W.T.p, top, ncap);
       W.freed_a.grow_keep(ncap, ncap > 0 ? W.freed_a.n : 0, s, "grow freed");
       W.freed_b.grow_keep(ncap, W.freed_b.n, s, "grow freed");
       W.newid.grow_keep(ncap, 0, s, "grow newid");
