@@ -80,10 +80,10 @@
 #ifndef WTET_WRITE_MINB
 #define WTET_WRITE_MINB 8
 #endif
-// Rounds whose graph may see at most this many uninserted points run with one
-// block per SM per kernel (a full wave of blocks costs more than their work).
+// Rounds of at most this many uninserted points (with the stratum that may
+// join next) run inside k_rounds.
 #ifndef WTET_SMALL_ROUND_POINTS
-#define WTET_SMALL_ROUND_POINTS 32768
+#define WTET_SMALL_ROUND_POINTS 8192
 #endif
 #ifndef WTET_RELOC_MINB
 #define WTET_RELOC_MINB 1
@@ -124,24 +124,37 @@ enum : uint32_t {
   kErrBig = 1u << 7,    // a cavity outgrew the large-cavity slot
 };
 
+// Counters of one round (two sets, by round parity: a round's last pass reads
+// its own while the next round's are already clear).
 struct Counters {
   uint32_t n_next;        // uninserted points carried to the next round
   uint32_t n_cand;        // candidates that completed a cavity
   uint32_t pool_used;     // cavity-list pool entries
   uint32_t alloc_used;    // tet slots handed out this round (virtual index)
   uint32_t n_freed_next;  // tets retired this round
-  uint32_t big_used;      // large-cavity slots used
   uint32_t n_inserted;    // winners this round
   uint32_t huge_used;     // huge-cavity slots used
   uint32_t nbigw;         // winners whose star a whole block writes
-  uint32_t work[4];       // dynamic work cursors of k_bfs, k_shared, k_write (one spare)
+  uint32_t work[3];       // dynamic work cursors of k_bfs, k_shared, k_write
+  uint32_t ticket;        // blocks that have finished the round's last kernel
+  uint32_t err;           // error flags when the round ended
   uint32_t sbc[kOrderBuckets + 1];  // starts per order bucket (the last: overflow region)
-  uint32_t err;           // error flags
+};
+
+// Totals of a run.
+struct Totals {
+  uint32_t err;   // error flags
+  uint32_t ndup;  // exact duplicates
   unsigned long long walk_steps;
   unsigned long long n_expanded;
   unsigned long long n_big;
   unsigned long long created;
 };
+
+// Round flags: the round belongs to k_rounds (few points), the learned
+// scheduler sets its claim priorities.
+constexpr uint32_t kSmallRound = 1u;
+constexpr uint32_t kLearnedRound = 2u;
 
 // Round-loop state kept on the device, so that a round is a fixed kernel
 // sequence that can be replayed from a CUDA graph without host round trips.
@@ -154,14 +167,12 @@ struct alignas(16) State {
   uint32_t tet_top;       // first never-used tet slot
   uint32_t done;          // all points inserted
   uint32_t stop;          // 1 device error, 2 capacity exhausted, 3 no convergence
-  uint32_t pad0;
+  uint32_t flags;         // kSmallRound, kLearnedRound
   int32_t next_level;     // next stratum to locate (-1: none left)
   uint32_t stratum_size;  // size of the last located stratum
-  uint32_t strata;
-  uint32_t act_level, act_total, act_base;  // stratum located this round
-  uint32_t max_rounds;
   uint32_t overlap_shift;
-  uint32_t carry_used, carry_left;
+  uint32_t strata;
+  uint32_t max_rounds;
   uint32_t log_used;      // scheduler training records reserved
   unsigned long long inserted;
   unsigned long long starts;  // vote winners that attempted an insertion
@@ -243,7 +254,9 @@ struct Dev {
   uint32_t* pool;
   uint32_t pool_cap;
   uint32_t* big;
-  Counters* ctr;
+  Counters* ctr;  // two, by round parity
+  Totals* tot;
+  uint32_t small_points;  // rounds of at most this many points run inside k_rounds (0: none)
   int rule;
   // learned scheduler (vote_mode 1) and its training log (vote_mode 2)
   uint32_t vote_mode;
@@ -269,18 +282,16 @@ struct RoundArgs {
   uint32_t n_active;
   uint32_t n_freed_prev;
   uint32_t tet_top;
+  uint32_t flags;
+  Counters* ctr;
   bool live;
 };
 
-// Reads this round's arguments from the device state, with the current list
-// buffers.  D is not modified and its address never escapes into an
-// out-of-line call, so the kernel parameter block is read in place rather
-// than copied into each thread's local memory.
-__device__ __forceinline__ RoundArgs load_round(const Dev& D) {
-  // The state was written by earlier kernels of the sequence; kernel
-  // boundaries make it visible, and no round kernel modifies these fields.
-  const uint4 h0 = __ldcg(reinterpret_cast<const uint4*>(D.st));
-  const uint4 h1 = __ldcg(reinterpret_cast<const uint4*>(D.st) + 1);
+// This round's arguments from the first eight words of the state.  D is not
+// modified and its address never escapes into an out-of-line call, so the
+// kernel parameter block is read in place rather than copied into each
+// thread's local memory.
+__device__ __forceinline__ RoundArgs round_args(const Dev& D, const uint4& h0, const uint4& h1) {
   RoundArgs R;
   R.live = !h1.y && !h1.z;  // !done && !stop
   R.round = h0.x;
@@ -288,11 +299,23 @@ __device__ __forceinline__ RoundArgs load_round(const Dev& D) {
   R.n_active = R.live ? h0.y : 0u;
   R.n_freed_prev = h0.w;
   R.tet_top = h1.x;
+  R.flags = h1.w;
   const uint32_t par = h0.z & 1u;
   R.active = par ? D.act[1] : D.act[0];
   R.active_next = par ? D.act[0] : D.act[1];
   R.freed_prev = par ? D.freed[1] : D.freed[0];
   R.freed_next = par ? D.freed[0] : D.freed[1];
+  R.ctr = D.ctr + par;
+  return R;
+}
+// For the kernels of a large round; not live in a round that belongs to
+// k_rounds.  The state was written by earlier kernels of the sequence; kernel
+// boundaries make it visible, and only the last block of a round's last kernel
+// changes it.
+__device__ __forceinline__ RoundArgs load_round(const Dev& D) {
+  RoundArgs R = round_args(D, __ldcg(reinterpret_cast<const uint4*>(D.st)),
+                           __ldcg(reinterpret_cast<const uint4*>(D.st) + 1));
+  R.live = R.live && !(R.flags & kSmallRound);
   return R;
 }
 
@@ -477,11 +500,11 @@ __device__ __forceinline__ int in_sphere(const Dev& D, const Tet* T, const float
   if (s != 0) return s;
   const uint4 V = ld_u4(&T->v);
   if (V.x >= D.nv || V.y >= D.nv || V.z >= D.nv || V.w >= D.nv) {
-    atomicOr(&D.ctr->err, kErrGuard);
+    atomicOr(&D.tot->err, kErrGuard);
     return 1;
   }
   return o4d_sos_slow(corner(X, Y, Z, 0), corner(X, Y, Z, 1), corner(X, Y, Z, 2), corner(X, Y, Z, 3), pq, V.x, V.y,
-                      V.z, V.w, p, D.sos, &D.ctr->err);
+                      V.z, V.w, p, D.sos, &D.tot->err);
 }
 
 // Visibility walk with exact orient3d + SoS from tet t to the tet containing p.
@@ -489,13 +512,13 @@ __device__ __forceinline__ uint32_t walk_to(const Dev& D, uint32_t t, uint32_t p
   int entry = -1;
   for (uint32_t s = 0; s < WALK_LIMIT; ++s) {
     if (t >= D.cap) {
-      atomicOr(&D.ctr->err, kErrGuard);
+      atomicOr(&D.tot->err, kErrGuard);
       return 0;
     }
     const uint4 V = ld_u4(&D.T[t].v), N = ld_u4(&D.T[t].n);
     const float4 X = ld_f4(&D.T[t].X), Y = ld_f4(&D.T[t].Y), Z = ld_f4(&D.T[t].Z);
     if (V.x >= D.nv || V.y >= D.nv || V.z >= D.nv || V.w >= D.nv) {
-      atomicOr(&D.ctr->err, kErrGuard);
+      atomicOr(&D.tot->err, kErrGuard);
       return t;
     }
     const float4 P0 = corner(X, Y, Z, 0), P1 = corner(X, Y, Z, 1), P2 = corner(X, Y, Z, 2), P3 = corner(X, Y, Z, 3);
@@ -505,7 +528,7 @@ __device__ __forceinline__ uint32_t walk_to(const Dev& D, uint32_t t, uint32_t p
       if (f == entry) continue;
       // the tet with vertex f replaced by p
       if (o3d_sos_f(f == 0 ? pq : P0, f == 1 ? pq : P1, f == 2 ? pq : P2, f == 3 ? pq : P3, f == 0 ? p : V.x,
-                    f == 1 ? p : V.y, f == 2 ? p : V.z, f == 3 ? p : V.w, D.sos, &D.ctr->err) == -1) {
+                    f == 1 ? p : V.y, f == 2 ? p : V.z, f == 3 ? p : V.w, D.sos, &D.tot->err) == -1) {
         moved = f;
         break;
       }
@@ -516,13 +539,13 @@ __device__ __forceinline__ uint32_t walk_to(const Dev& D, uint32_t t, uint32_t p
     }
     const uint32_t n = comp(N, moved);
     if (n == NONE) {
-      atomicOr(&D.ctr->err, kErrWalk);
+      atomicOr(&D.tot->err, kErrWalk);
       return t;
     }
     t = n >> 2;
     entry = int(n & 3);
   }
-  atomicOr(&D.ctr->err, kErrWalk);
+  atomicOr(&D.tot->err, kErrWalk);
   return t;
 }
 
@@ -725,7 +748,7 @@ __global__ void k_init_clouds(const CloudInfo* ci, uint32_t nc, Dev D) {
   }
   double P[4][3];
   for (int k = 0; k < 4; ++k) load_pt(D.pts, s0 + k, P[k]);
-  int o = o3d_sos(P[0], P[1], P[2], P[3], s0, s0 + 1, s0 + 2, s0 + 3, D.sos, &D.ctr->err);
+  int o = o3d_sos(P[0], P[1], P[2], P[3], s0, s0 + 1, s0 + 2, s0 + 3, D.sos, &D.tot->err);
   D.T[c].v = (o > 0) ? make_uint4(s0, s0 + 1, s0 + 2, s0 + 3) : make_uint4(s0 + 1, s0, s0 + 2, s0 + 3);
   D.T[c].n = make_uint4(NONE, NONE, NONE, NONE);
   float4 q[4];
@@ -774,71 +797,25 @@ __device__ __forceinline__ float vote_score(const Tet& t, float4 q, int rule) {
 // every slot it writes a new tet into.
 __device__ __forceinline__ void cast_vote(const Dev& D, uint32_t p, uint32_t t) {
   if (t >= D.cap) {
-    atomicOr(&D.ctr->err, kErrGuard);
+    atomicOr(&D.tot->err, kErrGuard);
     return;
   }
   const float sc = vote_score(D.T[t], D.pts[p], D.rule);
   atomicMax(&D.T[t].vote, ((unsigned long long)__float_as_uint(sc) << 32) | (unsigned long long)(~p));
 }
 
-// Locates the points of one stratum: walk from the tet of the point one
-// stride earlier on the Morton curve (a point of an earlier stratum: its tet
-// once inserted, else the tet that still contains it).  The located points are
-// appended to the uninserted list at position `base`.
-__global__ void __launch_bounds__(512, WTET_RELOC_MINB) k_activate(Dev D) {
-  RoundArgs R = load_round(D);
-  if (!R.live) return;
-  volatile State* S = D.st;
-  const uint32_t total = S->act_total;
-  if (total == 0) return;
-  const uint32_t level = S->act_level, base = S->act_base, nc = D.nc;
-  const uint64_t* lvl_off = D.lvl_off + size_t(level) * (nc + 1);
-  const CloudInfo* ci = D.ci;
-  uint32_t steps = 0;
-  for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
-    uint32_t lo = 0, hi = nc;
-    while (hi - lo > 1) {
-      uint32_t mid = (lo + hi) >> 1;
-      if (lvl_off[mid] <= idx) lo = mid;
-      else hi = mid;
-    }
-    uint32_t c = lo;
-    CloudInfo C = ci[c];
-    uint32_t k = idx - uint32_t(lvl_off[c]);
-    uint32_t stride = 1u << level;
-    uint32_t pos = (level == C.top) ? k * stride : (2u * k + 1u) * stride;
-    uint32_t p = C.vbase + pos;
-    R.active[base + idx] = p;
-    if (D.bigflag[p] & kDup) continue;  // never located, dropped by k_relocate
-    uint32_t t = NONE;
-    if (level < C.top) {
-      uint32_t hv = p - stride;
-      uint32_t hl = D.loc[hv];
-      uint32_t h = (hl & INS_BIT) ? D.vtet[hv] : hl;
-      if (h != NONE && h < D.cap) {
-        uint4 V = D.T[h].v;
-        if (V.x < D.nv && D.vcloud[V.x] == c) t = h;
-      }
-    }
-    if (t == NONE) t = D.centry[c];
-    const uint32_t lt = walk_to(D, t, p, D.pts[p], steps);
-    D.loc[p] = lt;
-    D.bigflag[p] = 0;
-    cast_vote(D, p, lt);
-  }
-  if (steps) atomicAdd(&D.ctr->walk_steps, (unsigned long long)steps);
-}
-
 // Prefix of the order buckets' start counts, in shared memory (sp has
 // kOrderBuckets + 2 entries; sp[kOrderBuckets + 1] is the total).  Called by
 // every thread of the block.
-__device__ __forceinline__ void load_start_prefix(const Dev& D, uint32_t* sp) {
+__device__ __forceinline__ void load_start_prefix(const Dev& D, const RoundArgs& R, uint32_t* sp) {
   if (threadIdx.x == 0) {
-    uint32_t acc = 0;
+    uint32_t acc = 0, cnt[kOrderBuckets + 1];
+#pragma unroll
+    for (uint32_t b = 0; b <= kOrderBuckets; ++b) cnt[b] = __ldcg(&R.ctr->sbc[b]);
+#pragma unroll
     for (uint32_t b = 0; b <= kOrderBuckets; ++b) {
       sp[b] = acc;
-      const uint32_t c = __ldcg(&D.ctr->sbc[b]);
-      acc += b < kOrderBuckets ? min(c, D.start_rc) : c;
+      acc += b < kOrderBuckets ? min(cnt[b], D.start_rc) : cnt[b];
     }
     sp[kOrderBuckets + 1] = acc;
   }
@@ -916,7 +893,7 @@ __global__ void k_log_features(Dev D) {
   const RoundArgs R = load_round(D);
   if (!R.live || R.n_active > D.learned_points) return;
   __shared__ uint32_t sp[kOrderBuckets + 2];
-  load_start_prefix(D, sp);
+  load_start_prefix(D, R, sp);
   const uint32_t nstart = sp[kOrderBuckets + 1];
   for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < nstart; s += gridDim.x * blockDim.x) {
     const uint32_t p = start_at(D, sp, s).x;
@@ -934,13 +911,12 @@ __global__ void k_log_features(Dev D) {
   }
 }
 
-// Shared memory of the learned candidate kernel: the network's weights and
+// Shared memory of the learned candidate pass, besides the network's weights:
 // one staged feature row per lane.
-constexpr uint32_t kCandWarps = 8;  // k_cands_learned runs 256-thread blocks
+template <uint32_t kWarps>
 struct CandSmem {
-  mlp::Smem S;
-  uint32_t rows[kCandWarps][32 * mlp::kRowStride];
-  float outs[kCandWarps][32];
+  uint32_t rows[kWarps][32 * mlp::kRowStride];
+  float outs[kWarps][32];
 };
 
 // Candidates: the vote winner of each tet (the reference's pick_winner_point
@@ -949,8 +925,8 @@ struct CandSmem {
 // With kLearned, the fused network scores the warp's winners and sets their
 // claim priority; the start list is bucketed by that priority (better first)
 // instead of by the claim hash.
-template <bool kLearned>
-__device__ __forceinline__ void cands_body(const Dev& D, const RoundArgs& R, CandSmem* sm) {
+template <bool kLearned, uint32_t kWarps>
+__device__ __forceinline__ void cands_body(const Dev& D, const RoundArgs& R, const mlp::Smem* net, CandSmem<kWarps>* sm) {
   const uint32_t lane = threadIdx.x & 31u;
   for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < R.n_active; i0 += gridDim.x * blockDim.x) {
     const uint32_t i = i0 + threadIdx.x;
@@ -965,7 +941,7 @@ __device__ __forceinline__ void cands_body(const Dev& D, const RoundArgs& R, Can
       if (!(tier & kDup) && t < D.cap && uint32_t(vote) == ~p) {
         if (D.losses && D.losses[p] < 255u) D.losses[p] += 1u;
         if (tier == 2) {
-          uint32_t b = atomicAdd(&D.ctr->huge_used, 1u);
+          uint32_t b = atomicAdd(&R.ctr->huge_used, 1u);
           if (b < HUGE_SLOTS) D.bigcand[b] = p;
         } else if (!tier) {
           start = true;
@@ -983,7 +959,7 @@ __device__ __forceinline__ void cands_body(const Dev& D, const RoundArgs& R, Can
         if (start) winner_features(D, R, p, t, vote, f);
         mlp::stage_row(sm->rows[w] + lane * mlp::kRowStride, f);
         __syncwarp();
-        mlp::score32(sm->S, sm->rows[w], sm->outs[w]);
+        mlp::score32(*net, sm->rows[w], sm->outs[w]);
         if (start) {
           float sc = sm->outs[w][lane];
           sc = (sc == sc) ? fminf(fmaxf(sc, -20.f), 20.f) : 0.f;
@@ -1001,18 +977,17 @@ __device__ __forceinline__ void cands_body(const Dev& D, const RoundArgs& R, Can
       b = start ? (mix32(p ^ (R.round * 0x9E3779B9u)) >> 28) : 0u;
     }
     if (start && D.prefilter) pre_claim(D, t, start_key(D, R, p));
-    warp_append(&D.ctr->big_used, start);  // total count
     const unsigned grp = __match_any_sync(0xFFFFFFFFu, start ? b : 0xFFFFFFFFu);
     const uint32_t leader = uint32_t(__ffs(grp) - 1);
     uint32_t base = 0;
-    if (start && lane == leader) base = atomicAdd(&D.ctr->sbc[b], uint32_t(__popc(grp)));
+    if (start && lane == leader) base = atomicAdd(&R.ctr->sbc[b], uint32_t(__popc(grp)));
     base = __shfl_sync(0xFFFFFFFFu, base, int(leader));
     if (start) {
       const uint32_t slot = base + uint32_t(__popc(grp & ((1u << lane) - 1u)));
       if (slot < D.start_rc) {
         D.starts[b * D.start_rc + slot] = make_uint2(p, t);
       } else {  // a bucket beyond its region (never expected): the overflow region
-        D.starts[D.start_ovf + atomicAdd(&D.ctr->sbc[kOrderBuckets], 1u)] = make_uint2(p, t);
+        D.starts[D.start_ovf + atomicAdd(&R.ctr->sbc[kOrderBuckets], 1u)] = make_uint2(p, t);
       }
     }
   }
@@ -1021,17 +996,22 @@ __device__ __forceinline__ void cands_body(const Dev& D, const RoundArgs& R, Can
 __global__ void k_cands(Dev D) {
   const RoundArgs R = load_round(D);
   if (!R.live) return;
-  cands_body<false>(D, R, nullptr);
+  cands_body<false, 1>(D, R, nullptr, nullptr);
 }
 
 // The learned scheduler's candidate kernel (256-thread blocks).
 __global__ void __launch_bounds__(256) k_cands_learned(Dev D) {
   const RoundArgs R = load_round(D);
   if (!R.live) return;
-  __shared__ __align__(16) CandSmem sm;
-  mlp::load_image(sm.S, D.mlp);
+  __shared__ __align__(16) mlp::Smem net;
+  __shared__ __align__(16) CandSmem<8> sm;
+  if (!(R.flags & kLearnedRound)) {
+    cands_body<false, 1>(D, R, nullptr, nullptr);
+    return;
+  }
+  mlp::load_image(net, D.mlp);
   __syncthreads();
-  cands_body<true>(D, R, &sm);
+  cands_body<true, 8>(D, R, &net, &sm);
 }
 
 // Cavity growth by groups of kBfsLanes lanes, kWarpGroups at a time per warp:
@@ -1172,16 +1152,16 @@ __device__ __forceinline__ void expand_big(const Dev& D, const RoundArgs& R, uin
         }
       }
       __syncthreads();
-      if (pass == 0 && tid == 0) h[kOff] = atomicAdd(&D.ctr->pool_used, 2u * h[kF]);
+      if (pass == 0 && tid == 0) h[kOff] = atomicAdd(&R.ctr->pool_used, 2u * h[kF]);
       __syncthreads();
     }
   }
   if (tid == 0) {
-    atomicAdd(&D.ctr->n_big, 1ull);
-    if (h[kBad] & 4u) atomicOr(&D.ctr->err, kErrGuard);
-    if (h[kBad] & 2u) atomicOr(&D.ctr->err, kErrBig);
+    atomicAdd(&D.tot->n_big, 1ull);
+    if (h[kBad] & 4u) atomicOr(&D.tot->err, kErrGuard);
+    if (h[kBad] & 2u) atomicOr(&D.tot->err, kErrBig);
     if (h[kBad] == 0u && h[kOff] + 2u * h[kF] <= D.pool_cap && h[kNew] == h[kF]) {
-      const uint32_t ci = atomicAdd(&D.ctr->n_cand, 1u);
+      const uint32_t ci = atomicAdd(&R.ctr->n_cand, 1u);
       D.cand[ci] = make_uint4(p, 0x80000000u | bi, K, h[kF]);
       D.cand_bf[ci] = h[kOff];
       D.stat[p].done = uint16_t(R.round);
@@ -1193,8 +1173,11 @@ __device__ __forceinline__ void expand_big(const Dev& D, const RoundArgs& R, uin
 template <uint32_t kWarps>
 __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSmem<kWarps>& sm) {
   constexpr uint32_t FULL = 0xFFFFFFFFu, GM = (kBfsLanes == 32) ? 0xFFFFFFFFu : ((1u << kBfsLanes) - 1u);
+  // the next round's counters (their last readers finished with the last round)
+  if (blockIdx.x == 0 && threadIdx.x < sizeof(Counters) / 4)
+    reinterpret_cast<uint32_t*>(D.ctr + (1u - uint32_t(R.ctr - D.ctr)))[threadIdx.x] = 0u;
   // one block per huge candidate, before the block's share of the starts
-  const uint32_t nhuge = min(__ldcg(&D.ctr->huge_used), HUGE_SLOTS);
+  const uint32_t nhuge = min(__ldcg(&R.ctr->huge_used), HUGE_SLOTS);
   for (uint32_t bi = blockIdx.x; bi < nhuge; bi += gridDim.x) expand_big(D, R, bi, sm.huge);
   const uint32_t lane = threadIdx.x & 31, gl = lane % kBfsLanes, shift = lane - gl;
   const uint32_t lt = (1u << gl) - 1u;
@@ -1206,7 +1189,7 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
   uint32_t* gq = D.wscratch + size_t(gid < D.wgroups ? gid : 0) * kScratchWords;
   uint2* gb = reinterpret_cast<uint2*>(gq + BIG_CAP);
   if (threadIdx.x == 0) sm.searches = 0;
-  load_start_prefix(D, sm.sp);
+  load_start_prefix(D, R, sm.sp);
   const uint32_t nstart = sm.sp[kOrderBuckets + 1];
   const uint32_t nwarps = gridDim.x * kWarps;
   // About four fetches per warp, between one start per lane group and one per lane.
@@ -1217,8 +1200,8 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
   unsigned long long searches = 0;
   uint32_t pool_at = 0, pool_end = 0;  // the group's reserved pool words
   const uint32_t lgrp = lane / kBfsLanes;
-  for (uint32_t base = (blockIdx.x * kWarps + warp) * chunk; base < nstart;
-       base = nwarps * chunk + warp_next(&D.ctr->work[0], chunk)) {
+  for (uint32_t base = (warp * gridDim.x + blockIdx.x) * chunk; base < nstart;
+       base = nwarps * chunk + warp_next(&R.ctr->work[0], chunk)) {
     // ---- one start per lane: its pre-claims (its tet and the four face neighbours) must all hold
     const uint32_t si = base + lane;
     bool ok = lane < chunk && si < nstart;
@@ -1351,7 +1334,7 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
       const uint32_t g_over = (__ballot_sync(FULL, my_over) >> shift) & GM;
       bool fin = false;
       if (running) {
-        if (g_guard && gl == 0) atomicOr(&D.ctr->err, kErrGuard);
+        if (g_guard && gl == 0) atomicOr(&D.tot->err, kErrGuard);
         lost = lost || g_lost || g_guard;
         overflow = overflow || g_over;
         head = min(head + kBfsLanes / 4u, K);
@@ -1371,7 +1354,7 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
         if (pool_at + need > pool_end) {
           const uint32_t want = max(need, pool_chunk);  // even
           uint32_t got = 0;
-          if (gl == 0) got = atomicAdd(&D.ctr->pool_used, want);
+          if (gl == 0) got = atomicAdd(&R.ctr->pool_used, want);
           got = __shfl_sync(GM << shift, got, int(shift));
           pool_at = got;
           pool_end = got + want;
@@ -1400,7 +1383,7 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
       __syncwarp();
     }
     // ---- one reservation for the batch's completed cavities
-    const uint32_t ci = warp_append(&D.ctr->n_cand, rec_k != 0u);
+    const uint32_t ci = warp_append(&R.ctr->n_cand, rec_k != 0u);
     if (rec_k) {
       D.cand[ci] = make_uint4(p_l, rec_off, rec_k, rec_f);
       D.cand_bf[ci] = rec_bf;
@@ -1411,7 +1394,7 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
   // per-block statistics, one atomic per block
   if (searches) atomicAdd(&sm.searches, searches);
   __syncthreads();
-  if (threadIdx.x == 0 && sm.searches) atomicAdd(&D.ctr->n_expanded, sm.searches);
+  if (threadIdx.x == 0 && sm.searches) atomicAdd(&D.tot->n_expanded, sm.searches);
 }
 
 __global__ void __launch_bounds__(128, WTET_BFS_MINB) k_bfs(Dev D) {
@@ -1456,12 +1439,12 @@ template <uint32_t kWarps>
 __device__ __forceinline__ void shared_body(const Dev& D, const RoundArgs& R) {
   constexpr uint32_t FULL = 0xFFFFFFFFu;
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t ncand = __ldcg(&D.ctr->n_cand);
+  const uint32_t ncand = __ldcg(&R.ctr->n_cand);
   const uint32_t ch = chunk_for(ncand);
   const uint32_t nwarps = gridDim.x * kWarps;
   const uint16_t stamp = uint16_t(R.round);
-  for (uint32_t c0 = (blockIdx.x * kWarps + (threadIdx.x >> 5)) * ch; c0 < ncand;
-       c0 = nwarps * ch + warp_next(&D.ctr->work[1], ch)) {
+  for (uint32_t c0 = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * ch; c0 < ncand;
+       c0 = nwarps * ch + warp_next(&R.ctr->work[1], ch)) {
     // the chunk's records, one per lane; a cavity that lost a tet is out
     uint4 rec_l = make_uint4(0, 0, 0, 0);
     uint32_t bf_l = 0;
@@ -1518,7 +1501,7 @@ __device__ __forceinline__ void shared_body(const Dev& D, const RoundArgs& R) {
         set_fcomp(Y, f, pq.y);
         set_fcomp(Z, f, pq.z);
         if (o4d_sos_call(corner(X, Y, Z, 0), corner(X, Y, Z, 1), corner(X, Y, Z, 2), corner(X, Y, Z, 3), D.pts[q], V.x,
-                         V.y, V.z, V.w, q, D.sos, &D.ctr->err) < 0)
+                         V.y, V.z, V.w, q, D.sos, &D.tot->err) < 0)
           bad = true;
       }
       bad = __any_sync(FULL, bad);
@@ -1536,7 +1519,7 @@ __device__ __forceinline__ void shared_body(const Dev& D, const RoundArgs& R) {
     }
     // one reservation for the chunk (the counter is shared by the whole grid)
     uint32_t b0 = 0;
-    if (lane == 0 && sum) b0 = atomicAdd(&D.ctr->alloc_used, sum);
+    if (lane == 0 && sum) b0 = atomicAdd(&R.ctr->alloc_used, sum);
     b0 = __shfl_sync(FULL, b0, 0);
     uint32_t flags_l = 0, base_l = 0, touch_l = 0;
 #pragma unroll
@@ -1546,7 +1529,7 @@ __device__ __forceinline__ void shared_body(const Dev& D, const RoundArgs& R) {
       const uint32_t bfo = __shfl_sync(FULL, bf_l, int(j));
       const uint32_t mybase = b0 + base[j], last = mybase + fresh[j];
       if (last > R.n_freed_prev && R.tet_top + (last - R.n_freed_prev) > D.cap) {
-        if (lane == 0) atomicOr(&D.ctr->err, kErrCapacity);
+        if (lane == 0) atomicOr(&D.tot->err, kErrCapacity);
         if (lane == j) keep_l = false;
         continue;
       }
@@ -1570,7 +1553,7 @@ __device__ __forceinline__ void shared_body(const Dev& D, const RoundArgs& R) {
         touch_l = touch[j];
         flags_l = F[j] <= kInPlaceFaces && !(off & 0x80000000u) ? kWinInPlace : 0u;
         if (F[j] > kBlockFaces) {
-          const uint32_t i = atomicAdd(&D.ctr->nbigw, 1u);
+          const uint32_t i = atomicAdd(&R.ctr->nbigw, 1u);
           if (i < kBigWinners) {
             D.bigw[i] = c0 + j;
             flags_l |= kWinBlock;
@@ -1849,15 +1832,15 @@ __device__ __forceinline__ void write_body(const Dev& D, const RoundArgs& R, Wri
   constexpr uint32_t FULL = 0xFFFFFFFFu;
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t w = threadIdx.x >> 5;
-  const uint32_t gwarp = blockIdx.x * kWarps + w;
-  const uint32_t ncand = __ldcg(&D.ctr->n_cand);
+  const uint32_t gwarp = w * gridDim.x + blockIdx.x;
+  const uint32_t ncand = __ldcg(&R.ctr->n_cand);
   if (threadIdx.x == 0) {
     sm.inserted = 0;
     sm.created = 0;
   }
   __syncthreads();
   // ---- the largest stars, one block each
-  const uint32_t nbig = min(__ldcg(&D.ctr->nbigw), kBigWinners);
+  const uint32_t nbig = min(__ldcg(&R.ctr->nbigw), kBigWinners);
   const uint32_t big_blocks = min(gridDim.x, kBigTables);
   for (uint32_t i = blockIdx.x; blockIdx.x < big_blocks && i < nbig; i += big_blocks) {
     const BlockTeam tm;
@@ -1878,12 +1861,12 @@ __device__ __forceinline__ void write_body(const Dev& D, const RoundArgs& R, Wri
     __syncthreads();
     if (!write_star(D, R, tm, rec, cav, bf, win.x, rec.w <= kBigTableFaces, E, make_key(D, R, rec.x), D.pts[rec.x]))
       sm.bad = 1;
-    if (threadIdx.x == 0) sm.fbase = atomicAdd(&D.ctr->n_freed_next, rec.z);
+    if (threadIdx.x == 0) sm.fbase = atomicAdd(&R.ctr->n_freed_next, rec.z);
     __syncthreads();  // every thread is done reading the cavity before it is retired
     const uint32_t s0 = star_slot(D, R, cav, 0u, win.x, 0u);
     retire(D, R, tm, rec, cav, bf, 0u, win.x, s0, sm.fbase);
     if (threadIdx.x == 0) {
-      if (sm.bad) atomicOr(&D.ctr->err, kErrRotate);
+      if (sm.bad) atomicOr(&D.tot->err, kErrRotate);
       mark_inserted(D, rec.x, s0);
       sm.inserted += 1;
       sm.created += rec.w;
@@ -1896,7 +1879,7 @@ __device__ __forceinline__ void write_body(const Dev& D, const RoundArgs& R, Wri
   unsigned long long created = 0;
   const uint32_t ch = chunk_for(ncand);
   const uint32_t nwarps = gridDim.x * kWarps;
-  for (uint32_t c0 = gwarp * ch; c0 < ncand; c0 = nwarps * ch + warp_next(&D.ctr->work[2], ch)) {
+  for (uint32_t c0 = gwarp * ch; c0 < ncand; c0 = nwarps * ch + warp_next(&R.ctr->work[2], ch)) {
     // the chunk's records, one per lane
     uint4 rec_l = make_uint4(0, 0, 0, 0), win_l = make_uint4(0, 0, 0, 0);
     uint32_t bf_l = 0;
@@ -1982,11 +1965,11 @@ __device__ __forceinline__ void write_body(const Dev& D, const RoundArgs& R, Wri
         bad = !write_star(D, R, tm, rec, cav, bf, base, use_table, E, make_key(D, R, p), pq);
         s0 = star_slot(D, R, cav, 0u, base, 0u);
       }
-      if (__any_sync(FULL, bad) && lane == 0) atomicOr(&D.ctr->err, kErrRotate);
+      if (__any_sync(FULL, bad) && lane == 0) atomicOr(&D.tot->err, kErrRotate);
       __syncwarp();  // every lane is done with the cavity before it is retired
       if (K > reused) {
         uint32_t fbase = 0;
-        if (lane == 0) fbase = atomicAdd(&D.ctr->n_freed_next, K - reused);
+        if (lane == 0) fbase = atomicAdd(&R.ctr->n_freed_next, K - reused);
         fbase = __shfl_sync(FULL, fbase, 0);
         retire(D, R, tm, rec, cav, bf, reused, base, s0, fbase);
       }
@@ -2005,8 +1988,8 @@ __device__ __forceinline__ void write_body(const Dev& D, const RoundArgs& R, Wri
   }
   __syncthreads();
   if (threadIdx.x == 0 && sm.inserted) {
-    atomicAdd(&D.ctr->n_inserted, sm.inserted);
-    atomicAdd(&D.ctr->created, sm.created);
+    atomicAdd(&R.ctr->n_inserted, sm.inserted);
+    atomicAdd(&D.tot->created, sm.created);
   }
 }
 
@@ -2017,13 +2000,75 @@ __global__ void __launch_bounds__(128, WTET_WRITE_MINB) k_write(Dev D) {
   write_body<4>(D, R, sm);
 }
 
-// Clears the votes, relocates points whose tet was retired, compacts the
-// uninserted list, and carries the recycled slots that were not handed out
-// this round over to the next round's list.
-__global__ void __launch_bounds__(512, WTET_RELOC_MINB) k_relocate(Dev D) {
-  const RoundArgs R = load_round(D);
-  if (!R.live) return;
+// The stratum that starts after a round which inserted `inserted` points: the
+// next non-empty one once the current one has thinned to 1/2^overlap_shift of
+// its size (duplicates that are still listed count as thinning later).
+struct NextStratum {
+  int32_t level;   // located now (total > 0)
+  uint32_t total;
+  int32_t next;    // the state's next_level afterwards
+};
+__device__ __forceinline__ NextStratum next_stratum(const Dev& D, int32_t next_level, uint32_t stratum_size,
+                                                    uint32_t overlap_shift, uint32_t n_active, uint32_t inserted) {
+  NextStratum ns{-1, 0u, next_level};
+  const uint32_t left = n_active - min(n_active, inserted);
+  while (ns.next >= 0 && (left == 0 || (uint64_t(left) << overlap_shift) <= stratum_size)) {
+    ns.level = ns.next--;
+    ns.total = D.lvl_total[ns.level];
+    if (ns.total) break;
+  }
+  return ns;
+}
+
+// Relocates the points whose tet was retired and compacts the uninserted list;
+// locates the next stratum when it is due (in front of the carried points);
+// carries the recycled slots that were not handed out this round over.
+//
+// A point of the new stratum walks from the tet of the point one stride
+// earlier on the curve (a point of an earlier stratum: its tet once inserted,
+// else the tet that contains it -- as of this round or, while this very pass
+// relocates it, of the last one; a retired tet forwards to a live one).
+__device__ __forceinline__ void relocate_body(const Dev& D, const RoundArgs& R, const NextStratum& ns) {
   uint32_t steps = 0;
+  if (ns.total) {
+    const uint32_t level = uint32_t(ns.level), nc = D.nc;
+    const uint64_t* lvl_off = D.lvl_off + size_t(level) * (nc + 1);
+    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < ns.total; idx += gridDim.x * blockDim.x) {
+      uint32_t lo = 0, hi = nc;
+      while (hi - lo > 1) {
+        uint32_t mid = (lo + hi) >> 1;
+        if (lvl_off[mid] <= idx) lo = mid;
+        else hi = mid;
+      }
+      const uint32_t c = lo;
+      const CloudInfo C = D.ci[c];
+      const uint32_t k = idx - uint32_t(lvl_off[c]);
+      const uint32_t stride = 1u << level;
+      const uint32_t pos = (level == C.top) ? k * stride : (2u * k + 1u) * stride;
+      const uint32_t p = C.vbase + pos;
+      R.active_next[idx] = p;
+      if (D.bigflag[p] & kDup) continue;  // never located, dropped by the next pass
+      uint32_t t = NONE;
+      if (level < C.top) {
+        const uint32_t hv = p - stride;
+        const uint32_t hl = __ldcg(&D.loc[hv]);
+        uint32_t h = (hl & INS_BIT) ? D.vtet[hv] : hl;
+        if (h < D.cap) {
+          uint4 V = ld_u4(&D.T[h].v);
+          if (V.x == DEAD && V.y < D.cap) {
+            h = V.y;
+            V = ld_u4(&D.T[h].v);
+          }
+          if (V.x < D.nv && D.vcloud[V.x] == c) t = h;
+        }
+      }
+      if (t == NONE) t = D.centry[c];
+      const uint32_t lt = walk_to(D, t, p, D.pts[p], steps);
+      D.loc[p] = lt;
+      D.bigflag[p] = 0;
+      cast_vote(D, p, lt);
+    }
+  }
   for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < R.n_active; i0 += gridDim.x * blockDim.x) {
     uint32_t i = i0 + threadIdx.x;
     bool keep = false;
@@ -2035,26 +2080,24 @@ __global__ void __launch_bounds__(512, WTET_RELOC_MINB) k_relocate(Dev D) {
       uint32_t L = D.loc[p];
       uint32_t t = L & ~INS_BIT;
       if (t >= D.cap) {
-        atomicOr(&D.ctr->err, kErrGuard);
+        atomicOr(&D.tot->err, kErrGuard);
         t = 0;
         L |= INS_BIT;
       }
       if (!(L & INS_BIT)) {
         keep = true;
         if (D.bigflag[p] & kPending) D.bigflag[p] &= uint8_t(~kPending);
-        const uint4 V = D.T[t].v;
+        const uint4 V = ld_u4(&D.T[t].v);
+        const unsigned long long cc = __ldcg(&D.T[t].cav);
         uint32_t from = NONE;
         if (V.x == DEAD) {
           from = V.y;  // retired: walk from a new tet on one of its faces
-        } else {
+        } else if (this_round(R, cc)) {
           // retired and overwritten by a star in place: t held a cavity tet
           // of a winner that inserted (its claim is this round's), and now
           // holds a tet of that winner's star, which covers the point
-          const unsigned long long cc = __ldcg(&D.T[t].cav);
-          if (this_round(R, cc)) {
-            const uint32_t q = key_owner(R, cc);
-            if (q < D.nv && D.stat[q].ins == uint16_t(R.round)) from = t;
-          }
+          const uint32_t q = key_owner(R, cc);
+          if (q < D.nv && D.stat[q].ins == uint16_t(R.round)) from = t;
         }
         if (from != NONE) {
           const uint32_t lt = walk_to(D, from, p, D.pts[p], steps);
@@ -2063,102 +2106,167 @@ __global__ void __launch_bounds__(512, WTET_RELOC_MINB) k_relocate(Dev D) {
         }
       }
     }
-    uint32_t slot = warp_append(&D.ctr->n_next, keep);
+    const uint32_t slot = ns.total + warp_append(&R.ctr->n_next, keep);
     if (keep) R.active_next[slot] = p;
   }
-  if (steps) atomicAdd(&D.ctr->walk_steps, (unsigned long long)steps);
+  if (steps) atomicAdd(&D.tot->walk_steps, (unsigned long long)steps);
   // recycled slots not handed out this round (k_write has appended this
   // round's retired tets in front of them)
-  const uint32_t used = __ldcg(&D.ctr->alloc_used);
+  const uint32_t used = __ldcg(&R.ctr->alloc_used);
   if (R.n_freed_prev > used) {
-    const uint32_t nfn = __ldcg(&D.ctr->n_freed_next);
+    const uint32_t nfn = __ldcg(&R.ctr->n_freed_next);
     const uint32_t left = R.n_freed_prev - used;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < left; i += gridDim.x * blockDim.x)
       R.freed_next[nfn + i] = R.freed_prev[used + i];
   }
 }
 
-// Start of a round (device side, one thread): locate the next stratum once
-// the current one has thinned to 1/2^overlap_shift of its size, stop when
-// nothing is left, reset the per-round counters.
-__device__ void begin_round(const Dev& D) {
-  State* S = D.st;
-  if (S->done || S->stop) return;
-  S->act_total = 0;
-  while (S->next_level >= 0 &&
-         (S->n_active == 0 || (uint64_t(S->n_active) << S->overlap_shift) <= S->stratum_size)) {
-    const int L = S->next_level--;
-    const uint32_t total = D.lvl_total[L];
-    if (total == 0) continue;
-    S->act_level = uint32_t(L);
-    S->act_total = total;
-    S->act_base = S->n_active;
-    S->n_active += total;
-    S->stratum_size = total;
-    S->strata += 1;
-    break;
-  }
-  if (S->n_active == 0) {
-    S->done = 1;
+// Starts the next round (one thread): stop when nothing is left.
+__device__ __forceinline__ void start_round(const Dev& D, State& S) {
+  S.flags = 0;
+  if (S.n_active == 0 && S.next_level < 0) {
+    S.done = 1;
     return;
   }
-  S->round += 1;
-  if (S->round > S->max_rounds) {
-    S->stop = 3;
+  S.round += 1;
+  if (S.round > S.max_rounds) {
+    S.stop = 3;
     return;
   }
-  Counters* C = D.ctr;
-  C->n_next = 0;
-  C->n_cand = 0;
-  C->pool_used = 0;
-  C->alloc_used = 0;
-  C->n_freed_next = 0;
-  C->big_used = 0;
-  C->n_inserted = 0;
-  C->huge_used = 0;
-  C->nbigw = 0;
-  C->work[0] = C->work[1] = C->work[2] = C->work[3] = 0;
-  for (uint32_t b = 0; b <= kOrderBuckets; ++b) C->sbc[b] = 0;
+  // A round belongs to k_rounds while it and the stratum that may join it next
+  // are small; the learned scheduler serves it while it and the next two
+  // strata (each about doubles the previous one) hold at most learned_points.
+  uint64_t up = S.n_active;
+  if (S.next_level >= 0) up += D.lvl_total[S.next_level];
+  if (up <= D.small_points) S.flags |= kSmallRound;
+  if (S.next_level >= 1) up += D.lvl_total[S.next_level - 1];
+  if (D.mlp && up <= D.learned_points) S.flags |= kLearnedRound;
 }
 
-// The first round's start (later rounds are started by k_end).
-__global__ void k_begin(Dev D) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  begin_round(D);
-}
-
-// End of a round: advance the slot top, swap the lists, stop on errors; then
-// start the next round, so that a round is one kernel shorter.
-__global__ void k_end(Dev D) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  State* S = D.st;
-  if (S->done || S->stop) return;
-  Counters* C = D.ctr;
-  if (C->err & ~uint32_t(kErrCapacity)) {
-    S->stop = 1;
+// Ends a round (one thread, after every other thread's last write of the
+// round): advance the slot top, swap the lists, stop on errors; then start the
+// next one.
+__device__ __forceinline__ void end_round(const Dev& D, State& S, const Counters* C, const NextStratum& ns) {
+  const uint32_t err = __ldcg(&C->err);
+  if (err & ~uint32_t(kErrCapacity)) {
+    S.stop = 1;
     return;
   }
-  const uint32_t used = C->alloc_used;
-  const uint32_t fresh = used > S->n_freed_prev ? used - S->n_freed_prev : 0u;
-  const uint32_t left = S->n_freed_prev > used ? S->n_freed_prev - used : 0u;
+  const uint32_t used = __ldcg(&C->alloc_used);
+  const uint32_t fresh = used > S.n_freed_prev ? used - S.n_freed_prev : 0u;
+  const uint32_t left = S.n_freed_prev > used ? S.n_freed_prev - used : 0u;
   // Winners that ran out of capacity reserved slot ranges they never wrote;
   // every written slot lies below the capacity, so the top never passes it
   // (the slots between are left dead).
-  S->tet_top = uint32_t(min(uint64_t(S->tet_top) + fresh, uint64_t(D.cap)));
-  S->n_freed_prev = C->n_freed_next + left;
-  S->par ^= 1u;
-  S->n_active = C->n_next;
-  S->inserted += C->n_inserted;
-  S->starts += C->big_used + min(C->huge_used, HUGE_SLOTS);
-  S->last_starts = C->big_used;
-  S->last_cand = C->n_cand;
-  S->last_inserted = C->n_inserted;
-  S->last_alloc = C->alloc_used;
-  if (C->err & kErrCapacity) {
-    S->stop = 2;
+  S.tet_top = uint32_t(min(uint64_t(S.tet_top) + fresh, uint64_t(D.cap)));
+  S.n_freed_prev = __ldcg(&C->n_freed_next) + left;
+  S.par ^= 1u;
+  S.n_active = __ldcg(&C->n_next) + ns.total;
+  S.next_level = ns.next;
+  if (ns.total) {
+    S.stratum_size = ns.total;
+    S.strata += 1;
+  }
+  uint32_t starts = 0;
+#pragma unroll
+  for (uint32_t b = 0; b < kOrderBuckets; ++b) starts += __ldcg(&C->sbc[b]);
+  S.inserted += __ldcg(&C->n_inserted);
+  S.starts += starts + min(__ldcg(&C->huge_used), HUGE_SLOTS);
+  S.last_starts = starts;
+  S.last_cand = __ldcg(&C->n_cand);
+  S.last_inserted = __ldcg(&C->n_inserted);
+  S.last_alloc = used;
+  if (err & kErrCapacity) {
+    S.stop = 2;
     return;
   }
-  begin_round(D);
+  start_round(D, S);
+}
+
+// A round's last kernel; its last block ends the round.
+__global__ void __launch_bounds__(512, WTET_RELOC_MINB) k_relocate(Dev D) {
+  const RoundArgs R = load_round(D);
+  if (!R.live) return;
+  const NextStratum ns = next_stratum(D, __ldcg(&D.st->next_level), __ldcg(&D.st->stratum_size),
+                                      __ldcg(&D.st->overlap_shift), R.n_active, __ldcg(&R.ctr->n_inserted));
+  relocate_body(D, R, ns);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(&R.ctr->ticket, 1u) == gridDim.x - 1) {
+    __threadfence();
+    R.ctr->err = *reinterpret_cast<volatile uint32_t*>(&D.tot->err);
+    __threadfence();
+    end_round(D, *D.st, R.ctr, ns);
+  }
+}
+
+// Resumes after the host has grown the tet arrays: the stopped round did not
+// start its successor.
+__global__ void k_begin(Dev D) {
+  if (threadIdx.x == 0 && blockIdx.x == 0) start_round(D, *D.st);
+}
+
+// ---- small rounds: many of them inside one kernel --------------------------
+//
+// A round of a few thousand points is a chain of dependent trips through five
+// passes; launched one by one, the gaps between the kernels and the cold start
+// of each cost more than the passes.  k_rounds runs such rounds in one
+// thread-block cluster (16 SMs, or 8 where the device has no room for 16):
+// the passes are separated by the cluster's hardware barrier, each block keeps
+// the round state in its own shared memory and derives the next round's from
+// the counters, and the kernel returns when a round is too large for it or the
+// job is done.
+constexpr uint32_t kRoundThreads = 512;
+constexpr uint32_t kRoundWarps = kRoundThreads / 32;
+union RoundSmem {
+  BfsSmem<kRoundWarps> bfs;
+  WriteSmem<kRoundWarps> write;
+  CandSmem<kRoundWarps> cand;
+};
+
+__device__ __forceinline__ void cluster_barrier() {
+  __syncthreads();
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+template <bool kLearned>
+__global__ void __launch_bounds__(kRoundThreads, 1) k_rounds(Dev D) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  RoundSmem& sm = *reinterpret_cast<RoundSmem*>(smem_raw);
+  mlp::Smem* net = kLearned ? reinterpret_cast<mlp::Smem*>(smem_raw + sizeof(RoundSmem)) : nullptr;
+  __shared__ State S;
+  for (uint32_t i = threadIdx.x; i < sizeof(State) / 4; i += kRoundThreads)
+    reinterpret_cast<uint32_t*>(&S)[i] = __ldcg(reinterpret_cast<const uint32_t*>(D.st) + i);
+  if (kLearned) mlp::load_image(*net, D.mlp);
+  // every block has read the state before the first one may write it back
+  cluster_barrier();
+  bool ran = false;
+  for (;;) {
+    const RoundArgs R = round_args(D, reinterpret_cast<const uint4*>(&S)[0], reinterpret_cast<const uint4*>(&S)[1]);
+    if (!R.live || !(R.flags & kSmallRound)) break;  // the same in every block
+    ran = true;
+    if (kLearned && (R.flags & kLearnedRound)) cands_body<kLearned, kRoundWarps>(D, R, net, &sm.cand);
+    else cands_body<false, 1>(D, R, nullptr, nullptr);
+    cluster_barrier();
+    bfs_body<kRoundWarps>(D, R, sm.bfs);
+    cluster_barrier();
+    shared_body<kRoundWarps>(D, R);
+    cluster_barrier();
+    write_body<kRoundWarps>(D, R, sm.write);
+    cluster_barrier();
+    const NextStratum ns =
+        next_stratum(D, S.next_level, S.stratum_size, S.overlap_shift, R.n_active, __ldcg(&R.ctr->n_inserted));
+    relocate_body(D, R, ns);
+    // The error flags are read once for all blocks, so that all of them take
+    // the same decision (a later flag is seen a round later).
+    if (blockIdx.x == 0 && threadIdx.x == 0) R.ctr->err = *reinterpret_cast<volatile uint32_t*>(&D.tot->err);
+    cluster_barrier();
+    if (threadIdx.x == 0) end_round(D, S, R.ctr, ns);
+    __syncthreads();
+  }
+  if (ran && blockIdx.x == 0)
+    for (uint32_t i = threadIdx.x; i < sizeof(State) / 4; i += kRoundThreads)
+      reinterpret_cast<uint32_t*>(D.st)[i] = reinterpret_cast<const uint32_t*>(&S)[i];
 }
 
 // ------------------------------------------------------ predicate check ----
@@ -2198,7 +2306,7 @@ __global__ void k_count(Dev D, uint32_t tet_top, uint32_t* ccount, uint32_t* hul
       if (comp(N, f) == NONE) {
         uint32_t h = atomicAdd(&hullcnt[c], 1u);
         if (h < 4) hull[4 * c + h] = make_uint2(t, uint32_t(f));
-        else atomicOr(&D.ctr->err, kErrHull);
+        else atomicOr(&D.tot->err, kErrHull);
       }
     }
   }
@@ -2233,7 +2341,7 @@ __global__ void k_emit(Dev D, uint32_t tet_top, const uint32_t* newid, const uin
     for (int f = 0; f < 4; ++f) {
       uint32_t nb = comp(N, f);
       if (nb != NONE && (nb >> 2) >= tet_top) {
-        atomicOr(&D.ctr->err, kErrGuard);
+        atomicOr(&D.tot->err, kErrGuard);
         nb = NONE;
       }
       set_comp(oa, f, nb == NONE ? NONE : ((newid[nb >> 2] << 5) | (nb & 3)));
@@ -2250,7 +2358,7 @@ __global__ void k_infinity(Dev D, const CloudInfo* ci, uint32_t nc, const uint32
   uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nc) return;
   if (hullcnt[c] != 4) {
-    atomicOr(&D.ctr->err, kErrHull);
+    atomicOr(&D.tot->err, kErrHull);
     return;
   }
   const uint32_t inf = ci[c].n + 4;
@@ -2361,6 +2469,7 @@ struct Workspace {
   DBuf<uint32_t> lvl_total;
   DBuf<State> state;
   DBuf<Counters> ctr;
+  DBuf<Totals> tot;
   DBuf<uint32_t> ccount, hullcnt, cfill, newid;
   DBuf<uint2> hull;
   DBuf<uint64_t> coff;
@@ -2370,7 +2479,8 @@ struct Workspace {
   DBuf<uint8_t> losses;
   DBuf<uint16_t> prio;
   std::vector<DBuf<uint32_t>> scan_tmp;
-  Counters* h_ctr = nullptr;
+  Totals* h_tot = nullptr;  // pinned: the totals and the state at the last host check
+  State* h_state = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaStream_t stream = nullptr;
   int device = -1;
@@ -2391,7 +2501,8 @@ Workspace& ws() {
   if (tl_ws->device != dev) {
     tl_ws->device = dev;
   }
-  if (!tl_ws->h_ctr) ck(cudaMallocHost(&tl_ws->h_ctr, sizeof(Counters)), "cudaMallocHost counters");
+  if (!tl_ws->h_tot) ck(cudaMallocHost(&tl_ws->h_tot, sizeof(Totals)), "cudaMallocHost totals");
+  if (!tl_ws->h_state) ck(cudaMallocHost(&tl_ws->h_state, sizeof(State)), "cudaMallocHost state");
   if (!tl_ws->ev0) {
     ck(cudaEventCreate(&tl_ws->ev0), "event");
     ck(cudaEventCreate(&tl_ws->ev1), "event");
@@ -2443,13 +2554,14 @@ void release_thread_workspace() {
   
   w.centry.release(); w.active.release(); w.active_next.release(); w.cand.release();
   w.cand_bf.release(); w.cwin.release(); w.stat.release(); w.bigw.release(); w.bigcand.release(); w.starts.release(); w.wscratch.release(); w.pool.release(); w.big.release();
-  w.freed_a.release(); w.freed_b.release(); w.lvl_off.release(); w.lvl_total.release(); w.state.release(); w.ctr.release();
+  w.freed_a.release(); w.freed_b.release(); w.lvl_off.release(); w.lvl_total.release(); w.state.release(); w.ctr.release(); w.tot.release();
   w.ccount.release(); w.hullcnt.release(); w.cfill.release(); w.newid.release();
   w.hull.release(); w.coff.release(); w.out_t.release(); w.out_a.release(); w.dtab.release(); w.dup.release();
   w.etab.release(); w.btab.release();
   w.log_pslot.release(); w.losses.release(); w.prio.release();
   for (auto& b : w.scan_tmp) b.release();
-  if (w.h_ctr) cudaFreeHost(w.h_ctr);
+  if (w.h_tot) cudaFreeHost(w.h_tot);
+  if (w.h_state) cudaFreeHost(w.h_state);
   if (w.ev0) cudaEventDestroy(w.ev0);
   if (w.ev1) cudaEventDestroy(w.ev1);
   if (w.stream) cudaStreamDestroy(w.stream);
@@ -2598,7 +2710,8 @@ void reserve_stack_once() {
   if (dev < 0 || dev >= 64 || done[dev]) return;
   size_t need = 0;
   const void* ks[] = {(const void*)k_bfs, (const void*)k_shared,
-                      (const void*)k_relocate, (const void*)k_activate, (const void*)k_init_clouds};
+                      (const void*)k_relocate, (const void*)k_rounds<false>, (const void*)k_rounds<true>,
+                      (const void*)k_init_clouds};
   for (const void* k : ks) {
     cudaFuncAttributes a{};
     if (cudaFuncGetAttributes(&a, k) == cudaSuccess) need = std::max<size_t>(need, a.localSizeBytes);
@@ -2609,6 +2722,52 @@ void reserve_stack_once() {
   if (cur < want) ck(cudaDeviceSetLimit(cudaLimitStackSize, want), "cudaDeviceSetLimit(stack)");
   done[dev] = true;
 }
+
+namespace {
+// Launches k_rounds as one cluster of 16 blocks, or of 8 where the device
+// cannot place 16 (decided once per device).
+void launch_small_rounds(const Dev& D, bool learned, cudaStream_t s) {
+  static std::mutex mu;
+  static uint32_t width[64] = {};
+  const size_t bytes = sizeof(RoundSmem) + (learned ? sizeof(mlp::Smem) : 0);
+  void (*k)(Dev) = learned ? k_rounds<true> : k_rounds<false>;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(kRoundThreads);
+  cfg.dynamicSmemBytes = bytes;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  int dev = 0;
+  ck(cudaGetDevice(&dev), "cudaGetDevice");
+  uint32_t w = 0;
+  {
+    std::lock_guard<std::mutex> g(mu);
+    uint32_t& slot = width[dev & 63];
+    if (slot == 0 || dev >= 64) {
+      const size_t most = sizeof(RoundSmem) + sizeof(mlp::Smem);
+      for (void (*f)(Dev) : {k_rounds<false>, k_rounds<true>}) {
+        ck(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most)), "small-round memory");
+        ck(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "small-round cluster");
+      }
+      slot = 8;
+      cudaLaunchConfig_t probe = cfg;
+      probe.gridDim = dim3(16);
+      probe.dynamicSmemBytes = most;
+      at.val.clusterDim.x = 16;
+      int fit = 0;
+      if (cudaOccupancyMaxActiveClusters(&fit, k_rounds<true>, &probe) == cudaSuccess && fit >= 1) slot = 16;
+      else (void)cudaGetLastError();
+    }
+    w = slot;
+  }
+  at.val.clusterDim.x = w;
+  cfg.gridDim = dim3(w);
+  ck(cudaLaunchKernelEx(&cfg, k, D), "small rounds");
+}
+}  // namespace
 
 JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t capacity) {
   reserve_stack_once();
@@ -2692,7 +2851,8 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
       std::min<uint64_t>(std::max<uint64_t>(n * pool_factor, 1 << 16) + 4 * n + 4096, 1ull << 30));
   W.pool.reserve(pool_cap, "pool");
   W.big.reserve(size_t(HUGE_SLOTS) * HUGE_CAP, "big");
-  W.ctr.reserve(1, "counters");
+  W.ctr.reserve(2, "counters");
+  W.tot.reserve(1, "totals");
   W.lvl_off.reserve(size_t(maxtop + 1) * (nc + 1), "levels");
   W.lvl_total.reserve(maxtop + 1, "levels");
   W.state.reserve(1, "state");
@@ -2716,7 +2876,8 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
   ck(cudaMemsetAsync(W.mx.p, 0x00, 3ull * nc * 4, s), "memset");
   ck(cudaMemsetAsync(W.hist.p, 0, (buckets + 1) * 4, s), "memset");
   ck(cudaMemsetAsync(W.stat.p, 0, nv * sizeof(Stat), s), "memset");
-  ck(cudaMemsetAsync(W.ctr.p, 0, sizeof(Counters), s), "memset");
+  ck(cudaMemsetAsync(W.ctr.p, 0, 2 * sizeof(Counters), s), "memset");
+  ck(cudaMemsetAsync(W.tot.p, 0, sizeof(Totals), s), "memset");
   k_init_slots<<<blocks_for(cap, 256, 148 * 16), 256, 0, s>>>(W.T.p, 0, cap);
   if (vmode) {
     W.losses.reserve(nv, "losses");
@@ -2729,6 +2890,11 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
   if (vmode == 1) W.prio.reserve(nv, "claim priorities");
   // Rounds whose graph may see at most this many uninserted points use the
   // learned scheduler (its training log records the same rounds).
+  const char* tr = getenv("WTET_TRACE");
+  const int trace = tr ? atoi(tr) : 0;
+  // Rounds of at most this many points run inside k_rounds (the training log
+  // has a kernel of its own between the passes, the trace times every round).
+  const uint32_t small_points = vmode == 2 || trace ? 0u : WTET_SMALL_ROUND_POINTS;
   const uint64_t learned_points = uint64_t(cfg.learned_gate ? cfg.learned_gate : 2048u) * 1024u;
 
   Dev D{};
@@ -2742,7 +2908,7 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
     D.start_rc = uint32_t(start_rc); D.start_ovf = uint32_t(start_ovf);
     D.etab = W.etab.p; D.etab_warps = etab_warps; D.btab = W.btab.p;
     D.prefilter = cfg.candidate_filter == 2 ? 0u : 1u; D.pool = W.pool.p; D.pool_cap = pool_cap; D.big = W.big.p;
-    D.ctr = W.ctr.p;
+    D.ctr = W.ctr.p; D.tot = W.tot.p; D.small_points = small_points;
     D.st = W.state.p; D.act[0] = W.active.p; D.act[1] = W.active_next.p;
     D.freed[0] = W.freed_a.p; D.freed[1] = W.freed_b.p; D.ci = W.ci.p; D.lvl_off = W.lvl_off.p;
     D.lvl_total = W.lvl_total.p; D.nc = nc;
@@ -2773,14 +2939,14 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
   hmask -= 1;
   ck(cudaMemsetAsync(W.dtab.p, 0xFF, size_t(hmask + 1) * 4, s), "memset");
   k_dedup_insert<<<nb, T, 0, s>>>(W.off.p, nc, n, W.tmp.p, W.dtab.p, hmask);
-  k_dedup_mark<<<nb, T, 0, s>>>(W.off.p, nc, n, W.tmp.p, W.dtab.p, hmask, W.dup.p, &W.ctr.p->huge_used);
+  k_dedup_mark<<<nb, T, 0, s>>>(W.off.p, nc, n, W.tmp.p, W.dtab.p, hmask, W.dup.p, &W.tot.p->ndup);
   uint64_t launches = 7;  // bbox, normalize, dedup x2, scatter, init, plus the scan below
   launches += scan_u32(W.hist.p, uint32_t(buckets + 1), s, W.scan_tmp);
   k_scatter_points<<<nb, T, 0, s>>>(W.off.p, W.ci.p, nc, n, W.tmp.p, W.bucket.p, W.hist.p, W.dup.p, D);
   k_init_clouds<<<(nc + 127) / 128, 128, 0, s>>>(W.ci.p, nc, D);
   ck(cudaGetLastError(), "setup kernels");
   uint32_t ndup = 0;
-  ck(cudaMemcpyAsync(&ndup, &W.ctr.p->huge_used, 4, cudaMemcpyDeviceToHost, s), "d2h");
+  ck(cudaMemcpyAsync(&ndup, &W.tot.p->ndup, 4, cudaMemcpyDeviceToHost, s), "d2h");
   ck(cudaStreamSynchronize(s), "dedup");
   if (ndup) {
     std::vector<uint8_t> flags(n);
@@ -2808,8 +2974,6 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
   // (the claim key holds a 16-bit round stamp)
   const uint32_t max_rounds = uint32_t(std::min<uint64_t>(
       uint64_t(std::max<uint32_t>(job.cfg.max_insert_iterations, 1u)) * (maxtop + 1), 65000ull));
-  const char* tr = getenv("WTET_TRACE");
-  const int trace = tr ? atoi(tr) : 0;
   const uint32_t TB = (cfg.block_size == 128 || cfg.block_size == 512) ? cfg.block_size : 256u;
 
   // ---- the round loop, driven from device state and replayed from a graph ----
@@ -2822,80 +2986,33 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
   S0.max_rounds = max_rounds;
   S0.overlap_shift = std::min<uint32_t>(cfg.overlap_shift, 16u);
   ck(cudaMemcpyAsync(W.state.p, &S0, sizeof(State), cudaMemcpyHostToDevice, s), "h2d");
-  ck(cudaMemsetAsync(W.ctr.p, 0, sizeof(Counters), s), "memset");
 
-  // Every round kernel loops grid-stride over its work, so each gets exactly
-  // one full wave of resident blocks: an idle round then costs one short
-  // wave per kernel.
-  struct Grids {
-    uint32_t act, vote, cand, candl, logf, bfs, sh, wr, rel;
+  // Every kernel of a large round loops grid-stride over its work, so each gets
+  // exactly one full wave of resident blocks: an idle round then costs one
+  // short wave per kernel.
+  const uint32_t g_cand = wave(k_cands, TB), g_candl = vmode == 1 ? wave(k_cands_learned, 256) : 0u;
+  const uint32_t g_log = wave(k_log_features, TB), g_bfs = wave(k_bfs, 128), g_sh = wave(k_shared, 128);
+  const uint32_t g_wr = wave(k_write, 128), g_rel = wave(k_relocate, TB);
+  const uint64_t kernels_per_round = 5 + (vmode == 2 ? 1 : 0);
+  auto enqueue_round = [&]() {
+    if (vmode == 1) k_cands_learned<<<g_candl, 256, 0, s>>>(D);
+    else k_cands<<<g_cand, TB, 0, s>>>(D);
+    if (vmode == 2) k_log_features<<<g_log, TB, 0, s>>>(D);
+    k_bfs<<<g_bfs, 128, 0, s>>>(D);
+    k_shared<<<g_sh, 128, 0, s>>>(D);
+    k_write<<<g_wr, 128, 0, s>>>(D);
+    k_relocate<<<g_rel, TB, 0, s>>>(D);
   };
-  const Grids big{wave(k_activate, TB), 0u,      wave(k_cands, TB),
-                  vmode == 1 ? wave(k_cands_learned, 256) : 0u,
-                  wave(k_log_features, TB), wave(k_bfs, 128), wave(k_shared, 128),
-                  wave(k_write, 128),  wave(k_relocate, TB)};
-  // Rounds of the first strata have a few thousand points: a full wave of
-  // blocks that exit at once costs more than their work, so those rounds
-  // replay a graph with one block per SM.
-  auto shrink = [](uint32_t g) { return std::min<uint32_t>(g, 148u); };
-  const Grids small{shrink(big.act), 0u, shrink(big.cand), shrink(big.candl), shrink(big.logf),
-                    shrink(big.bfs), shrink(big.sh),   shrink(big.wr),    shrink(big.rel)};
-  const uint64_t kernels_per_round = 7 + (vmode == 2 ? 1 : 0);
-
-  // One round: k_end also starts the next round (k_begin starts the first).
-  // `learned`: the learned scheduler's candidate kernel.
-  auto enqueue_round = [&](const Grids& G, bool learned) {
-    k_activate<<<G.act, TB, 0, s>>>(D);
-    if (learned) k_cands_learned<<<G.candl, 256, 0, s>>>(D);
-    else k_cands<<<G.cand, TB, 0, s>>>(D);
-    if (vmode == 2) k_log_features<<<G.logf, TB, 0, s>>>(D);
-    k_bfs<<<G.bfs, 128, 0, s>>>(D);
-    k_shared<<<G.sh, 128, 0, s>>>(D);
-    k_write<<<G.wr, 128, 0, s>>>(D);
-    k_relocate<<<G.rel, TB, 0, s>>>(D);
-    k_end<<<1, 32, 0, s>>>(D);
-  };
-  // Rounds per host check (the graph holds this many rounds).
+  // Rounds per host check.  Kernels of a finished job, and of rounds that
+  // belong to k_rounds, return at once.
   uint32_t rpg = std::min<uint32_t>(cfg.rounds_per_graph, 64u);
   if (trace) rpg = 1;
-  // Three graphs: the first strata's rounds (one block per SM), the bulk
-  // rounds (full waves), and with the learned scheduler the rounds in between
-  // (full waves, learned candidate kernel).
-  cudaGraphExec_t gexec = nullptr, gexec_small = nullptr, gexec_mid = nullptr;
-  auto capture = [&](const Grids& G, bool learned) {
-    cudaGraph_t g = nullptr;
-    cudaGraphExec_t e = nullptr;
-    ck(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "begin capture");
-    for (uint32_t r = 0; r < rpg; ++r) enqueue_round(G, learned);
-    ck(cudaStreamEndCapture(s, &g), "end capture");
-    ck(cudaGraphInstantiate(&e, g, 0), "graph instantiate");
-    cudaGraphDestroy(g);
-    return e;
-  };
-  auto destroy_graphs = [&]() {
-    if (gexec) cudaGraphExecDestroy(gexec);
-    if (gexec_small) cudaGraphExecDestroy(gexec_small);
-    if (gexec_mid) cudaGraphExecDestroy(gexec_mid);
-    gexec = gexec_small = gexec_mid = nullptr;
-  };
-  auto build_graph = [&]() {
-    destroy_graphs();
-    gexec = capture(big, false);
-    gexec_small = capture(small, vmode == 1);
-    if (vmode == 1) gexec_mid = capture(big, true);
-  };
-  // Points the next graph launch may see: the current list and the next two
-  // strata (each stratum about doubles the previous one).
-  auto upcoming = [&](const State& h) {
-    uint64_t u = h.n_active;
-    for (int L = h.next_level, k = 0; L >= 0 && k < 2; --L, ++k) u += lvl_total[L];
-    return u;
-  };
-  constexpr uint64_t kSmallRoundPoints = WTET_SMALL_ROUND_POINTS;
-  build_graph();
-  k_begin<<<1, 32, 0, s>>>(D);
+  // The first launch locates the first stratum ("round 0": nothing to insert).
+  k_relocate<<<g_rel, TB, 0, s>>>(D);
   launches += 1;
-  State hs = S0;
+  State& hs = *W.h_state;
+  hs = S0;
+  hs.flags = small_points ? kSmallRound : 0u;
   cudaEvent_t tr0 = nullptr, tr1 = nullptr;  // per-round device time when tracing
   if (trace) {
     ck(cudaEventCreate(&tr0), "event");
@@ -2903,16 +3020,20 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
   }
   for (;;) {
     if (trace) ck(cudaEventRecord(tr0, s), "event record");
-    const uint64_t u = upcoming(hs);
-    ck(cudaGraphLaunch(u <= kSmallRoundPoints ? gexec_small : (gexec_mid && u <= learned_points) ? gexec_mid : gexec,
-                       s),
-       "graph launch");
+    if (!(hs.flags & kSmallRound)) {
+      for (uint32_t r = 0; r < rpg; ++r) enqueue_round();
+      launches += uint64_t(rpg) * kernels_per_round;
+    }
+    if (small_points) {
+      launch_small_rounds(D, vmode == 1, s);
+      launches += 1;
+    }
+    ck(cudaGetLastError(), "round kernels");
     if (trace) ck(cudaEventRecord(tr1, s), "event record");
-    launches += uint64_t(rpg) * kernels_per_round;
     ck(cudaMemcpyAsync(&hs, W.state.p, sizeof(State), cudaMemcpyDeviceToHost, s), "d2h");
-    ck(cudaMemcpyAsync(W.h_ctr, W.ctr.p, sizeof(Counters), cudaMemcpyDeviceToHost, s), "d2h");
+    ck(cudaMemcpyAsync(W.h_tot, W.tot.p, sizeof(Totals), cudaMemcpyDeviceToHost, s), "d2h");
     ck(cudaStreamSynchronize(s), "rounds");
-    const Counters& h = *W.h_ctr;
+    const Totals& h = *W.h_tot;
     if (trace) {
       float rms = 0.f;
       cudaEventElapsedTime(&rms, tr0, tr1);
@@ -2923,13 +3044,11 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
               hs.last_inserted, (unsigned long long)h.n_big, hs.last_alloc, hs.tet_top, h.err, rms);
     }
     if (hs.stop == 1) {
-      destroy_graphs();
       char buf[160];
       snprintf(buf, sizeof buf, "device consistency check failed (flags 0x%x) in round %u", h.err, hs.round);
       throw Error{(h.err & kErrPrec) ? WTET_ERR_PRECISION : WTET_ERR_INTERNAL, buf};
     }
     if (hs.stop == 3) {
-      destroy_graphs();
       throw Error{WTET_ERR_NO_CONVERGE, "insertion did not converge within max_insert_iterations"};
     }
     if (hs.stop == 2) {
@@ -2947,27 +3066,24 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
       refresh();
       hs.stop = 0;
       ck(cudaMemcpyAsync(W.state.p, &hs, sizeof(State), cudaMemcpyHostToDevice, s), "h2d");
-      uint32_t zero = 0;
-      ck(cudaMemcpyAsync(&W.ctr.p->err, &zero, 4, cudaMemcpyHostToDevice, s), "clear err");
+      ck(cudaMemsetAsync(&W.tot.p->err, 0, 4, s), "clear err");
       ck(cudaStreamSynchronize(s), "grow");
-      build_graph();
       k_begin<<<1, 32, 0, s>>>(D);  // the stopped round did not start its successor
       launches += 1;
       continue;
     }
     if (hs.done) break;
   }
-  destroy_graphs();
   if (tr0) cudaEventDestroy(tr0);
   if (tr1) cudaEventDestroy(tr1);
   const uint32_t tet_top = hs.tet_top;
   const uint32_t round = hs.round;
   st.strata = hs.strata;
   st.inserted = hs.inserted;
-  st.walk_steps = W.h_ctr->walk_steps;
-  st.candidates = W.h_ctr->n_expanded;
-  st.big_cavities = W.h_ctr->n_big;
-  st.tets_created = W.h_ctr->created;
+  st.walk_steps = W.h_tot->walk_steps;
+  st.candidates = W.h_tot->n_expanded;
+  st.big_cavities = W.h_tot->n_big;
+  st.tets_created = W.h_tot->created;
   st.rounds = round;
   st.vote_winners = hs.starts;
   res.logged = std::min<uint64_t>(hs.log_used, job.log_cap);
@@ -3000,11 +3116,11 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
     ck(cudaGetLastError(), "output kernels");
   }
   ck(cudaEventRecord(W.ev1, s), "event record");
-  ck(cudaMemcpyAsync(W.h_ctr, W.ctr.p, sizeof(Counters), cudaMemcpyDeviceToHost, s), "d2h");
+  ck(cudaMemcpyAsync(W.h_tot, W.tot.p, sizeof(Totals), cudaMemcpyDeviceToHost, s), "d2h");
   ck(cudaStreamSynchronize(s), "output");
-  if (W.h_ctr->err) {
+  if (W.h_tot->err) {
     char buf[128];
-    snprintf(buf, sizeof buf, "device consistency check failed in output (flags 0x%x)", W.h_ctr->err);
+    snprintf(buf, sizeof buf, "device consistency check failed in output (flags 0x%x)", W.h_tot->err);
     throw Error{WTET_ERR_INTERNAL, buf};
   }
   float ms = 0.f;
@@ -3108,37 +3224,37 @@ void check_quality_device(const float* d_xyz, uint64_t n, const uint32_t* d_tets
   W.mn.reserve(3, "bbox");
   W.mx.reserve(3, "bbox");
   W.tmp.reserve(n, "tmp");
-  W.ctr.reserve(1, "ctr");
+  W.tot.reserve(1, "totals");
   uint64_t offs[2] = {0, n};
   ck(cudaMemcpyAsync(W.off.p, offs, 16, cudaMemcpyHostToDevice, s), "h2d");
   ck(cudaMemsetAsync(W.mn.p, 0xFF, 12, s), "memset");
   ck(cudaMemsetAsync(W.mx.p, 0, 12, s), "memset");
-  ck(cudaMemsetAsync(W.ctr.p, 0, sizeof(Counters), s), "memset");
+  ck(cudaMemsetAsync(W.tot.p, 0, sizeof(Totals), s), "memset");
   uint32_t nb = uint32_t((n + 255) / 256);
   k_bbox<<<nb, 256, 0, s>>>(d_xyz, W.off.p, 1, n, W.mn.p, W.mx.p);
   k_normalize_plain<<<nb, 256, 0, s>>>(d_xyz, n, W.mn.p, W.mx.p, W.tmp.p);
-  unsigned long long* out = reinterpret_cast<unsigned long long*>(&W.ctr.p->walk_steps);
+  unsigned long long* out = reinterpret_cast<unsigned long long*>(&W.tot.p->walk_steps);
   k_check_quality<<<blocks_for(m, 128, 148 * 16), 128, 0, s>>>(W.tmp.p, uint32_t(n), reinterpret_cast<const uint4*>(d_tets),
                                                                 reinterpret_cast<const uint4*>(d_adj), m, out,
-                                                                &W.ctr.p->err);
-  ck(cudaMemcpyAsync(W.h_ctr, W.ctr.p, sizeof(Counters), cudaMemcpyDeviceToHost, s), "d2h");
+                                                                &W.tot.p->err);
+  ck(cudaMemcpyAsync(W.h_tot, W.tot.p, sizeof(Totals), cudaMemcpyDeviceToHost, s), "d2h");
   ck(cudaStreamSynchronize(s), "check");
-  if (W.h_ctr->err & ~uint32_t(kErrPrec))
+  if (W.h_tot->err & ~uint32_t(kErrPrec))
     throw Error{WTET_ERR_ARG, "adjacency refers to a tet out of range"};
-  if (W.h_ctr->err & kErrPrec) throw Error{WTET_ERR_PRECISION, "exact arithmetic buffer overflow"};
-  *violations = W.h_ctr->walk_steps;
-  *interior = W.h_ctr->n_expanded;
+  if (W.h_tot->err & kErrPrec) throw Error{WTET_ERR_PRECISION, "exact arithmetic buffer overflow"};
+  *violations = W.h_tot->walk_steps;
+  *interior = W.h_tot->n_expanded;
 }
 
 void predicate_signs_device(const float* d_pts, const uint32_t* d_keys, uint64_t m, int32_t* d_o3, int32_t* d_o4,
                             cudaStream_t s) {
   Workspace& W = ws();
-  W.ctr.reserve(1, "counters");
-  ck(cudaMemsetAsync(W.ctr.p, 0, sizeof(Counters), s), "memset");
-  if (m) k_predicate_signs<<<blocks_for(m, 128, 148 * 8), 128, 0, s>>>(d_pts, d_keys, m, d_o3, d_o4, &W.ctr.p->err);
+  W.tot.reserve(1, "totals");
+  ck(cudaMemsetAsync(W.tot.p, 0, sizeof(Totals), s), "memset");
+  if (m) k_predicate_signs<<<blocks_for(m, 128, 148 * 8), 128, 0, s>>>(d_pts, d_keys, m, d_o3, d_o4, &W.tot.p->err);
   ck(cudaGetLastError(), "predicate kernel");
   uint32_t err = 0;
-  ck(cudaMemcpyAsync(&err, &W.ctr.p->err, 4, cudaMemcpyDeviceToHost, s), "d2h");
+  ck(cudaMemcpyAsync(&err, &W.tot.p->err, 4, cudaMemcpyDeviceToHost, s), "d2h");
   ck(cudaStreamSynchronize(s), "predicates");
   if (err) throw Error{WTET_ERR_PRECISION, "exact arithmetic buffer overflow"};
 }
