@@ -507,34 +507,110 @@ __device__ __forceinline__ int in_sphere(const Dev& D, const Tet* T, const float
                       V.z, V.w, p, D.sos, &D.tot->err);
 }
 
-// Visibility walk with exact orient3d + SoS from tet t to the tet containing p.
-__device__ __forceinline__ uint32_t walk_to(const Dev& D, uint32_t t, uint32_t p, const float4& pq, uint32_t& steps) {
+// Visibility walk from tet t to the tet that contains p, and p's vote there.
+//
+// A step takes one record load and all four orientation tests together: with p
+// as the base point the tests share the differences and the 2x2 minors (FP32
+// stage, Shewchuk's bound for each; the exact test with SoS decides the faces
+// it cannot), and the walk leaves through the face p is furthest beyond.  The
+// tests are independent, where four tests with an early exit were a chain.  In
+// a Delaunay triangulation a visibility walk ends whichever of the possible
+// faces it takes.
+//
+// The vote: 64-bit atomicMax of (score, ~p), so each tet's vote word names its
+// point with the largest score (ties: the smallest index).  A tet's points
+// change only when it is retired, so its vote word stays valid until then:
+// points vote when they are located or relocated, and k_write clears the word
+// of every slot it writes a new tet into.  Score (larger = inserted first):
+// circumcenter rule, the depth of p inside the circumsphere (f32 insphere from
+// the walk's minors, src/shaders/vote.wgsl:401-494 semantics); centroid rule,
+// the inverse squared distance to the centroid.
+__device__ __forceinline__ uint32_t locate(const Dev& D, uint32_t t, uint32_t p, const float4& pq, uint32_t& steps) {
   int entry = -1;
   for (uint32_t s = 0; s < WALK_LIMIT; ++s) {
     if (t >= D.cap) {
       atomicOr(&D.tot->err, kErrGuard);
       return 0;
     }
-    const uint4 V = ld_u4(&D.T[t].v), N = ld_u4(&D.T[t].n);
-    const float4 X = ld_f4(&D.T[t].X), Y = ld_f4(&D.T[t].Y), Z = ld_f4(&D.T[t].Z);
-    if (V.x >= D.nv || V.y >= D.nv || V.z >= D.nv || V.w >= D.nv) {
-      atomicOr(&D.tot->err, kErrGuard);
-      return t;
-    }
-    const float4 P0 = corner(X, Y, Z, 0), P1 = corner(X, Y, Z, 1), P2 = corner(X, Y, Z, 2), P3 = corner(X, Y, Z, 3);
+    const Tet* T = D.T + t;
+    const uint4 N = ld_u4(&T->n);
+    const float4 X = ld_f4(&T->X), Y = ld_f4(&T->Y), Z = ld_f4(&T->Z);
+    const float ax = __fsub_rn(X.x, pq.x), bx = __fsub_rn(X.y, pq.x), cx = __fsub_rn(X.z, pq.x), dx = __fsub_rn(X.w, pq.x);
+    const float ay = __fsub_rn(Y.x, pq.y), by = __fsub_rn(Y.y, pq.y), cy = __fsub_rn(Y.z, pq.y), dy = __fsub_rn(Y.w, pq.y);
+    const float az = __fsub_rn(Z.x, pq.z), bz = __fsub_rn(Z.y, pq.z), cz = __fsub_rn(Z.z, pq.z), dz = __fsub_rn(Z.w, pq.z);
+    const float axby = __fmul_rn(ax, by), bxay = __fmul_rn(bx, ay), ab = __fsub_rn(axby, bxay);
+    const float bxcy = __fmul_rn(bx, cy), cxby = __fmul_rn(cx, by), bc = __fsub_rn(bxcy, cxby);
+    const float cxdy = __fmul_rn(cx, dy), dxcy = __fmul_rn(dx, cy), cd = __fsub_rn(cxdy, dxcy);
+    const float dxay = __fmul_rn(dx, ay), axdy = __fmul_rn(ax, dy), da = __fsub_rn(dxay, axdy);
+    const float axcy = __fmul_rn(ax, cy), cxay = __fmul_rn(cx, ay), ac = __fsub_rn(axcy, cxay);
+    const float bxdy = __fmul_rn(bx, dy), dxby = __fmul_rn(dx, by), bd = __fsub_rn(bxdy, dxby);
+    // orient3d of each face's vertices and p
+    const float abc = __fadd_rn(__fsub_rn(__fmul_rn(az, bc), __fmul_rn(bz, ac)), __fmul_rn(cz, ab));
+    const float bcd = __fadd_rn(__fsub_rn(__fmul_rn(bz, cd), __fmul_rn(cz, bd)), __fmul_rn(dz, bc));
+    const float cda = __fadd_rn(__fadd_rn(__fmul_rn(cz, da), __fmul_rn(dz, ac)), __fmul_rn(az, cd));
+    const float dab = __fadd_rn(__fadd_rn(__fmul_rn(dz, ab), __fmul_rn(az, bd)), __fmul_rn(bz, da));
+    const float p_ab = __fadd_rn(fabsf(axby), fabsf(bxay)), p_bc = __fadd_rn(fabsf(bxcy), fabsf(cxby));
+    const float p_cd = __fadd_rn(fabsf(cxdy), fabsf(dxcy)), p_da = __fadd_rn(fabsf(dxay), fabsf(axdy));
+    const float p_ac = __fadd_rn(fabsf(axcy), fabsf(cxay)), p_bd = __fadd_rn(fabsf(bxdy), fabsf(dxby));
+    const float fa = fabsf(az), fb = fabsf(bz), fc = fabsf(cz), fd = fabsf(dz);
+    // out[f] > 0: p is beyond the face opposite vertex f (the tet with vertex f
+    // replaced by p has Shewchuk orient3d > 0); perm[f]: the test's permanent
+    const float out[4] = {-bcd, cda, -dab, abc};
+    const float perm[4] = {
+        __fadd_rn(__fadd_rn(__fmul_rn(p_cd, fb), __fmul_rn(p_bd, fc)), __fmul_rn(p_bc, fd)),
+        __fadd_rn(__fadd_rn(__fmul_rn(p_da, fc), __fmul_rn(p_ac, fd)), __fmul_rn(p_cd, fa)),
+        __fadd_rn(__fadd_rn(__fmul_rn(p_ab, fd), __fmul_rn(p_bd, fa)), __fmul_rn(p_da, fb)),
+        __fadd_rn(__fadd_rn(__fmul_rn(p_bc, fa), __fmul_rn(p_ac, fb)), __fmul_rn(p_ab, fc))};
     int moved = -1;
-    for (int i = 0; i < 4; ++i) {
-      const int f = (i + int(s)) & 3;
+    uint32_t unsure = 0;
+    float best = 0.f;
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
       if (f == entry) continue;
-      // the tet with vertex f replaced by p
-      if (o3d_sos_f(f == 0 ? pq : P0, f == 1 ? pq : P1, f == 2 ? pq : P2, f == 3 ? pq : P3, f == 0 ? p : V.x,
-                    f == 1 ? p : V.y, f == 2 ? p : V.z, f == 3 ? p : V.w, D.sos, &D.tot->err) == -1) {
-        moved = f;
-        break;
+      const float err = __fadd_rn(__fmul_rn(ex::kO3dBoundF, perm[f]), ex::kUnderflowSlackF);
+      const bool usable = perm[f] >= ex::kPermMinF && perm[f] < 1.0e30f;
+      if (usable && out[f] > err) {
+        if (moved < 0 || out[f] > best) {
+          moved = f;
+          best = out[f];
+        }
+      } else if (!(usable && -out[f] > err)) {
+        unsure |= 1u << f;
+      }
+    }
+    if (moved < 0 && unsure) {
+      const uint4 V = ld_u4(&T->v);
+      if (V.x >= D.nv || V.y >= D.nv || V.z >= D.nv || V.w >= D.nv) {
+        atomicOr(&D.tot->err, kErrGuard);
+        return t;
+      }
+      const float4 P0 = corner(X, Y, Z, 0), P1 = corner(X, Y, Z, 1), P2 = corner(X, Y, Z, 2), P3 = corner(X, Y, Z, 3);
+#pragma unroll 1
+      for (int f = 0; f < 4; ++f) {
+        if (!((unsure >> f) & 1u)) continue;
+        // the tet with vertex f replaced by p
+        if (o3d_sos_slow(f == 0 ? pq : P0, f == 1 ? pq : P1, f == 2 ? pq : P2, f == 3 ? pq : P3, f == 0 ? p : V.x,
+                         f == 1 ? p : V.y, f == 2 ? p : V.z, f == 3 ? p : V.w, D.sos, &D.tot->err) == -1) {
+          moved = f;
+          break;
+        }
       }
     }
     if (moved < 0) {
       steps += s + 1;
+      float score;
+      if (D.rule == 1) {
+        const float gx = 0.25f * (X.x + X.y + X.z + X.w) - pq.x, gy = 0.25f * (Y.x + Y.y + Y.z + Y.w) - pq.y,
+                    gz = 0.25f * (Z.x + Z.y + Z.z + Z.w) - pq.z;
+        score = 1.0f / (1e-30f + gx * gx + gy * gy + gz * gz);
+      } else {
+        const float al = ax * ax + ay * ay + az * az, bl = bx * bx + by * by + bz * bz;
+        const float cl = cx * cx + cy * cy + cz * cz, dl = dx * dx + dy * dy + dz * dz;
+        // tets have Shewchuk orient3d < 0, so inside means a determinant < 0
+        const float depth = -((dl * abc - cl * dab) + (bl * cda - al * bcd));
+        score = (depth > 0.f && depth < 3.0e38f) ? depth : 0.f;
+      }
+      atomicMax(&D.T[t].vote, ((unsigned long long)__float_as_uint(score) << 32) | (unsigned long long)(~p));
       return t;
     }
     const uint32_t n = comp(N, moved);
@@ -762,48 +838,6 @@ __global__ void k_init_clouds(const CloudInfo* ci, uint32_t nc, Dev D) {
 
 // ---------------------------------------------------------------- rounds ----
 
-// Vote score: larger = inserted first.  Circumcenter rule: depth of p inside
-// the circumsphere (f32 insphere, src/shaders/vote.wgsl:401-494 semantics);
-// centroid rule: inverse squared distance to the centroid.
-__device__ __forceinline__ float vote_score(const Tet& t, float4 q, int rule) {
-  const float4 X = t.X, Y = t.Y, Z = t.Z;
-  const float4 a = corner(X, Y, Z, 0), b = corner(X, Y, Z, 1), c = corner(X, Y, Z, 2), d = corner(X, Y, Z, 3);
-  if (rule == 1) {
-    float cx = 0.25f * (a.x + b.x + c.x + d.x) - q.x;
-    float cy = 0.25f * (a.y + b.y + c.y + d.y) - q.y;
-    float cz = 0.25f * (a.z + b.z + c.z + d.z) - q.z;
-    return 1.0f / (1e-30f + cx * cx + cy * cy + cz * cz);
-  }
-  float aex = a.x - q.x, aey = a.y - q.y, aez = a.z - q.z;
-  float bex = b.x - q.x, bey = b.y - q.y, bez = b.z - q.z;
-  float cex = c.x - q.x, cey = c.y - q.y, cez = c.z - q.z;
-  float dex = d.x - q.x, dey = d.y - q.y, dez = d.z - q.z;
-  float ab = aex * bey - bex * aey, bc = bex * cey - cex * bey, cd = cex * dey - dex * cey;
-  float da = dex * aey - aex * dey, ac = aex * cey - cex * aey, bd = bex * dey - dex * bey;
-  float abc = aez * bc - bez * ac + cez * ab, bcd = bez * cd - cez * bd + dez * bc;
-  float cda = cez * da + dez * ac + aez * cd, dab = dez * ab + aez * bd + bez * da;
-  float al = aex * aex + aey * aey + aez * aez, bl = bex * bex + bey * bey + bez * bez;
-  float cl = cex * cex + cey * cey + cez * cez, dl = dex * dex + dey * dey + dez * dez;
-  float det = (dl * abc - cl * dab) + (bl * cda - al * bcd);
-  float depth = -det;  // tets have Shewchuk orient3d < 0, so inside means det < 0
-  return (depth > 0.f && depth < 3.0e38f) ? depth : 0.f;
-}
-
-// The vote of uninserted point p for tet t: 64-bit atomicMax of (score, ~p),
-// so each tet's vote word names its point with the largest score (ties: the
-// smallest index).  A tet's points change only when it is retired, so its
-// vote word stays valid until then: points vote when they are located
-// (k_activate) or relocated (k_relocate), and k_write clears the word of
-// every slot it writes a new tet into.
-__device__ __forceinline__ void cast_vote(const Dev& D, uint32_t p, uint32_t t) {
-  if (t >= D.cap) {
-    atomicOr(&D.tot->err, kErrGuard);
-    return;
-  }
-  const float sc = vote_score(D.T[t], D.pts[p], D.rule);
-  atomicMax(&D.T[t].vote, ((unsigned long long)__float_as_uint(sc) << 32) | (unsigned long long)(~p));
-}
-
 // Prefix of the order buckets' start counts, in shared memory (sp has
 // kOrderBuckets + 2 entries; sp[kOrderBuckets + 1] is the total).  Called by
 // every thread of the block.
@@ -1028,11 +1062,15 @@ __global__ void __launch_bounds__(256) k_cands_learned(Dev D) {
 // marked holds the minimum claim on all its tets.  The queue and the list
 // start in shared memory and continue in the group's global region; cavities
 // beyond BIG_CAP tets move to the huge path next round.
-#ifndef WTET_BFS_LANES
-#define WTET_BFS_LANES 16
-#endif
-constexpr uint32_t kBfsLanes = WTET_BFS_LANES;
-constexpr uint32_t kWarpGroups = 32 / kBfsLanes;
+//
+// A claim's answer is not waited for: a small set of the cavity's tets in
+// shared memory tells a new tet from one already found, and the answer (a
+// better claim: lost) is looked at in the next pass, after that pass has
+// issued its loads.  Once a cavity outgrows the set, claims are waited for and
+// tell the two apart themselves.
+constexpr uint32_t kBulkLanes = 16;  // lanes per search in large rounds; k_rounds has lanes to spare and uses 32
+constexpr uint32_t kHashSlots = 128;
+constexpr uint32_t kHashTets = 64;   // largest cavity at the start of a pass that uses the set (adds at most 32)
 constexpr uint32_t kBfsShared = 48;  // queue entries (tet + neighbour words) per group in shared memory
 constexpr uint32_t kBfsFaces = 48;   // boundary faces per group in shared memory
 // A cavity of K tets joined through at least K - 1 faces has at most 2K + 2 boundary faces.
@@ -1040,11 +1078,13 @@ constexpr uint32_t kMaxFaces = 2 * BIG_CAP + 2;
 constexpr uint32_t kScratchWords = BIG_CAP + 2 * kMaxFaces;
 constexpr uint32_t kPoolChunk = 512;  // pool words a lane group reserves at a time
 
-template <uint32_t kWarps>
+template <uint32_t kWarps, uint32_t kBfsLanes>
 struct BfsSmem {
-  uint4 n[kWarps * kWarpGroups][kBfsShared];
-  uint2 b[kWarps * kWarpGroups][kBfsFaces];
-  uint32_t q[kWarps * kWarpGroups][kBfsShared];
+  static constexpr uint32_t kGroups = kWarps * (32 / kBfsLanes);
+  uint4 n[kGroups][kBfsShared];
+  uint2 b[kGroups][kBfsFaces];
+  uint32_t q[kGroups][kBfsShared];
+  __align__(16) uint32_t set[kGroups][kHashSlots];
   uint32_t sp[kOrderBuckets + 2];
   uint32_t huge[6];
   unsigned long long searches;
@@ -1058,15 +1098,22 @@ __device__ __forceinline__ const uint32_t* cand_cavity(const Dev& D, uint32_t of
   return (off & 0x80000000u) ? big_slot(D, off & 0x7FFFFFFFu) : D.pool + off;
 }
 
+// Marks the owner of a claim of this round that `key` displaced: it has lost a
+// tet of its cavity.
+__device__ __forceinline__ void displaced(const Dev& D, const RoundArgs& R, unsigned long long key,
+                                          unsigned long long old) {
+  if (old > key && this_round(R, old)) {
+    const uint32_t q = key_owner(R, old);
+    if (q < D.nv) D.stat[q].lost = uint16_t(R.round);
+  }
+}
+
 // Claims tet t for `key`; true when a better claim holds it.  A displaced
 // owner of this round is marked: it has lost a tet of its cavity.
 __device__ __forceinline__ bool claim(const Dev& D, const RoundArgs& R, uint32_t t, unsigned long long key,
                                       unsigned long long& old) {
   old = atomicMin(&D.T[t].cav, key);
-  if (old > key && this_round(R, old)) {
-    const uint32_t q = key_owner(R, old);
-    if (q < D.nv) D.stat[q].lost = uint16_t(R.round);
-  }
+  displaced(D, R, key, old);
   return old < key;
 }
 
@@ -1170,8 +1217,20 @@ __device__ __forceinline__ void expand_big(const Dev& D, const RoundArgs& R, uin
   __syncthreads();
 }
 
-template <uint32_t kWarps>
-__device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSmem<kWarps>& sm) {
+// Adds tet t to a search's set; false when it was there.
+__device__ __forceinline__ bool set_add(uint32_t* set, uint32_t t) {
+  uint32_t h = (t * 0x9E3779B1u) >> 25;  // 128 slots
+  for (;;) {  // ends: at most kHashTets + 32 tets in kHashSlots slots
+    const uint32_t o = atomicCAS(&set[h], NONE, t);
+    if (o == NONE) return true;
+    if (o == t) return false;
+    h = (h + 1) & (kHashSlots - 1);
+  }
+}
+
+template <uint32_t kWarps, uint32_t kBfsLanes>
+__device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSmem<kWarps, kBfsLanes>& sm) {
+  constexpr uint32_t kWarpGroups = 32 / kBfsLanes;
   constexpr uint32_t FULL = 0xFFFFFFFFu, GM = (kBfsLanes == 32) ? 0xFFFFFFFFu : ((1u << kBfsLanes) - 1u);
   // the next round's counters (their last readers finished with the last round)
   if (blockIdx.x == 0 && threadIdx.x < sizeof(Counters) / 4)
@@ -1186,6 +1245,7 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
   uint32_t* sq = sm.q[threadIdx.x / kBfsLanes];
   uint4* sn = sm.n[threadIdx.x / kBfsLanes];
   uint2* sb = sm.b[threadIdx.x / kBfsLanes];
+  uint32_t* set = sm.set[threadIdx.x / kBfsLanes];
   uint32_t* gq = D.wscratch + size_t(gid < D.wgroups ? gid : 0) * kScratchWords;
   uint2* gb = reinterpret_cast<uint2*>(gq + BIG_CAP);
   if (threadIdx.x == 0) sm.searches = 0;
@@ -1234,7 +1294,7 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
     uint32_t cur = 0;  // the lane whose start this group works on
     bool running = false, lost = false, overflow = false;
     uint32_t p = 0, K = 0, F = 0, head = 0;
-    unsigned long long key = 0;
+    unsigned long long key = 0, pend = ~0ull;  // pend: the answer to this lane's last claim
     float4 pq = pq_l;
     for (;;) {
       const uint32_t busy = __ballot_sync(FULL, running);
@@ -1271,6 +1331,15 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
             sq[0] = t_s;
             sn[0] = make_uint4(n0, n1, n2, n3);
           }
+          // the slot set_add() looks at first holds t0 from the start
+#pragma unroll
+          for (uint32_t i = 0; i < kHashSlots / 4 / kBfsLanes; ++i) {
+            const uint32_t w = 4u * (gl + i * kBfsLanes), h = (t_s * 0x9E3779B1u) >> 25;
+            reinterpret_cast<uint4*>(set)[w / 4u] =
+                make_uint4(w == h ? t_s : NONE, w + 1u == h ? t_s : NONE, w + 2u == h ? t_s : NONE,
+                           w + 3u == h ? t_s : NONE);
+          }
+          pend = ~0ull;
         }
         __syncwarp();
       } else if (!busy) {
@@ -1280,8 +1349,15 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
       bool add = false, bnd = false, my_lost = false, my_guard = false;
       uint32_t nt = 0, code = 0, outer = NONE;
       uint4 nn = make_uint4(NONE, NONE, NONE, NONE);
+      // a search that outgrew its set tells tets apart by its claims alone: all
+      // of them must have arrived
+      if (running && K > kHashTets && pend != ~0ull) {
+        my_lost = pend < key;
+        displaced(D, R, key, pend);
+        pend = ~0ull;
+      }
       unsigned long long old0 = ~0ull;
-      if (fresh && gl == 0) my_lost = claim(D, R, sq[0], key, old0);
+      if (fresh && gl == 0) old0 = atomicMin(&D.T[sq[0]].cav, key);
       const uint32_t idx = head + gl / 4u;
       const uint32_t f = gl & 3u;
       if (running && idx < K) {
@@ -1299,16 +1375,36 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
           const unsigned long long cc = __ldcg(&T->cav);
           nn = ld_u4(&T->n);
           const float4 X = ld_f4(&T->X), Y = ld_f4(&T->Y), Z = ld_f4(&T->Z);
+          // the last pass's claims, and the fresh search's own tet
+          my_lost = my_lost || pend < key || old0 < key;
+          displaced(D, R, key, pend);
+          displaced(D, R, key, old0);
+          pend = old0 = ~0ull;
           if (cc != key) {
-            if (in_sphere(D, T, X, Y, Z, pq, p) < 0) {
+            if (in_sphere(D, T, X, Y, Z, pq, p) >= 0) {
+              bnd = true;
+            } else if (cc < key) {
+              my_lost = true;  // a better claim holds it
+            } else if (K <= kHashTets) {
+              add = set_add(set, nt);
+              if (add) pend = atomicMin(&D.T[nt].cav, key);
+            } else {
               unsigned long long old;
               if (claim(D, R, nt, key, old)) my_lost = true;
               else add = old != key;
-            } else {
-              bnd = true;
             }
           }
         }
+      }
+      // answers not looked at above (no pair in this pass)
+      if (running && !add && pend != ~0ull) {
+        my_lost = my_lost || pend < key;
+        displaced(D, R, key, pend);
+        pend = ~0ull;
+      }
+      if (old0 != ~0ull) {
+        my_lost = my_lost || old0 < key;
+        displaced(D, R, key, old0);
       }
       const uint32_t aball = (__ballot_sync(FULL, add) >> shift) & GM;
       const uint32_t bball = (__ballot_sync(FULL, bnd) >> shift) & GM;
@@ -1342,6 +1438,11 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
         F += __popc(bball);
         running = !lost && !overflow && head < K;
         fin = !running;
+        // a search that ends lost still displaced what its last claims displaced
+        if (fin && pend != ~0ull) {
+          displaced(D, R, key, pend);
+          pend = ~0ull;
+        }
       }
       __syncwarp();
       if (!__any_sync(FULL, fin)) continue;
@@ -1400,8 +1501,8 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
 __global__ void __launch_bounds__(128, WTET_BFS_MINB) k_bfs(Dev D) {
   const RoundArgs R = load_round(D);
   if (!R.live) return;
-  __shared__ BfsSmem<4> sm;
-  bfs_body<4>(D, R, sm);
+  __shared__ BfsSmem<4, kBulkLanes> sm;
+  bfs_body<4, kBulkLanes>(D, R, sm);
 }
 
 __device__ __forceinline__ uint32_t slot_of(const Dev& D, const RoundArgs& R, uint32_t v) {
@@ -1433,9 +1534,13 @@ __device__ __forceinline__ uint32_t edge_hi(const uint4& V, int f, int k) {
 constexpr uint32_t kWinInPlace = 1u;  // the star takes the cavity's own slots
 constexpr uint32_t kWinBlock = 2u;    // a whole block writes the star
 constexpr uint32_t kBigWinners = 4096;
-constexpr uint32_t kBlockFaces = 340;  // larger stars are written by a whole block
+// Stars of more faces than this are written by a whole block: in large rounds
+// those beyond the per-warp tables, in k_rounds (which waits for the slowest
+// star of every round, with blocks to spare) those beyond shared memory.
+constexpr uint32_t kBlockFaces = 340;
+constexpr uint32_t kBlockFacesSmall = 64;
 
-template <uint32_t kWarps>
+template <uint32_t kWarps, uint32_t kBlock>
 __device__ __forceinline__ void shared_body(const Dev& D, const RoundArgs& R) {
   constexpr uint32_t FULL = 0xFFFFFFFFu;
   const uint32_t lane = threadIdx.x & 31;
@@ -1552,7 +1657,7 @@ __device__ __forceinline__ void shared_body(const Dev& D, const RoundArgs& R) {
         base_l = mybase;
         touch_l = touch[j];
         flags_l = F[j] <= kInPlaceFaces && !(off & 0x80000000u) ? kWinInPlace : 0u;
-        if (F[j] > kBlockFaces) {
+        if (F[j] > kBlock) {
           const uint32_t i = atomicAdd(&R.ctr->nbigw, 1u);
           if (i < kBigWinners) {
             D.bigw[i] = c0 + j;
@@ -1572,7 +1677,7 @@ __device__ __forceinline__ void shared_body(const Dev& D, const RoundArgs& R) {
 __global__ void __launch_bounds__(128, WTET_SHARED_MINB) k_shared(Dev D) {
   const RoundArgs R = load_round(D);
   if (!R.live) return;
-  shared_body<4>(D, R);
+  shared_body<4, kBlockFaces>(D, R);
 }
 
 // Writes the new tets of every winner.  The three faces through p of a new
@@ -2024,8 +2129,8 @@ __device__ __forceinline__ NextStratum next_stratum(const Dev& D, int32_t next_l
 // locates the next stratum when it is due (in front of the carried points);
 // carries the recycled slots that were not handed out this round over.
 //
-// A point of the new stratum walks from the tet of the point one stride
-// earlier on the curve (a point of an earlier stratum: its tet once inserted,
+// A point of the new stratum walks from the tet of the nearer of the points one
+// stride earlier and later on the curve (a point of an earlier stratum: its tet once inserted,
 // else the tet that contains it -- as of this round or, while this very pass
 // relocates it, of the last one; a retired tet forwards to a live one).
 __device__ __forceinline__ void relocate_body(const Dev& D, const RoundArgs& R, const NextStratum& ns) {
@@ -2049,8 +2154,17 @@ __device__ __forceinline__ void relocate_body(const Dev& D, const RoundArgs& R, 
       R.active_next[idx] = p;
       if (D.bigflag[p] & kDup) continue;  // never located, dropped by the next pass
       uint32_t t = NONE;
+      const float4 pq = ld_f4(&D.pts[p]);
       if (level < C.top) {
-        const uint32_t hv = p - stride;
+        // the nearer of the two neighbours on the curve (a curve jumps: the
+        // other one may be far off)
+        uint32_t hv = p - stride;
+        if (pos + stride < C.n) {
+          const float4 a = ld_f4(&D.pts[p - stride]), b = ld_f4(&D.pts[p + stride]);
+          const float da = (a.x - pq.x) * (a.x - pq.x) + (a.y - pq.y) * (a.y - pq.y) + (a.z - pq.z) * (a.z - pq.z);
+          const float db = (b.x - pq.x) * (b.x - pq.x) + (b.y - pq.y) * (b.y - pq.y) + (b.z - pq.z) * (b.z - pq.z);
+          if (db < da && !(D.bigflag[p + stride] & kDup)) hv = p + stride;
+        }
         const uint32_t hl = __ldcg(&D.loc[hv]);
         uint32_t h = (hl & INS_BIT) ? D.vtet[hv] : hl;
         if (h < D.cap) {
@@ -2063,10 +2177,8 @@ __device__ __forceinline__ void relocate_body(const Dev& D, const RoundArgs& R, 
         }
       }
       if (t == NONE) t = D.centry[c];
-      const uint32_t lt = walk_to(D, t, p, D.pts[p], steps);
-      D.loc[p] = lt;
       D.bigflag[p] = 0;
-      cast_vote(D, p, lt);
+      D.loc[p] = locate(D, t, p, pq, steps);
     }
   }
   for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < R.n_active; i0 += gridDim.x * blockDim.x) {
@@ -2100,9 +2212,7 @@ __device__ __forceinline__ void relocate_body(const Dev& D, const RoundArgs& R, 
           if (q < D.nv && D.stat[q].ins == uint16_t(R.round)) from = t;
         }
         if (from != NONE) {
-          const uint32_t lt = walk_to(D, from, p, D.pts[p], steps);
-          D.loc[p] = lt;
-          cast_vote(D, p, lt);
+          D.loc[p] = locate(D, from, p, ld_f4(&D.pts[p]), steps);
         }
       }
     }
@@ -2219,7 +2329,7 @@ __global__ void k_begin(Dev D) {
 constexpr uint32_t kRoundThreads = 512;
 constexpr uint32_t kRoundWarps = kRoundThreads / 32;
 union RoundSmem {
-  BfsSmem<kRoundWarps> bfs;
+  BfsSmem<kRoundWarps, 32> bfs;
   WriteSmem<kRoundWarps> write;
   CandSmem<kRoundWarps> cand;
 };
@@ -2248,9 +2358,9 @@ __global__ void __launch_bounds__(kRoundThreads, 1) k_rounds(Dev D) {
     if (kLearned && (R.flags & kLearnedRound)) cands_body<kLearned, kRoundWarps>(D, R, net, &sm.cand);
     else cands_body<false, 1>(D, R, nullptr, nullptr);
     cluster_barrier();
-    bfs_body<kRoundWarps>(D, R, sm.bfs);
+    bfs_body<kRoundWarps, 32>(D, R, sm.bfs);
     cluster_barrier();
-    shared_body<kRoundWarps>(D, R);
+    shared_body<kRoundWarps, kBlockFacesSmall>(D, R);
     cluster_barrier();
     write_body<kRoundWarps>(D, R, sm.write);
     cluster_barrier();
@@ -2839,7 +2949,7 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
   W.starts.reserve(start_ovf + n, "starts");
   // one overflow region per lane group of a k_bfs wave, one edge table per
   // warp of a k_write wave
-  const uint32_t wgroups = wave(k_bfs, 128) * 4 * kWarpGroups;
+  const uint32_t wgroups = wave(k_bfs, 128) * (128 / kBulkLanes);
   W.wscratch.reserve(size_t(wgroups) * kScratchWords, "cavity queues");
   const uint32_t etab_warps = wave(k_write, 128) * 4;
   W.etab.reserve(size_t(etab_warps) * kEdgeWordsG, "edge tables");
