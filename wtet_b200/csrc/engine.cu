@@ -468,27 +468,30 @@ __device__ __forceinline__ int o3d_sos_f(const float4& a, const float4& b, const
   if (s != 0) return s < 0 ? 1 : -1;
   return o3d_sos_slow(a, b, c, d, va, vb, vc, vd, sos, err);
 }
-__device__ __noinline__ int o4d_sos_slow(float4 a, float4 b, float4 c, float4 d, float4 e, uint32_t va,
-                                         uint32_t vb, uint32_t vc, uint32_t vd, uint32_t ve, const uint32_t* sos,
-                                         uint32_t* err) {
-  const double A[3] = {a.x, a.y, a.z}, B[3] = {b.x, b.y, b.z}, C[3] = {c.x, c.y, c.z}, Dd[3] = {d.x, d.y, d.z};
+// `known`: what insphere_mid said (0: nothing, 2: exactly 0, SoS decides).
+__device__ __noinline__ int o4d_sos_slow(float4 X, float4 Y, float4 Z, float4 e, uint32_t va, uint32_t vb, uint32_t vc,
+                                         uint32_t vd, uint32_t ve, const uint32_t* sos, uint32_t* err, int known) {
+  const double A[3] = {X.x, Y.x, Z.x}, B[3] = {X.y, Y.y, Z.y}, C[3] = {X.z, Y.z, Z.z}, Dd[3] = {X.w, Y.w, Z.w};
   const double E[3] = {e.x, e.y, e.z};
+  if (known == 2)
+    return ex::orient4d_sos_degenerate(A, B, C, Dd, E, sos[va], sos[vb], sos[vc], sos[vd], sos[ve], err);
   return o4d_sos(A, B, C, Dd, E, va, vb, vc, vd, ve, sos, err);
 }
-__device__ __forceinline__ int o4d_sos_f(const float4& a, const float4& b, const float4& c, const float4& d,
-                                         const float4& e, uint32_t va, uint32_t vb, uint32_t vc, uint32_t vd,
-                                         uint32_t ve, const uint32_t* sos, uint32_t* err) {
-  const int s = ex::insphere_f32(a, b, c, d, e);
+__device__ __forceinline__ int o4d_sos_f(const float4& X, const float4& Y, const float4& Z, const float4& e,
+                                         uint32_t va, uint32_t vb, uint32_t vc, uint32_t vd, uint32_t ve,
+                                         const uint32_t* sos, uint32_t* err) {
+  int s = ex::insphere_f32(corner(X, Y, Z, 0), corner(X, Y, Z, 1), corner(X, Y, Z, 2), corner(X, Y, Z, 3), e);
   if (s != 0) return s;
-  return o4d_sos_slow(a, b, c, d, e, va, vb, vc, vd, ve, sos, err);
+  s = ex::insphere_mid(X, Y, Z, e);
+  if (s == 1 || s == -1) return s;
+  return o4d_sos_slow(X, Y, Z, e, va, vb, vc, vd, ve, sos, err, s);
 }
 
 // The same insphere test out of line (FP32 stage included), for kernels that
 // test a face only now and then: their main path then keeps fewer registers.
-__device__ __noinline__ int o4d_sos_call(float4 a, float4 b, float4 c, float4 d, float4 e, uint32_t va, uint32_t vb,
-                                         uint32_t vc, uint32_t vd, uint32_t ve, const uint32_t* sos,
-                                         uint32_t* err) {
-  return o4d_sos_f(a, b, c, d, e, va, vb, vc, vd, ve, sos, err);
+__device__ __noinline__ int o4d_sos_call(float4 X, float4 Y, float4 Z, float4 e, uint32_t va, uint32_t vb, uint32_t vc,
+                                         uint32_t vd, uint32_t ve, const uint32_t* sos, uint32_t* err) {
+  return o4d_sos_f(X, Y, Z, e, va, vb, vc, vd, ve, sos, err);
 }
 
 // Insphere test of p (coordinates pq) against tet T, whose coordinates were
@@ -496,15 +499,16 @@ __device__ __noinline__ int o4d_sos_call(float4 a, float4 b, float4 c, float4 d,
 // cannot decide.
 __device__ __forceinline__ int in_sphere(const Dev& D, const Tet* T, const float4& X, const float4& Y,
                                          const float4& Z, const float4& pq, uint32_t p) {
-  const int s = ex::insphere_f32(corner(X, Y, Z, 0), corner(X, Y, Z, 1), corner(X, Y, Z, 2), corner(X, Y, Z, 3), pq);
+  int s = ex::insphere_f32(corner(X, Y, Z, 0), corner(X, Y, Z, 1), corner(X, Y, Z, 2), corner(X, Y, Z, 3), pq);
   if (s != 0) return s;
+  s = ex::insphere_mid(X, Y, Z, pq);
+  if (s == 1 || s == -1) return s;
   const uint4 V = ld_u4(&T->v);
   if (V.x >= D.nv || V.y >= D.nv || V.z >= D.nv || V.w >= D.nv) {
     atomicOr(&D.tot->err, kErrGuard);
     return 1;
   }
-  return o4d_sos_slow(corner(X, Y, Z, 0), corner(X, Y, Z, 1), corner(X, Y, Z, 2), corner(X, Y, Z, 3), pq, V.x, V.y,
-                      V.z, V.w, p, D.sos, &D.tot->err);
+  return o4d_sos_slow(X, Y, Z, pq, V.x, V.y, V.z, V.w, p, D.sos, &D.tot->err, s);
 }
 
 // Visibility walk from tet t to the tet that contains p, and p's vote there.
@@ -1605,8 +1609,7 @@ __device__ __forceinline__ void shared_body(const Dev& D, const RoundArgs& R) {
         set_fcomp(X, f, pq.x);
         set_fcomp(Y, f, pq.y);
         set_fcomp(Z, f, pq.z);
-        if (o4d_sos_call(corner(X, Y, Z, 0), corner(X, Y, Z, 1), corner(X, Y, Z, 2), corner(X, Y, Z, 3), D.pts[q], V.x,
-                         V.y, V.z, V.w, q, D.sos, &D.tot->err) < 0)
+        if (o4d_sos_call(X, Y, Z, D.pts[q], V.x, V.y, V.z, V.w, q, D.sos, &D.tot->err) < 0)
           bad = true;
       }
       bad = __any_sync(FULL, bad);
@@ -2393,7 +2396,8 @@ __global__ void k_predicate_signs(const float* pts, const uint32_t* keys, uint64
     const float4 e = make_float4(q[12], q[13], q[14], 0.f);
     const uint32_t* k = keys + 5 * i;
     o3[i] = o3d_sos_f(a, b, c, d, 0, 1, 2, 3, k, err);
-    o4[i] = o4d_sos_f(a, b, c, d, e, 0, 1, 2, 3, 4, k, err);
+    o4[i] = o4d_sos_f(make_float4(a.x, b.x, c.x, d.x), make_float4(a.y, b.y, c.y, d.y), make_float4(a.z, b.z, c.z, d.z),
+                      e, 0, 1, 2, 3, 4, k, err);
   }
 }
 

@@ -490,6 +490,96 @@ __device__ __noinline__ int lifted_modular(const double* pa, const double* pb, c
   return crt_sign(det);
 }
 
+// ---- Exact stage for box corners ----
+//
+// Points whose coordinates take at most two values on every axis are corners of
+// one axis-parallel box: lattice cells and their faces, the sets on which the
+// filters always fail.  Corner i is lo + b_i (hi - lo) per axis with a bit b_i,
+// so the determinants reduce to bits:
+//   insphere   five corners lie on the box's circumsphere: exactly 0
+//   orient3d   det(bits) times the three (positive) extents
+//   lifted     |p|^2 is linear in the bits, so det[[u, v, |p|^2, 1]] is
+//              det(bits) times the extents of u and v and hi_w^2 - lo_w^2,
+//              whose sign is that of hi_w + lo_w
+// An axis with a single value has all bits 0 and the determinant is 0, as it
+// must be.  Equal values are compared as numbers (-0 = +0), which is what the
+// determinants see.  Measured on the 72^3 lattice with a tenth of the sites
+// missing (8.2M tests that no filter decides): see in_sphere in engine.cu.
+
+// Bits of n values that take at most two values; false otherwise.  lo, hi: the
+// two values (equal when there is one).
+template <int N>
+__device__ __forceinline__ bool two_values(const double* v, uint32_t& bits, double& lo, double& hi) {
+  lo = hi = v[0];
+#pragma unroll
+  for (int i = 1; i < N; ++i) {
+    lo = fmin(lo, v[i]);
+    hi = fmax(hi, v[i]);
+  }
+  bits = 0;
+  bool ok = true;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    ok = ok && (v[i] == lo || v[i] == hi);
+    if (v[i] != lo) bits |= 1u << i;
+  }
+  return ok;
+}
+
+// Sign of det[[x_i - x_3, y_i - y_3, z_i - z_3]], i = 0..2, of bit vectors x, y, z.
+__device__ __forceinline__ int det_bits(uint32_t x, uint32_t y, uint32_t z) {
+  int X[3], Y[3], Z[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    X[i] = int((x >> i) & 1u) - int(x >> 3);
+    Y[i] = int((y >> i) & 1u) - int(y >> 3);
+    Z[i] = int((z >> i) & 1u) - int(z >> 3);
+  }
+  const int d = X[0] * (Y[1] * Z[2] - Y[2] * Z[1]) - Y[0] * (X[1] * Z[2] - X[2] * Z[1]) +
+                Z[0] * (X[1] * Y[2] - X[2] * Y[1]);
+  return (d > 0) - (d < 0);
+}
+
+// Sign of orient3d of four corners of one box, or 2.
+__device__ __forceinline__ int orient3d_box(const double* a, const double* b, const double* c, const double* d) {
+  uint32_t bit[3];
+  double lo, hi;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const double v[4] = {a[k], b[k], c[k], d[k]};
+    if (v[0] == v[1] && v[0] == v[2] && v[0] == v[3]) return 0;  // one plane
+    if (!two_values<4>(v, bit[k], lo, hi)) return 2;
+  }
+  return det_bits(bit[0], bit[1], bit[2]);
+}
+
+// Sign of det[[p_0, p_1, |p|^2, 1]] of four corners of one box, or 2.
+__device__ __forceinline__ int lifted_box(const double* a, const double* b, const double* c, const double* d) {
+  uint32_t bit[3];
+  double lo, hi;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const double v[4] = {a[k], b[k], c[k], d[k]};
+    if (!two_values<4>(v, bit[k], lo, hi)) return 2;
+  }
+  const double w = dadd(hi, lo);
+  const int s = det_bits(bit[0], bit[1], bit[2]);
+  return w > 0.0 ? s : w < 0.0 ? -s : 0;
+}
+
+// Whether five points are corners of one box.
+__device__ __forceinline__ bool five_box(const double* a, const double* b, const double* c, const double* d,
+                                         const double* e) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const double v[5] = {a[k], b[k], c[k], d[k], e[k]};
+    uint32_t bit;
+    double lo, hi;
+    if (!two_values<5>(v, bit, lo, hi)) return false;
+  }
+  return true;
+}
+
 // Sign of Shewchuk orient3d(a,b,c,d): FP64 filter, then exact.
 __device__ __forceinline__ int orient3d(const double* pa, const double* pb, const double* pc, const double* pd,
                                         uint32_t* flags) {
@@ -511,6 +601,8 @@ __device__ __forceinline__ int orient3d(const double* pa, const double* pb, cons
   // arrays never have their address taken, so they stay in registers.
   double a[3] = {pa[0], pa[1], pa[2]}, b[3] = {pb[0], pb[1], pb[2]};
   double c[3] = {pc[0], pc[1], pc[2]}, d[3] = {pd[0], pd[1], pd[2]};
+  const int sb = orient3d_box(a, b, c, d);
+  if (sb != 2) return sb;
   const int sm = orient3d_modular(a, b, c, d, err);
   if (sm != 2) return sm;
   return orient3d_exact_sign(a, b, c, d, flags);
@@ -551,6 +643,7 @@ __device__ __forceinline__ int insphere(const double* pa, const double* pb, cons
   double a[3] = {pa[0], pa[1], pa[2]}, b[3] = {pb[0], pb[1], pb[2]};
   double c[3] = {pc[0], pc[1], pc[2]}, d[3] = {pd[0], pd[1], pd[2]};
   double e[3] = {pe[0], pe[1], pe[2]};
+  if (five_box(a, b, c, d, e)) return 0;
   const int sm = insphere_modular(a, b, c, d, e, err);
   if (sm != 2) return sm;
   return insphere_exact_sign(a, b, c, d, e, flags);
@@ -637,6 +730,59 @@ __device__ __forceinline__ int insphere_f32(const float4& pa, const float4& pb, 
   return 0;
 }
 
+// Sign of Shewchuk insphere(a,b,c,d,e), when certain from f64 arithmetic with a
+// bound on the permanent instead of the permanent itself, or 0; 2 when the
+// points are corners of one box (exactly 0).  X, Y, Z: the coordinates of a..d
+// by axis.
+//
+// With r_i the largest coordinate difference of point i to e, each 2x2 minor's
+// permanent is at most 2 r_i r_j, each lift at most 3 r_i^2, so Shewchuk's
+// permanent is at most 18 r_a r_b r_c r_d (r_a + r_b + r_c + r_d).  The r_i are
+// taken in f32 (relative error 2^-24 each); the factor 1 + 2^-18 covers them and
+// the product's own rounding, and the points are f32 values, far from f64
+// underflow.  The stage has half the operations and registers of the full
+// filter, which decides what this one cannot; it exists for inputs that defeat
+// the FP32 stage wholesale (points on a sphere: nearly half of all tests).
+__device__ __noinline__ int insphere_mid(float4 X, float4 Y, float4 Z, float4 e) {
+  const float ra = fmaxf(fmaxf(fabsf(X.x - e.x), fabsf(Y.x - e.y)), fabsf(Z.x - e.z));
+  const float rb = fmaxf(fmaxf(fabsf(X.y - e.x), fabsf(Y.y - e.y)), fabsf(Z.y - e.z));
+  const float rc = fmaxf(fmaxf(fabsf(X.z - e.x), fabsf(Y.z - e.y)), fabsf(Z.z - e.z));
+  const float rd = fmaxf(fmaxf(fabsf(X.w - e.x), fabsf(Y.w - e.y)), fabsf(Z.w - e.z));
+  const double bound = dmul(dmul(dmul(kIspBoundA * 18.0 * (1.0 + 0x1p-18), dmul(double(ra), double(rb))),
+                                 dmul(double(rc), double(rd))),
+                            dadd(dadd(double(ra), double(rb)), dadd(double(rc), double(rd))));
+  const double ex = e.x, ey = e.y, ez = e.z;
+  const double ax = dsub(X.x, ex), bx = dsub(X.y, ex), cx = dsub(X.z, ex), dx = dsub(X.w, ex);
+  const double ay = dsub(Y.x, ey), by = dsub(Y.y, ey), cy = dsub(Y.z, ey), dy = dsub(Y.w, ey);
+  const double az = dsub(Z.x, ez), bz = dsub(Z.y, ez), cz = dsub(Z.z, ez), dz = dsub(Z.w, ez);
+  const double ab = dsub(dmul(ax, by), dmul(bx, ay)), bc = dsub(dmul(bx, cy), dmul(cx, by));
+  const double cd = dsub(dmul(cx, dy), dmul(dx, cy)), da = dsub(dmul(dx, ay), dmul(ax, dy));
+  const double ac = dsub(dmul(ax, cy), dmul(cx, ay)), bd = dsub(dmul(bx, dy), dmul(dx, by));
+  const double abc = dadd(dsub(dmul(az, bc), dmul(bz, ac)), dmul(cz, ab));
+  const double bcd = dadd(dsub(dmul(bz, cd), dmul(cz, bd)), dmul(dz, bc));
+  const double cda = dadd(dadd(dmul(cz, da), dmul(dz, ac)), dmul(az, cd));
+  const double dab = dadd(dadd(dmul(dz, ab), dmul(az, bd)), dmul(bz, da));
+  const double al = dadd(dadd(dmul(ax, ax), dmul(ay, ay)), dmul(az, az));
+  const double bl = dadd(dadd(dmul(bx, bx), dmul(by, by)), dmul(bz, bz));
+  const double cl = dadd(dadd(dmul(cx, cx), dmul(cy, cy)), dmul(cz, cz));
+  const double dl = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
+  const double det = dadd(dsub(dmul(dl, abc), dmul(cl, dab)), dsub(dmul(bl, cda), dmul(al, bcd)));
+  if (det > bound) return 1;
+  if (-det > bound) return -1;
+  // corners of one box: at most two values on every axis
+  const float lx = fminf(fminf(X.x, X.y), fminf(X.z, X.w)), hx = fmaxf(fmaxf(X.x, X.y), fmaxf(X.z, X.w));
+  const float ly = fminf(fminf(Y.x, Y.y), fminf(Y.z, Y.w)), hy = fmaxf(fmaxf(Y.x, Y.y), fmaxf(Y.z, Y.w));
+  const float lz = fminf(fminf(Z.x, Z.y), fminf(Z.z, Z.w)), hz = fmaxf(fmaxf(Z.x, Z.y), fmaxf(Z.z, Z.w));
+  // (a..d span no degenerate box: one value on an axis would make the tet flat)
+  const bool bxs = (X.x == lx || X.x == hx) && (X.y == lx || X.y == hx) && (X.z == lx || X.z == hx) &&
+                   (X.w == lx || X.w == hx) && (e.x == lx || e.x == hx);
+  const bool bys = (Y.x == ly || Y.x == hy) && (Y.y == ly || Y.y == hy) && (Y.z == ly || Y.z == hy) &&
+                   (Y.w == ly || Y.w == hy) && (e.y == ly || e.y == hy);
+  const bool bzs = (Z.x == lz || Z.x == hz) && (Z.y == lz || Z.y == hz) && (Z.z == lz || Z.z == hz) &&
+                   (Z.w == lz || Z.w == hz) && (e.z == lz || e.z == hz);
+  return bxs && bys && bzs ? 2 : 0;
+}
+
 // ---- SoS cascade pieces (src/predicates.rs) ----
 
 // Plain double orient2d on coordinates (u, v): src/predicates.rs:73-75.
@@ -668,6 +814,8 @@ __device__ __noinline__ int orient3d_lifted(const double* a0, const double* b0, 
                      dmul(dadd(fabs(adxbdy), fabs(bdxady)), fabs(cdz)));
   double err = dmul(kO3dBoundLifted, perm);
   if (det > err || -det > err) return (det > 0.0) - (det < 0.0);
+  const int sb = lifted_box(pa, pb, pc, pd);
+  if (sb != 2) return sb;
   const int sm = lifted_modular(pa, pb, pc, pd);
   if (sm != 2) return sm;
   int kl[4];
