@@ -770,10 +770,12 @@ __device__ __noinline__ int insphere_mid(float4 X, float4 Y, float4 Z, float4 e)
   if (det > bound) return 1;
   if (-det > bound) return -1;
   // corners of one box: at most two values on every axis
-  const float lx = fminf(fminf(X.x, X.y), fminf(X.z, X.w)), hx = fmaxf(fmaxf(X.x, X.y), fmaxf(X.z, X.w));
-  const float ly = fminf(fminf(Y.x, Y.y), fminf(Y.z, Y.w)), hy = fmaxf(fmaxf(Y.x, Y.y), fmaxf(Y.z, Y.w));
-  const float lz = fminf(fminf(Z.x, Z.y), fminf(Z.z, Z.w)), hz = fmaxf(fmaxf(Z.x, Z.y), fmaxf(Z.z, Z.w));
-  // (a..d span no degenerate box: one value on an axis would make the tet flat)
+  const float lx = fminf(fminf(fminf(X.x, X.y), fminf(X.z, X.w)), e.x);
+  const float hx = fmaxf(fmaxf(fmaxf(X.x, X.y), fmaxf(X.z, X.w)), e.x);
+  const float ly = fminf(fminf(fminf(Y.x, Y.y), fminf(Y.z, Y.w)), e.y);
+  const float hy = fmaxf(fmaxf(fmaxf(Y.x, Y.y), fmaxf(Y.z, Y.w)), e.y);
+  const float lz = fminf(fminf(fminf(Z.x, Z.y), fminf(Z.z, Z.w)), e.z);
+  const float hz = fmaxf(fmaxf(fmaxf(Z.x, Z.y), fmaxf(Z.z, Z.w)), e.z);
   const bool bxs = (X.x == lx || X.x == hx) && (X.y == lx || X.y == hx) && (X.z == lx || X.z == hx) &&
                    (X.w == lx || X.w == hx) && (e.x == lx || e.x == hx);
   const bool bys = (Y.x == ly || Y.x == hy) && (Y.y == ly || Y.y == hy) && (Y.z == ly || Y.z == hy) &&
@@ -1006,6 +1008,106 @@ __device__ __noinline__ int orient4d_sos_degenerate(const double* a, const doubl
     }
   }
   return parity ? -sg : sg;
+}
+
+// Five distinct corners of one box in the cascade, on bits.  Sorted by key, the
+// first term is orient3d of points 1..4: a determinant of bits.  When it is 0
+// the four span a rectangle, whose corners are concyclic: the three lifted
+// terms of the same points, linear in the bits, are 0 too (exactly, so also
+// within the reference's filter bound).  The next term is orient3d of points 0,
+// 2, 3, 4, and point 0 is not on the rectangle's plane (a plane through three
+// corners holds at most four).  So the cascade always ends there; 0 is returned
+// for points that are not distinct, and the general cascade decides.
+__device__ __forceinline__ int orient4d_box(float4 X, float4 Y, float4 Z, float4 e, const uint32_t* key) {
+  const float hx = fmaxf(fmaxf(fmaxf(X.x, X.y), fmaxf(X.z, X.w)), e.x);
+  const float hy = fmaxf(fmaxf(fmaxf(Y.x, Y.y), fmaxf(Y.z, Y.w)), e.y);
+  const float hz = fmaxf(fmaxf(fmaxf(Z.x, Z.y), fmaxf(Z.z, Z.w)), e.z);
+  // one word per point: key, corner bits x | y << 1 | z << 2
+  uint32_t k[5], b[5];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) k[i] = key[i];
+  b[0] = uint32_t(X.x == hx) | uint32_t(Y.x == hy) << 1 | uint32_t(Z.x == hz) << 2;
+  b[1] = uint32_t(X.y == hx) | uint32_t(Y.y == hy) << 1 | uint32_t(Z.y == hz) << 2;
+  b[2] = uint32_t(X.z == hx) | uint32_t(Y.z == hy) << 1 | uint32_t(Z.z == hz) << 2;
+  b[3] = uint32_t(X.w == hx) | uint32_t(Y.w == hy) << 1 | uint32_t(Z.w == hz) << 2;
+  b[4] = uint32_t(e.x == hx) | uint32_t(e.y == hy) << 1 | uint32_t(e.z == hz) << 2;
+  int parity = 0;
+#pragma unroll
+  for (int i = 1; i < 5; ++i) {
+#pragma unroll
+    for (int j = i; j > 0; --j) {
+      if (k[j] < k[j - 1]) {
+        uint32_t t = k[j];
+        k[j] = k[j - 1];
+        k[j - 1] = t;
+        t = b[j];
+        b[j] = b[j - 1];
+        b[j - 1] = t;
+        parity ^= 1;
+      }
+    }
+  }
+  uint32_t wx = 0, wy = 0, wz = 0;  // bit i: sorted point i
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    wx |= (b[i] & 1u) << i;
+    wy |= ((b[i] >> 1) & 1u) << i;
+    wz |= ((b[i] >> 2) & 1u) << i;
+  }
+  int s = -det_bits(wx >> 1, wy >> 1, wz >> 1);  // points 1..4, flipped term
+  if (s == 0) {
+    // points 0, 2, 3, 4
+    s = det_bits((wx >> 1 & 14u) | (wx & 1u), (wy >> 1 & 14u) | (wy & 1u), (wz >> 1 & 14u) | (wz & 1u));
+  }
+  return parity ? -s : s;
+}
+
+// orient3d_sos_degenerate on f32 points, in registers.
+__device__ __forceinline__ int orient3d_sos_degenerate_f(float4 a, float4 b, float4 c, float4 d, uint32_t ia,
+                                                         uint32_t ib, uint32_t ic, uint32_t id) {
+  float4 p[4] = {a, b, c, d};
+  uint32_t k[4] = {ia, ib, ic, id};
+  int parity = 0;
+#pragma unroll
+  for (int i = 1; i < 4; ++i) {
+#pragma unroll
+    for (int j = i; j > 0; --j) {
+      if (k[j] < k[j - 1]) {
+        const uint32_t t = k[j];
+        k[j] = k[j - 1];
+        k[j - 1] = t;
+        const float4 q = p[j];
+        p[j] = p[j - 1];
+        p[j - 1] = q;
+        parity ^= 1;
+      }
+    }
+  }
+  const double x0 = p[0].x, y0 = p[0].y, z0 = p[0].z, x1 = p[1].x, y1 = p[1].y, z1 = p[1].z;
+  const double x2 = p[2].x, y2 = p[2].y, z2 = p[2].z, x3 = p[3].x, y3 = p[3].y, z3 = p[3].z;
+  // the plain-double orient2d of (a, b, c) on coordinates (u, v)
+  auto o2 = [](double au, double av, double bu, double bv, double cu, double cv) {
+    return dsub(dmul(dsub(au, cu), dsub(bv, cv)), dmul(dsub(av, cv), dsub(bu, cu)));
+  };
+  double v = o2(x1, y1, x2, y2, x3, y3);
+  bool flip = false;
+  if (v == 0.0) { v = o2(x1, z1, x2, z2, x3, z3); flip = true; }
+  if (v == 0.0) { v = o2(y1, z1, y2, z2, y3, z3); flip = false; }
+  if (v == 0.0) { v = o2(x0, y0, x2, y2, x3, y3); flip = true; }
+  if (v == 0.0) { v = dsub(x2, x3); flip = false; }
+  if (v == 0.0) { v = dsub(y2, y3); flip = true; }
+  if (v == 0.0) { v = o2(x0, z0, x2, z2, x3, z3); flip = false; }
+  if (v == 0.0) { v = dsub(z2, z3); flip = false; }
+  if (v == 0.0) { v = o2(y0, z0, y2, z2, y3, z3); flip = true; }
+  if (v == 0.0) { v = o2(x0, y0, x1, y1, x3, y3); flip = false; }
+  if (v == 0.0) { v = dsub(x1, x3); flip = true; }
+  if (v == 0.0) { v = dsub(y1, y3); flip = false; }
+  if (v == 0.0) { v = dsub(x0, x3); flip = false; }
+  if (v == 0.0) { v = 1.0; flip = false; }
+  int sg = (v > 0.0) - (v < 0.0);
+  if (flip) sg = -sg;
+  if (parity) sg = -sg;
+  return sg < 0 ? 1 : -1;
 }
 
 // gDel3D sphere orientation with SoS: -1 = e inside the circumsphere of the
