@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -44,6 +45,13 @@ void require_device() {
 
 void fill_stats(wtet_stats* dst, const wtet_stats& s) {
   if (dst) *dst = s;
+}
+
+void to_device(std::initializer_list<wtet::HostCopy> seg, cudaStream_t s, const char* what) {
+  wtet::host_copy(seg.begin(), seg.size(), false, s, what);
+}
+void to_host(std::initializer_list<wtet::HostCopy> seg, cudaStream_t s, const char* what) {
+  wtet::host_copy(seg.begin(), seg.size(), true, s, what);
 }
 
 // Runs one job whose input already sits in device memory; returns device
@@ -105,7 +113,7 @@ int wtet_delaunay_into(const float* xyz, uint64_t n, const wtet_config* cfg, uin
     wtet_config c = resolve(cfg);
     cudaStream_t s = nullptr;
     float* d_xyz = wtet::ws_input(3 * n);
-    ck(cudaMemcpyAsync(d_xyz, xyz, 3 * n * sizeof(float), cudaMemcpyHostToDevice, s), "copy points to device");
+    to_device({{const_cast<float*>(xyz), d_xyz, 3 * n * sizeof(float)}}, s, "copy points to device");
     uint32_t *d_t = nullptr, *d_a = nullptr;
     wtet::JobResult r = run_dev(d_xyz, {0, n}, c, s, &d_t, &d_a);
     uint64_t m = r.tet_offsets.back();
@@ -116,8 +124,7 @@ int wtet_delaunay_into(const float* xyz, uint64_t n, const wtet_config* cfg, uin
       for (size_t k = 0; k < r.failed.size(); ++k) failed_verts[k] = uint32_t(r.failed[k]);
     if (m > capacity || !tets || !adjacency)
       return fail(WTET_ERR_CAPACITY, "output capacity " + std::to_string(capacity) + " < " + std::to_string(m) + " tets");
-    ck(cudaMemcpyAsync(tets, d_t, m * 16, cudaMemcpyDeviceToHost, s), "copy tets to host");
-    ck(cudaMemcpyAsync(adjacency, d_a, m * 16, cudaMemcpyDeviceToHost, s), "copy adjacency to host");
+    to_host({{tets, d_t, m * 16}, {adjacency, d_a, m * 16}}, s, "copy tets and adjacency to host");
     ck(cudaStreamSynchronize(s), "synchronize");
     return WTET_OK;
   } catch (const wtet::Error& e) {
@@ -134,7 +141,7 @@ int wtet_delaunay(const float* xyz, uint64_t n, const wtet_config* cfg, wtet_res
     wtet_config c = resolve(cfg);
     cudaStream_t s = nullptr;
     float* d_xyz = wtet::ws_input(3 * n);
-    ck(cudaMemcpyAsync(d_xyz, xyz, 3 * n * sizeof(float), cudaMemcpyHostToDevice, s), "copy points to device");
+    to_device({{const_cast<float*>(xyz), d_xyz, 3 * n * sizeof(float)}}, s, "copy points to device");
     uint32_t *d_t = nullptr, *d_a = nullptr;
     wtet::JobResult r = run_dev(d_xyz, {0, n}, c, s, &d_t, &d_a);
     uint64_t m = r.tet_offsets.back();
@@ -145,8 +152,7 @@ int wtet_delaunay(const float* xyz, uint64_t n, const wtet_config* cfg, wtet_res
       wtet_result_free(out);
       return fail(WTET_ERR_CAPACITY, "host allocation failed");
     }
-    ck(cudaMemcpyAsync(out->tets, d_t, m * 16, cudaMemcpyDeviceToHost, s), "copy tets to host");
-    ck(cudaMemcpyAsync(out->adjacency, d_a, m * 16, cudaMemcpyDeviceToHost, s), "copy adjacency to host");
+    to_host({{out->tets, d_t, m * 16}, {out->adjacency, d_a, m * 16}}, s, "copy tets and adjacency to host");
     ck(cudaStreamSynchronize(s), "synchronize");
     out->num_tets = m;
     out->num_failed = r.failed.size();
@@ -203,7 +209,7 @@ int wtet_delaunay_batched(const float* xyz, const uint64_t* offsets, uint32_t nu
     cudaStream_t s = nullptr;
     uint64_t n = off.back();
     float* d_xyz = wtet::ws_input(3 * n);
-    ck(cudaMemcpyAsync(d_xyz, xyz, 3 * n * sizeof(float), cudaMemcpyHostToDevice, s), "copy points to device");
+    to_device({{const_cast<float*>(xyz), d_xyz, 3 * n * sizeof(float)}}, s, "copy points to device");
     uint32_t *d_t = nullptr, *d_a = nullptr;
     wtet::JobResult r = run_dev(d_xyz, off, c, s, &d_t, &d_a);
     for (uint32_t k = 0; k <= num_clouds; ++k) tet_offsets[k] = r.tet_offsets[k];
@@ -212,8 +218,7 @@ int wtet_delaunay_batched(const float* xyz, const uint64_t* offsets, uint32_t nu
     uint64_t m = r.tet_offsets.back();
     if (m > capacity || !tets || !adjacency)
       return fail(WTET_ERR_CAPACITY, "output capacity " + std::to_string(capacity) + " < " + std::to_string(m) + " tets");
-    ck(cudaMemcpyAsync(tets, d_t, m * 16, cudaMemcpyDeviceToHost, s), "copy tets to host");
-    ck(cudaMemcpyAsync(adjacency, d_a, m * 16, cudaMemcpyDeviceToHost, s), "copy adjacency to host");
+    to_host({{tets, d_t, m * 16}, {adjacency, d_a, m * 16}}, s, "copy tets and adjacency to host");
     ck(cudaStreamSynchronize(s), "synchronize");
     return WTET_OK;
   } catch (const wtet::Error& e) {
@@ -231,11 +236,10 @@ int wtet_check_quality(const float* xyz, uint64_t n, const uint32_t* tets, const
     float* d_xyz = wtet::ws_input(3 * n + 8 * m + 8);
     uint32_t* d_t = reinterpret_cast<uint32_t*>(d_xyz + 3 * n + ((4 - (3 * n) % 4) % 4));
     uint32_t* d_a = d_t + 4 * m;
-    ck(cudaMemcpyAsync(d_xyz, xyz, 3 * n * 4, cudaMemcpyHostToDevice, s), "copy points");
-    if (m) {
-      ck(cudaMemcpyAsync(d_t, tets, m * 16, cudaMemcpyHostToDevice, s), "copy tets");
-      ck(cudaMemcpyAsync(d_a, adjacency, m * 16, cudaMemcpyHostToDevice, s), "copy adjacency");
-    }
+    to_device({{const_cast<float*>(xyz), d_xyz, 3 * n * 4},
+               {const_cast<uint32_t*>(tets), d_t, m * 16},
+               {const_cast<uint32_t*>(adjacency), d_a, m * 16}},
+              s, "copy points, tets and adjacency");
     wtet::check_quality_device(d_xyz, n, d_t, d_a, m, violations, interior_tets, s);
     return WTET_OK;
   } catch (const wtet::Error& e) {
@@ -264,11 +268,10 @@ int wtet_verify(const float* xyz, uint64_t n, const uint32_t* tets, const uint32
     float* d_xyz = wtet::ws_input(3 * n + 8 * m + 8);
     uint32_t* d_t = reinterpret_cast<uint32_t*>(d_xyz + 3 * n + ((4 - (3 * n) % 4) % 4));
     uint32_t* d_a = d_t + 4 * m;
-    ck(cudaMemcpyAsync(d_xyz, xyz, 3 * n * 4, cudaMemcpyHostToDevice, s), "copy points");
-    if (m) {
-      ck(cudaMemcpyAsync(d_t, tets, m * 16, cudaMemcpyHostToDevice, s), "copy tets");
-      ck(cudaMemcpyAsync(d_a, adjacency, m * 16, cudaMemcpyHostToDevice, s), "copy adjacency");
-    }
+    to_device({{const_cast<float*>(xyz), d_xyz, 3 * n * 4},
+               {const_cast<uint32_t*>(tets), d_t, m * 16},
+               {const_cast<uint32_t*>(adjacency), d_a, m * 16}},
+              s, "copy points, tets and adjacency");
     wtet::verify_device(d_xyz, n, d_t, d_a, m, report, s);
     return WTET_OK;
   } catch (const wtet::Error& e) {
@@ -301,16 +304,11 @@ int wtet_canonicalize(const uint32_t* tets, const uint32_t* adjacency, uint64_t 
     uint32_t* d_in = reinterpret_cast<uint32_t*>(wtet::ws_input(8 * m + 4));
     uint32_t *d_ot = nullptr, *d_oa = nullptr;
     wtet::ws_outputs(std::max<uint64_t>(m, 1), &d_ot, &d_oa);
-    if (m) {
-      ck(cudaMemcpyAsync(d_in, tets, m * 16, cudaMemcpyHostToDevice, s), "copy tets");
-      ck(cudaMemcpyAsync(d_in + 4 * m, adjacency, m * 16, cudaMemcpyHostToDevice, s), "copy adjacency");
-    }
+    to_device({{const_cast<uint32_t*>(tets), d_in, m * 16}, {const_cast<uint32_t*>(adjacency), d_in + 4 * m, m * 16}},
+              s, "copy tets and adjacency");
     const uint64_t k = wtet::canonicalize_device(d_in, d_in + 4 * m, m, n, d_ot, d_oa, s);
     *num_rows = k;
-    if (k) {
-      ck(cudaMemcpyAsync(out_tets, d_ot, k * 16, cudaMemcpyDeviceToHost, s), "copy canonical tets");
-      ck(cudaMemcpyAsync(out_adjacency, d_oa, k * 16, cudaMemcpyDeviceToHost, s), "copy canonical adjacency");
-    }
+    to_host({{out_tets, d_ot, k * 16}, {out_adjacency, d_oa, k * 16}}, s, "copy canonical tets and adjacency");
     ck(cudaStreamSynchronize(s), "synchronize");
     return WTET_OK;
   } catch (const wtet::Error& e) {

@@ -93,6 +93,16 @@ wtet_config tuned_config(const wtet_config& cfg, uint64_t n, uint32_t num_clouds
 // Message returned by wtet_last_error() on this thread.
 void set_last_error(const std::string& msg);
 
+// Copies the segments to the host (to_host) or to the device, in the order of
+// stream s; host memory may be pageable (hostcopy.cu).  Asynchronous only for
+// pinned and small segments: synchronise s before reading the host side.
+struct HostCopy {
+  void* host;
+  void* dev;
+  size_t bytes;
+};
+void host_copy(const HostCopy* seg, size_t n, bool to_host, cudaStream_t s, const char* what);
+
 // Per-thread device buffers reused across calls (grown on demand).
 float* ws_input(size_t nfloats);
 void ws_outputs(size_t rows, uint32_t** tets, uint32_t** adj);

@@ -1,0 +1,219 @@
+// Copies between the device and ordinary (pageable) host memory for the C ABI's
+// host entry points.
+//
+// A pageable cudaMemcpy is one driver thread that copies through its own
+// staging buffer and takes every first-touch page fault of a fresh result array
+// itself: 2-6 GB/s on the measured box, where the link gives ~50.  Here a large
+// copy is cut into chunks that several threads move through pinned buffers of
+// their own: each thread keeps one DMA in flight while it copies the previous
+// chunk, so page faults, host copies and the link overlap.  Pinned and managed
+// memory, and copies below kStagedBytes, go straight to cudaMemcpyAsync.
+//
+// The threads live for one copy only (a pool that outlives the call would not
+// survive a fork of the host process); the pinned buffers are borrowed from a
+// free list of at most kKeptSets sets, so concurrent callers each have their own.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <atomic>
+#include <cstdint>
+#include <cstring>
+#include <mutex>
+#include <system_error>
+#include <thread>
+#include <vector>
+
+#include "engine.cuh"
+
+namespace wtet {
+namespace {
+
+constexpr size_t kStagedBytes = 1u << 20;  // smaller copies: thread start-up costs more than it saves
+constexpr size_t kSlotBytes = 2u << 20;
+constexpr uint32_t kLanes = 8;
+constexpr size_t kKeptSets = 2;
+
+struct Lane {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t done[2] = {nullptr, nullptr};
+  char* slot[2] = {nullptr, nullptr};
+};
+struct LaneSet {
+  int dev = -1;
+  char* pinned = nullptr;
+  Lane lane[kLanes];
+
+  bool create(int device) {
+    dev = device;
+    if (cudaMallocHost(&pinned, kLanes * 2 * kSlotBytes) != cudaSuccess) {
+      pinned = nullptr;
+      return false;
+    }
+    for (uint32_t i = 0; i < kLanes; ++i) {
+      if (cudaStreamCreateWithFlags(&lane[i].stream, cudaStreamNonBlocking) != cudaSuccess) return false;
+      for (int k = 0; k < 2; ++k) {
+        if (cudaEventCreateWithFlags(&lane[i].done[k], cudaEventDisableTiming) != cudaSuccess) return false;
+        lane[i].slot[k] = pinned + (2 * i + k) * kSlotBytes;
+      }
+    }
+    return true;
+  }
+  void destroy() {
+    for (Lane& l : lane) {
+      for (cudaEvent_t e : l.done)
+        if (e) cudaEventDestroy(e);
+      if (l.stream) cudaStreamDestroy(l.stream);
+    }
+    if (pinned) cudaFreeHost(pinned);
+  }
+};
+
+std::mutex g_mu;
+std::vector<LaneSet*>& kept() {  // never destroyed: CUDA may be gone at exit
+  static std::vector<LaneSet*>* v = new std::vector<LaneSet*>;
+  return *v;
+}
+
+LaneSet* borrow(int dev) {
+  {
+    std::lock_guard<std::mutex> g(g_mu);
+    for (size_t i = 0; i < kept().size(); ++i)
+      if (kept()[i]->dev == dev) {
+        LaneSet* s = kept()[i];
+        kept().erase(kept().begin() + long(i));
+        return s;
+      }
+  }
+  LaneSet* s = new (std::nothrow) LaneSet;
+  if (s && !s->create(dev)) {
+    s->destroy();
+    delete s;
+    s = nullptr;
+    (void)cudaGetLastError();  // no pinned memory: the caller copies directly
+  }
+  return s;
+}
+void give_back(LaneSet* s) {
+  {
+    std::lock_guard<std::mutex> g(g_mu);
+    if (kept().size() < kKeptSets) {
+      kept().push_back(s);
+      return;
+    }
+  }
+  s->destroy();
+  delete s;
+}
+
+bool pageable(const void* p) {
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return true;
+  }
+  return a.type == cudaMemoryTypeUnregistered;
+}
+
+struct Chunk {
+  char* host;
+  char* dev;
+  size_t bytes;
+};
+
+// One thread's share: chunks first, first + step, ...
+cudaError_t move_chunks(LaneSet* set, uint32_t li, const std::vector<Chunk>& c, size_t first, size_t step, bool to_host) {
+  cudaError_t e = cudaSetDevice(set->dev);
+  Lane& l = set->lane[li];
+  size_t k = first;
+  int64_t prev = -1;
+  for (uint32_t i = 0; e == cudaSuccess && k < c.size(); ++i, k += step) {
+    const uint32_t b = i & 1u;
+    if (to_host) {
+      e = cudaMemcpyAsync(l.slot[b], c[k].dev, c[k].bytes, cudaMemcpyDeviceToHost, l.stream);
+      if (e == cudaSuccess) e = cudaEventRecord(l.done[b], l.stream);
+      if (e == cudaSuccess && prev >= 0) {
+        e = cudaEventSynchronize(l.done[b ^ 1u]);
+        if (e == cudaSuccess) std::memcpy(c[size_t(prev)].host, l.slot[b ^ 1u], c[size_t(prev)].bytes);
+      }
+      prev = int64_t(k);
+    } else {
+      if (i >= 2) e = cudaEventSynchronize(l.done[b]);
+      if (e != cudaSuccess) break;
+      std::memcpy(l.slot[b], c[k].host, c[k].bytes);
+      e = cudaMemcpyAsync(c[k].dev, l.slot[b], c[k].bytes, cudaMemcpyHostToDevice, l.stream);
+      if (e == cudaSuccess) e = cudaEventRecord(l.done[b], l.stream);
+    }
+  }
+  // the slots go back to the free list: nothing of this copy may be in flight
+  const cudaError_t f = cudaStreamSynchronize(l.stream);
+  if (e == cudaSuccess) e = f;
+  if (e == cudaSuccess && to_host && prev >= 0) {
+    const uint32_t b = uint32_t((size_t(prev) - first) / step) & 1u;
+    std::memcpy(c[size_t(prev)].host, l.slot[b], c[size_t(prev)].bytes);
+  }
+  return e;
+}
+
+void direct(const HostCopy* seg, size_t n, bool to_host, cudaStream_t s, const char* what) {
+  for (size_t i = 0; i < n; ++i) {
+    if (!seg[i].bytes) continue;
+    const cudaError_t e =
+        to_host ? cudaMemcpyAsync(seg[i].host, seg[i].dev, seg[i].bytes, cudaMemcpyDeviceToHost, s)
+                : cudaMemcpyAsync(seg[i].dev, seg[i].host, seg[i].bytes, cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess) throw Error{WTET_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e)};
+  }
+}
+
+}  // namespace
+
+void host_copy(const HostCopy* seg, size_t n, bool to_host, cudaStream_t s, const char* what) {
+  size_t total = 0;
+  bool staged = true;
+  for (size_t i = 0; i < n; ++i) {
+    total += seg[i].bytes;
+    if (seg[i].bytes && !pageable(seg[i].host)) staged = false;
+  }
+  const uint32_t hw = std::max(1u, std::thread::hardware_concurrency());
+  const uint32_t lanes = std::min(kLanes, std::max(1u, hw / 2));
+  LaneSet* set = nullptr;
+  int dev = 0;
+  if (staged && total >= kStagedBytes && lanes > 1 && cudaGetDevice(&dev) == cudaSuccess) set = borrow(dev);
+  if (!set) {
+    direct(seg, n, to_host, s, what);
+    return;
+  }
+  // the source of a device-to-host copy, or the last users of a destination
+  cudaError_t e = cudaStreamSynchronize(s);
+  const size_t chunk = std::min(kSlotBytes, std::max<size_t>(256u << 10, (total / (2 * lanes) + 4095) & ~size_t(4095)));
+  std::vector<Chunk> c;
+  for (size_t i = 0; i < n; ++i)
+    for (size_t o = 0; o < seg[i].bytes; o += chunk)
+      c.push_back(Chunk{static_cast<char*>(seg[i].host) + o, static_cast<char*>(seg[i].dev) + o,
+                        std::min(chunk, seg[i].bytes - o)});
+  const uint32_t w = uint32_t(std::min<size_t>(lanes, c.size()));
+  std::atomic<int> bad{int(cudaSuccess)};
+  if (e == cudaSuccess) {
+    std::vector<std::thread> th;
+    uint32_t started = 1;  // the calling thread is lane 0
+    try {
+      th.reserve(w);
+      for (; started < w; ++started)
+        th.emplace_back([&, started] {
+          const cudaError_t r = move_chunks(set, started, c, started, w, to_host);
+          if (r != cudaSuccess) bad = int(r);
+        });
+    } catch (const std::exception&) {
+      // no more threads: the calling thread takes the remaining shares too
+    }
+    for (uint32_t k = 0; k < w; k = k == 0 ? started : k + 1) {
+      const cudaError_t r = move_chunks(set, k, c, k, w, to_host);
+      if (r != cudaSuccess) bad = int(r);
+    }
+    for (auto& t : th) t.join();
+    e = cudaError_t(bad.load());
+  }
+  give_back(set);
+  if (e != cudaSuccess) throw Error{WTET_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e)};
+}
+
+}  // namespace wtet
