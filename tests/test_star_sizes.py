@@ -1,0 +1,50 @@
+"""Cavities and stars of every size class against the oracle: a star is written
+by one warp with one face per lane (up to 32 faces), by a warp with its table in
+shared memory (up to 64) or in global memory (up to 340), or by a whole block
+(with a large table up to 5,461 faces, by rotation beyond); a cavity is searched
+by a lane group (up to 512 tets, its queue in shared memory up to 48) or by a
+block.  A few points inside an empty sphere of n points give stars of up to 2n
+faces, whichever of them comes late in the insertion order.  The same set is
+exactly what defeats the FP32 insphere stage (cospherical up to rounding)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def ball_in_sphere(n, seed, inner=6):
+    r = np.random.default_rng(seed)
+    g = r.standard_normal((n, 3))
+    p = np.concatenate([g / np.linalg.norm(g, axis=1, keepdims=True), 0.05 * r.standard_normal((inner, 3))])
+    return p.astype(np.float32)[r.permutation(n + inner)]
+
+
+def check(gpu, oracle_mod, pts, vote="plain"):
+    r = gpu.delaunay(pts, gpu.Config(vote=vote))
+    tets, adj, _ = oracle_mod.delaunay(pts, 1)
+    got = oracle_mod.canonical(r.tets, r.adjacency, len(pts))
+    want = oracle_mod.canonical(tets, adj, len(pts))
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+    return r
+
+
+@pytest.mark.parametrize("n", [4, 5, 9, 14, 17, 18, 33, 48, 65, 170, 171, 172, 260, 700])
+def test_star_classes(gpu, oracle_mod, n):
+    for seed in range(3):
+        check(gpu, oracle_mod, ball_in_sphere(n, 100 * n + seed))
+
+
+@pytest.mark.parametrize("n,vote", [(1500, "plain"), (1500, "learned"), (6000, "plain")])
+def test_block_stars(gpu, oracle_mod, n, vote):
+    """One point inside: its star is the whole sphere's if it comes late (the
+    order decides which of the seeds take the huge path)."""
+    big = [check(gpu, oracle_mod, ball_in_sphere(n, n + seed, inner=1), vote).stats["big_cavities"] for seed in range(4)]
+    assert vote == "learned" or sum(big) > 0
+
+
+@pytest.mark.parametrize("m", [4_000, 9_000, 17_000, 40_000])
+def test_small_round_boundary(gpu, oracle_mod, m):
+    """Sizes around the largest round that runs inside k_rounds."""
+    pts = np.random.default_rng(m).random((m, 3)).astype(np.float32)
+    check(gpu, oracle_mod, pts)
+    check(gpu, oracle_mod, pts, "learned")

@@ -248,7 +248,7 @@ class Config:
     ``learned_gate`` bounds the rounds the learned scheduler serves (rounds
     that may see at most learned_gate x 1024 uninserted points; 0 = 2048);
     ``initial_capacity`` sets the initial tet slots per point in eighths (0 =
-    9 per point; smaller values exercise the in-place growth of the tet
+    7.25 per point; smaller values exercise the in-place growth of the tet
     arrays).  No option changes the resulting triangulation."""
 
     def __init__(self, insertion_rule: str = "circumcenter", enable_flipping: bool = True,

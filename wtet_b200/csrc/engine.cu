@@ -346,6 +346,14 @@ __device__ __forceinline__ void set_fcomp(float4& v, int i, float x) {
   else v.w = x;
 }
 
+// The round's words of a slot's first tet: claims at the largest key (any
+// claim beats them), no vote.  Slots get them when they are first written, so
+// the arrays need no initialisation.
+__device__ __forceinline__ void fresh_words(Tet* T) {
+  T->cav = ~0ull;
+  T->pre = ~0ull;
+  T->vote = 0ull;
+}
 struct Coords {
   float4 X, Y, Z;
 };
@@ -817,18 +825,6 @@ __global__ void k_scatter_points(const uint64_t* off, const CloudInfo* ci, uint3
   D.vtet[v] = NONE;
 }
 
-// Unused tet slots: dead, no links; claims and pre-claims at the largest key
-// (any claim beats them), no vote.
-__global__ void k_init_slots(Tet* T, uint64_t from, uint64_t to) {
-  for (uint64_t i = from + uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < to;
-       i += uint64_t(gridDim.x) * blockDim.x) {
-    T[i].v = make_uint4(DEAD, DEAD, DEAD, DEAD);
-    T[i].n = make_uint4(NONE, NONE, NONE, NONE);
-    T[i].cav = T[i].pre = ~0ull;
-    T[i].vote = 0ull;
-  }
-}
-
 // Super vertices (src/gpu/mod.rs:151-158) and the initial super tet of every
 // cloud, oriented with orient3d_sos > 0 (src/phase2.rs:404-410).
 __global__ void k_init_clouds(const CloudInfo* ci, uint32_t nc, Dev D) {
@@ -850,6 +846,7 @@ __global__ void k_init_clouds(const CloudInfo* ci, uint32_t nc, Dev D) {
   int o = o3d_sos(P[0], P[1], P[2], P[3], s0, s0 + 1, s0 + 2, s0 + 3, D.sos, &D.tot->err);
   D.T[c].v = (o > 0) ? make_uint4(s0, s0 + 1, s0 + 2, s0 + 3) : make_uint4(s0 + 1, s0, s0 + 2, s0 + 3);
   D.T[c].n = make_uint4(NONE, NONE, NONE, NONE);
+  fresh_words(D.T + c);
   float4 q[4];
   const uint4 V0 = D.T[c].v;
   for (int k = 0; k < 4; ++k) q[k] = D.pts[comp(V0, k)];
@@ -1658,6 +1655,14 @@ __device__ __forceinline__ void shared_body(const Dev& D, const RoundArgs& R) {
       if (last > R.n_freed_prev && R.tet_top + (last - R.n_freed_prev) > D.cap) {
         if (lane == 0) atomicOr(&D.tot->err, kErrCapacity);
         if (lane == j) keep_l = false;
+        // the fresh slots of the reservation that exist are never written: dead
+        for (uint32_t v = max(mybase, R.n_freed_prev) + lane; v < last; v += 32) {
+          const uint32_t t = R.tet_top + (v - R.n_freed_prev);
+          if (t >= D.cap) break;
+          D.T[t].v = make_uint4(DEAD, DEAD, DEAD, DEAD);
+          D.T[t].n = make_uint4(NONE, NONE, NONE, NONE);
+          fresh_words(D.T + t);
+        }
         continue;
       }
       const uint32_t* cav = cand_cavity(D, off);
@@ -1870,14 +1875,15 @@ __device__ __forceinline__ void star_face(const Dev& D, const RoundArgs& R, uint
 }
 
 // Writes one new tet and what points at it.
-__device__ __forceinline__ void star_commit(const Dev& D, const NewTet& t, int f) {
+__device__ __forceinline__ void star_commit(const Dev& D, const RoundArgs& R, const NewTet& t, int f) {
   Tet* T = D.T + t.sl;
   T->v = t.v;
   T->n = t.n;
   T->X = t.q.X;
   T->Y = t.q.Y;
   T->Z = t.q.Z;
-  T->vote = 0ull;  // the new tet's points vote in k_relocate
+  if (t.sl >= R.tet_top) fresh_words(T);
+  else T->vote = 0ull;  // the new tet's points vote in k_relocate
   // Every vertex on the cavity boundary gets a live incident tet, so a
   // vertex's hint tet is alive whenever it is read (strata activation).
 #pragma unroll
@@ -1921,7 +1927,7 @@ __device__ __forceinline__ bool write_star(const Dev& D, const RoundArgs& R, con
       set_comp(t.n, k, link);
       ++i;
     }
-    star_commit(D, t, f);
+    star_commit(D, R, t, f);
   }
   return !bad;
 }
@@ -2074,7 +2080,7 @@ __device__ __forceinline__ void write_body(const Dev& D, const RoundArgs& R, Wri
             set_comp(t.n, k, link);
             ++i;
           }
-          star_commit(D, t, f);
+          star_commit(D, R, t, f);
         }
         s0 = __shfl_sync(FULL, t.sl, 0);
       } else {
@@ -2289,7 +2295,7 @@ __device__ __forceinline__ void end_round(const Dev& D, State& S, const Counters
   const uint32_t left = S.n_freed_prev > used ? S.n_freed_prev - used : 0u;
   // Winners that ran out of capacity reserved slot ranges they never wrote;
   // every written slot lies below the capacity, so the top never passes it
-  // (the slots between are left dead).
+  // (the slots between are marked dead).
   S.tet_top = uint32_t(min(uint64_t(S.tet_top) + fresh, uint64_t(D.cap)));
   S.n_freed_prev = __ldcg(&C->n_freed_next) + left;
   S.par ^= 1u;
@@ -2422,7 +2428,58 @@ __global__ void k_predicate_signs(const float* pts, const uint32_t* keys, uint64
 
 // --------------------------------------------------------------- output ----
 
-// Counts live tets per cloud and records the hull faces (no neighbour).
+// Output numbers of live tets.  One cloud: the rank of the slot among the live
+// ones, from a bitmap and its prefix counts (14 MB for 8M points: the four
+// neighbour look-ups of a row stay in L2, and no counter is shared by the
+// grid -- one atomic per warp on one address was most of the old numbering's
+// 7 ms at 8M points).  Several clouds: numbers handed out per cloud.
+struct RankNumber {
+  const uint32_t* live;
+  const uint32_t* rank;
+  __device__ __forceinline__ uint32_t operator()(uint32_t t) const {
+    return __ldg(rank + (t >> 5)) + __popc(__ldg(live + (t >> 5)) & ((1u << (t & 31u)) - 1u));
+  }
+};
+struct ListNumber {
+  const uint32_t* newid;
+  __device__ __forceinline__ uint32_t operator()(uint32_t t) const { return __ldg(newid + t); }
+};
+
+// Records hull faces (no neighbour).
+__device__ __forceinline__ void note_hull(const Dev& D, uint32_t t, uint32_t c, const uint4& N, uint32_t* hullcnt,
+                                          uint2* hull) {
+  for (int f = 0; f < 4; ++f) {
+    if (comp(N, f) == NONE) {
+      const uint32_t h = atomicAdd(&hullcnt[c], 1u);
+      if (h < 4) hull[4 * c + h] = make_uint2(t, uint32_t(f));
+      else atomicOr(&D.tot->err, kErrHull);
+    }
+  }
+}
+
+// One cloud: bitmap of live slots, their number per word (rank[words]: 0), hull faces.
+__global__ void k_live(Dev D, uint32_t tet_top, uint32_t words, uint32_t* live, uint32_t* rank, uint32_t* hullcnt,
+                       uint2* hull) {
+  const uint32_t lane = threadIdx.x & 31u, nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < words; w += nwarps) {
+    const uint32_t t = 32 * w + lane;
+    bool on = false;
+    if (t < tet_top) {
+      const uint32_t v = D.T[t].v.x;
+      const uint4 N = ld_u4(&D.T[t].n);
+      on = v != DEAD;
+      if (on && (N.x == NONE || N.y == NONE || N.z == NONE || N.w == NONE)) note_hull(D, t, 0, N, hullcnt, hull);
+    }
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, on);
+    if (lane == 0) {
+      live[w] = m;
+      rank[w] = __popc(m);
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) rank[words] = 0;
+}
+
+// Several clouds: counts live tets per cloud, hull faces.
 __global__ void k_count(Dev D, uint32_t tet_top, uint32_t* ccount, uint32_t* hullcnt, uint2* hull) {
   for (uint32_t t0 = blockIdx.x * blockDim.x; t0 < tet_top; t0 += gridDim.x * blockDim.x) {
     const uint32_t t = t0 + threadIdx.x;
@@ -2433,15 +2490,7 @@ __global__ void k_count(Dev D, uint32_t tet_top, uint32_t* ccount, uint32_t* hul
     const unsigned grp = __match_any_sync(0xFFFFFFFFu, c);
     const int lane = threadIdx.x & 31;
     if (live && lane == __ffs(grp) - 1) atomicAdd(&ccount[c], __popc(grp));
-    if (!live) continue;
-    uint4 N = D.T[t].n;
-    for (int f = 0; f < 4; ++f) {
-      if (comp(N, f) == NONE) {
-        uint32_t h = atomicAdd(&hullcnt[c], 1u);
-        if (h < 4) hull[4 * c + h] = make_uint2(t, uint32_t(f));
-        else atomicOr(&D.tot->err, kErrHull);
-      }
-    }
+    if (live) note_hull(D, t, c, D.T[t].n, hullcnt, hull);
   }
 }
 
@@ -2461,32 +2510,33 @@ __global__ void k_number(Dev D, uint32_t tet_top, uint32_t* cfill, uint32_t* new
   }
 }
 
-__global__ void k_emit(Dev D, uint32_t tet_top, const uint32_t* newid, const uint64_t* coff, uint32_t* out_t,
-                       uint32_t* out_a) {
+template <class Num>
+__global__ void k_emit(Dev D, uint32_t tet_top, Num num, const uint64_t* coff, uint32_t* out_t, uint32_t* out_a) {
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < tet_top; t += gridDim.x * blockDim.x) {
-    uint4 V = D.T[t].v;
+    const uint4 V = ld_u4(&D.T[t].v), N = ld_u4(&D.T[t].n);
     if (V.x == DEAD) continue;
-    uint32_t c = D.vcloud[V.x];
-    uint64_t row = coff[c] + newid[t];
-    uint4 N = D.T[t].n;
-    uint4 ov = make_uint4(D.sos[V.x], D.sos[V.y], D.sos[V.z], D.sos[V.w]);
+    const uint32_t c = D.nc == 1 ? 0u : D.vcloud[V.x];
+    const uint64_t row = coff[c] + num(t);
+    const uint4 ov = make_uint4(__ldg(D.sos + V.x), __ldg(D.sos + V.y), __ldg(D.sos + V.z), __ldg(D.sos + V.w));
     uint4 oa;
+#pragma unroll
     for (int f = 0; f < 4; ++f) {
       uint32_t nb = comp(N, f);
       if (nb != NONE && (nb >> 2) >= tet_top) {
         atomicOr(&D.tot->err, kErrGuard);
         nb = NONE;
       }
-      set_comp(oa, f, nb == NONE ? NONE : ((newid[nb >> 2] << 5) | (nb & 3)));
+      set_comp(oa, f, nb == NONE ? NONE : ((num(nb >> 2) << 5) | (nb & 3)));
     }
-    reinterpret_cast<uint4*>(out_t)[row] = ov;
-    reinterpret_cast<uint4*>(out_a)[row] = oa;
+    __stcs(reinterpret_cast<uint4*>(out_t) + row, ov);
+    __stcs(reinterpret_cast<uint4*>(out_a) + row, oa);
   }
 }
 
 // Four infinity tets per cloud on the super tetrahedron's hull faces.
+template <class Num>
 __global__ void k_infinity(Dev D, const CloudInfo* ci, uint32_t nc, const uint32_t* ccount,
-                           const uint32_t* hullcnt, const uint2* hull, const uint32_t* newid, const uint64_t* coff,
+                           const uint32_t* hullcnt, const uint2* hull, Num num, const uint64_t* coff,
                            uint32_t* out_t, uint32_t* out_a) {
   uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nc) return;
@@ -2524,7 +2574,7 @@ __global__ void k_infinity(Dev D, const CloudInfo* ci, uint32_t nc, const uint32
     uint32_t adj[4];
     for (int q = 0; q < 4; ++q) {
       if (q == int(h.y)) {
-        adj[q] = (newid[h.x] << 5) | h.y;
+        adj[q] = (num(h.x) << 5) | h.y;
         continue;
       }
       // Face opposite slot q holds inf and the two other face vertices.
@@ -2552,7 +2602,7 @@ __global__ void k_infinity(Dev D, const CloudInfo* ci, uint32_t nc, const uint32
     reinterpret_cast<uint4*>(out_t)[row] = rows[j];
     reinterpret_cast<uint4*>(out_a)[row] = make_uint4(adj[0], adj[1], adj[2], adj[3]);
     // The regular tet's hull face points at this infinity tet.
-    uint64_t rrow = coff[c] + newid[h.x];
+    uint64_t rrow = coff[c] + num(h.x);
     out_a[4 * rrow + h.y] = ((base + j) << 5) | h.y;
   }
 }
@@ -2603,7 +2653,7 @@ struct Workspace {
   DBuf<State> state;
   DBuf<Counters> ctr;
   DBuf<Totals> tot;
-  DBuf<uint32_t> ccount, hullcnt, cfill, newid;
+  DBuf<uint32_t> ccount, hullcnt, cfill, newid, live, rank;
   DBuf<uint2> hull;
   DBuf<uint64_t> coff;
   DBuf<uint32_t> out_t, out_a, dtab;
@@ -2688,7 +2738,7 @@ void release_thread_workspace() {
   w.centry.release(); w.active.release(); w.active_next.release(); w.cand.release();
   w.cand_bf.release(); w.cwin.release(); w.stat.release(); w.bigw.release(); w.bigcand.release(); w.starts.release(); w.wscratch.release(); w.pool.release(); w.big.release();
   w.freed_a.release(); w.freed_b.release(); w.lvl_off.release(); w.lvl_total.release(); w.state.release(); w.ctr.release(); w.tot.release();
-  w.ccount.release(); w.hullcnt.release(); w.cfill.release(); w.newid.release();
+  w.ccount.release(); w.hullcnt.release(); w.cfill.release(); w.newid.release(); w.live.release(); w.rank.release();
   w.hull.release(); w.coff.release(); w.out_t.release(); w.out_a.release(); w.dtab.release(); w.dup.release();
   w.etab.release(); w.btab.release();
   w.log_pslot.release(); w.losses.release(); w.prio.release();
@@ -2939,8 +2989,8 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
   }
   const uint64_t nv = n + 4ull * nc;
   uint64_t cap0 = 0;
-  const uint64_t slots_x8 = job.cfg.initial_capacity ? std::min<uint32_t>(job.cfg.initial_capacity, 1024u) : 72u;
-  for (uint32_t c = 0; c < nc; ++c) cap0 += uint64_t(ci[c].n) * slots_x8 / 8 + 64;  // 9 n by default
+  const uint64_t slots_x8 = job.cfg.initial_capacity ? std::min<uint32_t>(job.cfg.initial_capacity, 1024u) : 58u;
+  for (uint32_t c = 0; c < nc; ++c) cap0 += uint64_t(ci[c].n) * slots_x8 / 8 + 64;  // 7.25 n by default (finished clouds use up to 6.75 n)
   cap0 = std::min<uint64_t>(cap0, 0x7FFFFFF0ull);
 
   W.off.reserve(nc + 1, "offsets");
@@ -2998,7 +3048,6 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
     W.T.reserve(cap, "tets");
     W.freed_a.reserve(cap, "freed");
     W.freed_b.reserve(cap, "freed");
-    W.newid.reserve(cap, "newid");
   };
   reserve_tets(cap0);
   uint64_t cap = cap0;
@@ -3011,7 +3060,6 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
   ck(cudaMemsetAsync(W.stat.p, 0, nv * sizeof(Stat), s), "memset");
   ck(cudaMemsetAsync(W.ctr.p, 0, 2 * sizeof(Counters), s), "memset");
   ck(cudaMemsetAsync(W.tot.p, 0, sizeof(Totals), s), "memset");
-  k_init_slots<<<blocks_for(cap, 256, 148 * 16), 256, 0, s>>>(W.T.p, 0, cap);
   if (vmode) {
     W.losses.reserve(nv, "losses");
     ck(cudaMemsetAsync(W.losses.p, 0, nv, s), "memset");
@@ -3190,10 +3238,8 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
       if (ncap <= cap) throw Error{WTET_ERR_CAPACITY, "tet capacity exhausted"};
       const uint32_t top = hs.tet_top;
       W.T.grow_keep(ncap, top, s, "grow tets");
-      k_init_slots<<<blocks_for(ncap - top, 256, 148 * 16), 256, 0, s>>>(W.T.p, top, ncap);
       W.freed_a.grow_keep(ncap, ncap > 0 ? W.freed_a.n : 0, s, "grow freed");
       W.freed_b.grow_keep(ncap, W.freed_b.n, s, "grow freed");
-      W.newid.grow_keep(ncap, 0, s, "grow newid");
       cap = ncap;
       st.capacity_grows += 1;
       refresh();
@@ -3225,9 +3271,19 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
   ck(cudaMemsetAsync(W.ccount.p, 0, nc * 4, s), "memset");
   ck(cudaMemsetAsync(W.hullcnt.p, 0, nc * 4, s), "memset");
   ck(cudaMemsetAsync(W.cfill.p, 0, nc * 4, s), "memset");
-  uint32_t gt = blocks_for(tet_top, TB, 148 * 32);
-  k_count<<<gt, TB, 0, s>>>(D, tet_top, W.ccount.p, W.hullcnt.p, W.hull.p);
-  launches += 1;
+  const uint32_t gt = blocks_for(tet_top, TB, 148 * 32);
+  const uint32_t words = (tet_top + 31) / 32;
+  if (nc == 1) {
+    W.live.reserve(words, "live slots");
+    W.rank.reserve(words + 1, "live slots");
+    k_live<<<blocks_for(words, TB / 32, 148 * 64), TB, 0, s>>>(D, tet_top, words, W.live.p, W.rank.p, W.hullcnt.p,
+                                                              W.hull.p);
+    launches += 1 + scan_u32(W.rank.p, words + 1, s, W.scan_tmp);
+    ck(cudaMemcpyAsync(W.ccount.p, W.rank.p + words, 4, cudaMemcpyDeviceToDevice, s), "d2d");
+  } else {
+    k_count<<<gt, TB, 0, s>>>(D, tet_top, W.ccount.p, W.hullcnt.p, W.hull.p);
+    launches += 1;
+  }
   std::vector<uint32_t> ccount(nc);
   ck(cudaMemcpyAsync(ccount.data(), W.ccount.p, nc * 4, cudaMemcpyDeviceToHost, s), "d2h");
   ck(cudaStreamSynchronize(s), "count");
@@ -3241,11 +3297,20 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
   st.num_tets = acc;
   if (d_out_t && d_out_a && acc <= capacity) {
     ck(cudaMemcpyAsync(W.coff.p, res.tet_offsets.data(), (nc + 1) * 8, cudaMemcpyHostToDevice, s), "h2d");
-    k_number<<<gt, TB, 0, s>>>(D, tet_top, W.cfill.p, W.newid.p);
-    k_emit<<<gt, TB, 0, s>>>(D, tet_top, W.newid.p, W.coff.p, d_out_t, d_out_a);
-    k_infinity<<<(nc + 127) / 128, 128, 0, s>>>(D, W.ci.p, nc, W.ccount.p, W.hullcnt.p, W.hull.p, W.newid.p,
-                                                W.coff.p, d_out_t, d_out_a);
-    launches += 3;
+    if (nc == 1) {
+      const RankNumber num{W.live.p, W.rank.p};
+      k_emit<<<gt, TB, 0, s>>>(D, tet_top, num, W.coff.p, d_out_t, d_out_a);
+      k_infinity<<<1, 128, 0, s>>>(D, W.ci.p, nc, W.ccount.p, W.hullcnt.p, W.hull.p, num, W.coff.p, d_out_t, d_out_a);
+      launches += 2;
+    } else {
+      W.newid.reserve(cap, "newid");
+      const ListNumber num{W.newid.p};
+      k_number<<<gt, TB, 0, s>>>(D, tet_top, W.cfill.p, W.newid.p);
+      k_emit<<<gt, TB, 0, s>>>(D, tet_top, num, W.coff.p, d_out_t, d_out_a);
+      k_infinity<<<(nc + 127) / 128, 128, 0, s>>>(D, W.ci.p, nc, W.ccount.p, W.hullcnt.p, W.hull.p, num, W.coff.p,
+                                                  d_out_t, d_out_a);
+      launches += 3;
+    }
     ck(cudaGetLastError(), "output kernels");
   }
   ck(cudaEventRecord(W.ev1, s), "event record");
