@@ -63,6 +63,20 @@ static __global__ void k_scan_add(uint32_t* out, const uint32_t* sums, uint32_t 
 }
 
 
+// Adds every thread's x to *out with one atomic per block (called by the whole
+// block): same-address atomics take about a nanosecond each, so one per thread
+// of a full grid costs more than the pass that counted.
+__device__ __forceinline__ void block_add(unsigned long long* out, unsigned long long x) {
+  __shared__ unsigned long long sum;
+  if (threadIdx.x == 0) sum = 0ull;
+  __syncthreads();
+  for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xFFFFFFFFu, x, o);
+  if ((threadIdx.x & 31u) == 0 && x) atomicAdd(&sum, x);
+  __syncthreads();
+  if (threadIdx.x == 0 && sum) atomicAdd(out, sum);
+  __syncthreads();
+}
+
 inline void ck(cudaError_t e, const char* what) {
   if (e != cudaSuccess) throw Error{WTET_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e)};
 }

@@ -78,7 +78,7 @@
 #define WTET_SHARED_MINB 8
 #endif
 #ifndef WTET_WRITE_MINB
-#define WTET_WRITE_MINB 8
+#define WTET_WRITE_MINB 6
 #endif
 // Rounds of at most this many uninserted points (with the stratum that may
 // join next) run inside k_rounds.
@@ -3366,8 +3366,8 @@ __global__ void k_check_quality(const float4* pts, uint32_t n, const uint4* tets
       if (s < 0) ++viol;
     }
   }
-  atomicAdd(&out[0], viol);
-  atomicAdd(&out[1], interior);
+  dev::block_add(&out[0], viol);
+  dev::block_add(&out[1], interior);
 }
 
 __global__ void k_normalize_plain(const float* xyz, uint64_t n, const uint32_t* mn, const uint32_t* mx, float4* out) {

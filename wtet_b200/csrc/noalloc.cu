@@ -21,6 +21,7 @@
 #include <string>
 
 #include "../../include/wtet.h"
+#include "devbuf.cuh"
 #include "engine.cuh"
 #include "exact.cuh"
 
@@ -127,8 +128,8 @@ __global__ void k_check(uint64_t n, const uint4* tets, const uint4* adj, uint64_
       if (s < 0) ++viol;
     }
   }
-  atomicAdd(&cnt[0], viol);
-  atomicAdd(&cnt[1], interior);
+  wtet::dev::block_add(&cnt[0], viol);
+  wtet::dev::block_add(&cnt[1], interior);
 }
 
 // The device address of g_scratch belongs to the context the module was

@@ -157,42 +157,62 @@ __global__ void __launch_bounds__(128) k_verify(const float4* pts, uint32_t n, c
       if (s < 0) ++viol;
     }
   }
-  atomicAdd(&out->finite, finite);
-  atomicAdd(&out->faces, faces);
-  atomicAdd(&out->violations, viol);
-  atomicAdd(&out->misoriented, mis);
-  atomicAdd(&out->broken, broken);
-  atomicAdd(&out->hull, hull);
-  atomicAdd(&out->bad_ids, bad);
+  dev::block_add(&out->finite, finite);
+  dev::block_add(&out->faces, faces);
+  dev::block_add(&out->violations, viol);
+  dev::block_add(&out->misoriented, mis);
+  dev::block_add(&out->broken, broken);
+  dev::block_add(&out->hull, hull);
+  dev::block_add(&out->bad_ids, bad);
 }
 
 // ---- canonical form ----
 
-// Finite rows: counted by their smallest vertex; infinity rows get perm NONE.
+// The order of a row's slots by vertex id as one of 24 codes: base 4, 3, 2
+// digits of the ranks of slots 0..2 among the ranks still free.  kOddRow: the row
+// repeats an id (no triangulation does), and ranks are taken from its ids.
+constexpr uint32_t kOddRow = 31u;
+__device__ __forceinline__ uint32_t row_code(const uint4& v) {
+  if (v.x == v.y || v.x == v.z || v.x == v.w || v.y == v.z || v.y == v.w || v.z == v.w) return kOddRow;
+  const uint32_t r0 = rank_in_row(v, 0), r1 = rank_in_row(v, 1), r2 = rank_in_row(v, 2);
+  return r0 * 6u + (r1 - (r1 > r0)) * 2u + (r2 - (r2 > r0) - (r2 > r1));
+}
+// Rank of slot j in a row with this code.
+__device__ __forceinline__ uint32_t code_rank(uint32_t code, uint32_t j) {
+  const uint32_t r0 = code / 6u, d1 = code % 6u / 2u, d2 = code & 1u;
+  const uint32_t r1 = d1 + (d1 >= r0);
+  const uint32_t lo = min(r0, r1), hi = max(r0, r1);
+  uint32_t r2 = d2 + (d2 >= lo);
+  r2 += r2 >= hi;
+  return j == 0 ? r0 : j == 1 ? r1 : j == 2 ? r2 : 6u - r0 - r1 - r2;
+}
+
+// Finite rows: counted by their smallest vertex; perm: the row's number within
+// its bucket (one atomic per row serves the count and the scatter), NONE for
+// infinity rows.
 __global__ void k_canon_count(const uint4* tets, uint64_t m, uint32_t n, uint32_t* hist, uint32_t* perm,
                               uint32_t* bad) {
   const uint32_t inf = n + 4;
   for (uint64_t r = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; r < m; r += uint64_t(gridDim.x) * blockDim.x) {
     const uint4 v = tets[r];
-    perm[r] = NONE;
+    uint32_t k = NONE;
     if (v.x > inf || v.y > inf || v.z > inf || v.w > inf) {
       atomicOr(bad, 1u);
-      continue;
+    } else if (!has(v, inf)) {
+      k = atomicAdd(&hist[min(min(v.x, v.y), min(v.z, v.w))], 1u);
     }
-    if (has(v, inf)) continue;
-    atomicAdd(&hist[sorted4(v).x], 1u);
+    perm[r] = k;
   }
 }
 
 // Scatter into buckets (order inside a bucket is arbitrary; ranked next).
-__global__ void k_canon_scatter(const uint4* tets, uint64_t m, uint32_t n, uint32_t* cursor, uint4* rows,
+__global__ void k_canon_scatter(const uint4* tets, uint64_t m, const uint32_t* bstart, const uint32_t* perm, uint4* rows,
                                 uint32_t* lead) {
-  const uint32_t inf = n + 4;
   for (uint64_t r = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; r < m; r += uint64_t(gridDim.x) * blockDim.x) {
-    const uint4 v = tets[r];
-    if (v.x > inf || v.y > inf || v.z > inf || v.w > inf || has(v, inf)) continue;
-    const uint4 s = sorted4(v);
-    const uint32_t i = atomicAdd(&cursor[s.x], 1u);
+    const uint32_t k = perm[r];
+    if (k == NONE) continue;
+    const uint4 s = sorted4(tets[r]);
+    const uint32_t i = bstart[s.x] + k;
     rows[i] = make_uint4(s.y, s.z, s.w, uint32_t(r));
     lead[i] = s.x;
   }
@@ -205,9 +225,11 @@ __device__ __forceinline__ bool row_less(const uint4& a, const uint4& b) {
   return a.w < b.w;  // duplicate rows (invalid input) keep a strict order by source row
 }
 
-// Final position of each row: bucket start + rank inside the bucket.
-__global__ void k_canon_place(const uint4* rows, const uint32_t* lead, const uint32_t* bstart, uint64_t k,
-                              uint4* out_t, uint32_t* perm, uint32_t* srcof) {
+// Final position of each row: bucket start + rank inside the bucket.  perm:
+// (position << 5) | the row's slot order, all that a neighbour needs to know of
+// it (its ids would be a random 16-byte gather per face).
+__global__ void k_canon_place(const uint4* tets, const uint4* rows, const uint32_t* lead, const uint32_t* bstart,
+                              uint64_t k, uint4* out_t, uint32_t* perm, uint32_t* srcof) {
   for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < k; i += uint64_t(gridDim.x) * blockDim.x) {
     const uint4 me = rows[i];
     const uint32_t a = lead[i];
@@ -216,7 +238,7 @@ __global__ void k_canon_place(const uint4* rows, const uint32_t* lead, const uin
     for (uint32_t j = b0; j < b1; ++j) rank += row_less(rows[j], me) ? 1u : 0u;
     const uint32_t dst = b0 + rank;
     out_t[dst] = make_uint4(a, me.x, me.y, me.z);
-    perm[me.w] = dst;
+    perm[me.w] = (dst << 5) | row_code(tets[me.w]);
     srcof[dst] = me.w;
   }
 }
@@ -225,17 +247,19 @@ __global__ void k_canon_adj(const uint4* tets, const uint4* adj, uint64_t m, uin
                             const uint32_t* srcof, uint4* out_a) {
   for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < k; i += uint64_t(gridDim.x) * blockDim.x) {
     const uint32_t r = srcof[i];
-    const uint4 v = tets[r];
     const uint4 a = adj[r];
+    const uint32_t mine = perm[r] & 31u;
     uint4 o = make_uint4(NONE, NONE, NONE, NONE);
+#pragma unroll
     for (int j = 0; j < 4; ++j) {
       const uint32_t x = cmp4(a, j);
       uint32_t val = NONE;
-      if (x != NONE) {
-        const uint64_t nb = x >> 5;
-        if (nb < m && perm[nb] != NONE) val = (perm[nb] << 5) | rank_in_row(tets[nb], int(x & 3u));
+      if (x != NONE && (x >> 5) < m) {
+        const uint32_t w = perm[x >> 5];
+        if (w != NONE)
+          val = (w & ~31u) | ((w & 31u) == kOddRow ? rank_in_row(tets[x >> 5], int(x & 3u)) : code_rank(w & 31u, x & 3u));
       }
-      const uint32_t s = rank_in_row(v, j);
+      const uint32_t s = mine == kOddRow ? rank_in_row(tets[r], j) : code_rank(mine, uint32_t(j));
       if (s == 0) o.x = val;
       else if (s == 1) o.y = val;
       else if (s == 2) o.z = val;
@@ -247,7 +271,7 @@ __global__ void k_canon_adj(const uint4* tets, const uint4* adj, uint64_t m, uin
 
 struct VerifyWorkspace {
   dev::DBuf<float4> pts;
-  dev::DBuf<uint32_t> box, hist, cursor, lead, perm, srcof, bad;
+  dev::DBuf<uint32_t> box, hist, lead, perm, srcof, bad;
   dev::DBuf<uint4> rows;
   dev::DBuf<VerifyCounts> cnt;
   std::vector<dev::DBuf<uint32_t>> scan_tmp;
@@ -321,13 +345,10 @@ uint64_t canonicalize_device(const uint32_t* d_tets, const uint32_t* d_adj, uint
   ck(cudaStreamSynchronize(s), "canon count");
   if (bad) throw Error{WTET_ERR_ARG, "a tet refers to a vertex beyond the infinity vertex n+4"};
   const uint64_t k = k32;
-  // each bucket's fill cursor starts at the bucket's start
-  W.cursor.reserve(nb + 1, "canon cursor");
-  ck(cudaMemcpyAsync(W.cursor.p, W.hist.p, (nb + 1) * 4ull, cudaMemcpyDeviceToDevice, s), "d2d");
-  if (m) k_canon_scatter<<<g, 256, 0, s>>>(T, m, uint32_t(n), W.cursor.p, W.rows.p, W.lead.p);
+  if (m) k_canon_scatter<<<g, 256, 0, s>>>(T, m, W.hist.p, W.perm.p, W.rows.p, W.lead.p);
   if (k) {
     const uint32_t gk = grid_for(k, 256, 148 * 32);
-    k_canon_place<<<gk, 256, 0, s>>>(W.rows.p, W.lead.p, W.hist.p, k, reinterpret_cast<uint4*>(d_out_t), W.perm.p,
+    k_canon_place<<<gk, 256, 0, s>>>(T, W.rows.p, W.lead.p, W.hist.p, k, reinterpret_cast<uint4*>(d_out_t), W.perm.p,
                                      W.srcof.p);
     k_canon_adj<<<gk, 256, 0, s>>>(T, A, m, k, W.perm.p, W.srcof.p, reinterpret_cast<uint4*>(d_out_a));
   }
@@ -342,7 +363,6 @@ void release_verify_workspace() {
   w.pts.release();
   w.box.release();
   w.hist.release();
-  w.cursor.release();
   w.lead.release();
   w.perm.release();
   w.srcof.release();
