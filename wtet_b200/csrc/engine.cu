@@ -109,7 +109,11 @@ constexpr uint32_t WALK_LIMIT = 1u << 22;
 // that the cavity search takes better-keyed winners first: a winner that
 // meets a better one's claims then stops at its first contested tet instead
 // of completing a cavity it loses later.
-constexpr uint32_t kOrderBuckets = 16;
+// Finer order (64, 256 buckets) measured no faster on the 8M mixture (186.5 and
+// 192.5 ms against 186.6), ordering inside windows of the curve for L2 reuse
+// slower (190 ms with 8 windows, 198 with 16).
+constexpr uint32_t kOrderBits = 4;
+constexpr uint32_t kOrderBuckets = 1u << kOrderBits;
 constexpr int ROT_LIMIT = 1 << 16;
 constexpr int kMaxLevels = 15;
 
@@ -134,11 +138,13 @@ struct Counters {
   uint32_t n_freed_next;  // tets retired this round
   uint32_t n_inserted;    // winners this round
   uint32_t huge_used;     // huge-cavity slots used
+  uint32_t n_starts;      // vote winners that start a search
   uint32_t nbigw;         // winners whose star a whole block writes
   uint32_t work[3];       // dynamic work cursors of k_bfs, k_shared, k_write
   uint32_t ticket;        // blocks that have finished the round's last kernel
   uint32_t err;           // error flags when the round ended
-  uint32_t sbc[kOrderBuckets + 1];  // starts per order bucket (the last: overflow region)
+  uint32_t n_ovf;         // starts in the overflow region
+  uint32_t sbc[kOrderBuckets];  // starts per order bucket
 };
 
 // Totals of a run.
@@ -858,33 +864,48 @@ __global__ void k_init_clouds(const CloudInfo* ci, uint32_t nc, Dev D) {
 
 // ---------------------------------------------------------------- rounds ----
 
-// Prefix of the order buckets' start counts, in shared memory (sp has
-// kOrderBuckets + 2 entries; sp[kOrderBuckets + 1] is the total).  Called by
+// Prefix of the order buckets' start counts, in shared memory (sp[kOrderBuckets]:
+// the overflow region's first, sp[kOrderBuckets + 1]: the total).  Called by
 // every thread of the block.
 __device__ __forceinline__ void load_start_prefix(const Dev& D, const RoundArgs& R, uint32_t* sp) {
-  if (threadIdx.x == 0) {
-    uint32_t acc = 0, cnt[kOrderBuckets + 1];
+  constexpr uint32_t per = (kOrderBuckets + 31u) / 32u;
+  if (threadIdx.x < 32) {
+    uint32_t cnt[per], sum = 0;
 #pragma unroll
-    for (uint32_t b = 0; b <= kOrderBuckets; ++b) cnt[b] = __ldcg(&R.ctr->sbc[b]);
-#pragma unroll
-    for (uint32_t b = 0; b <= kOrderBuckets; ++b) {
-      sp[b] = acc;
-      acc += b < kOrderBuckets ? min(cnt[b], D.start_rc) : cnt[b];
+    for (uint32_t i = 0; i < per; ++i) {
+      const uint32_t b = threadIdx.x * per + i;
+      cnt[i] = b < kOrderBuckets ? min(__ldcg(&R.ctr->sbc[b]), D.start_rc) : 0u;
+      sum += cnt[i];
     }
-    sp[kOrderBuckets + 1] = acc;
+    const uint32_t ovf = __ldcg(&R.ctr->n_ovf);
+    uint32_t x = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+      if (threadIdx.x >= uint32_t(o)) x += y;
+    }
+    uint32_t acc = x - sum;
+#pragma unroll
+    for (uint32_t i = 0; i < per; ++i) {
+      if (threadIdx.x * per + i < kOrderBuckets) sp[threadIdx.x * per + i] = acc;
+      acc += cnt[i];
+    }
+    if (threadIdx.x == 31) {
+      sp[kOrderBuckets] = x;
+      sp[kOrderBuckets + 1] = x + ovf;
+    }
   }
   __syncthreads();
 }
 
 // Start i of the round in bucket order.
 __device__ __forceinline__ uint2 start_at(const Dev& D, const uint32_t* sp, uint32_t i) {
-  uint32_t b = 0;
+  uint32_t b = 0;  // the last bucket whose first start is at most i
 #pragma unroll
-  for (uint32_t k = 1; k <= kOrderBuckets; ++k) b += i >= sp[k] ? 1u : 0u;
+  for (uint32_t step = kOrderBuckets; step; step >>= 1)
+    if (b + step <= kOrderBuckets && sp[b + step] <= i) b += step;
   const uint32_t region = b < kOrderBuckets ? b * D.start_rc : D.start_ovf;
   return D.starts[region + (i - sp[b])];
 }
-
 
 // Inverse of mix32: recovers the point that owns a claim key.
 __device__ __forceinline__ uint32_t unmix32(uint32_t h) {
@@ -1022,13 +1043,13 @@ __device__ __forceinline__ void cands_body(const Dev& D, const RoundArgs& R, con
           const float pr = 1.f / (1.f + __expf(-sc));
           const uint32_t prio = 1u + uint32_t(fminf(pr * 1022.f + 0.5f, 1022.f));
           D.prio[p] = uint16_t(prio);
-          b = prio >> 6;  // 16 order buckets
+          b = prio >> (10 - kOrderBits);
         }
         __syncwarp();
       }
     } else {
       if (start && D.prio) D.prio[p] = 1;
-      b = start ? (mix32(p ^ (R.round * 0x9E3779B9u)) >> 28) : 0u;
+      b = start ? (mix32(p ^ (R.round * 0x9E3779B9u)) >> (32 - kOrderBits)) : 0u;
     }
     if (start && D.prefilter) pre_claim(D, t, start_key(D, R, p));
     const unsigned grp = __match_any_sync(0xFFFFFFFFu, start ? b : 0xFFFFFFFFu);
@@ -1041,7 +1062,7 @@ __device__ __forceinline__ void cands_body(const Dev& D, const RoundArgs& R, con
       if (slot < D.start_rc) {
         D.starts[b * D.start_rc + slot] = make_uint2(p, t);
       } else {  // a bucket beyond its region (never expected): the overflow region
-        D.starts[D.start_ovf + atomicAdd(&R.ctr->sbc[kOrderBuckets], 1u)] = make_uint2(p, t);
+        D.starts[D.start_ovf + atomicAdd(&R.ctr->n_ovf, 1u)] = make_uint2(p, t);
       }
     }
   }
@@ -1071,7 +1092,7 @@ __global__ void __launch_bounds__(256) k_cands_learned(Dev D) {
 // Cavity growth by groups of kBfsLanes lanes, kWarpGroups at a time per warp:
 // a group tests kBfsLanes (queued tet, face) pairs per pass, so a pass costs
 // one dependent chain (record -> insphere -> claim), and a warp keeps several
-// such chains in flight.  A warp takes up to 32 starts per fetch: each lane
+// such chains in flight.  A warp takes kStartChunk starts per fetch: each lane
 // checks one start's pre-claims (the four neighbours' words in one trip for
 // the whole warp), the survivors -- about half of them -- are handed to the
 // lane groups one by one, and a group that finishes takes the next survivor
@@ -1096,6 +1117,10 @@ constexpr uint32_t kBfsFaces = 48;   // boundary faces per group in shared memor
 // A cavity of K tets joined through at least K - 1 faces has at most 2K + 2 boundary faces.
 constexpr uint32_t kMaxFaces = 2 * BIG_CAP + 2;
 constexpr uint32_t kScratchWords = BIG_CAP + 2 * kMaxFaces;
+// Starts a warp takes per fetch in large rounds.  More in flight means more
+// searches that run beside a better one they would have found claims of: 8M
+// mixture 186.6 ms with 8, 195 with 32; with 4 the filter's trips show (191).
+constexpr uint32_t kStartChunk = 8;
 constexpr uint32_t kPoolChunk = 512;  // pool words a lane group reserves at a time
 
 template <uint32_t kWarps, uint32_t kBfsLanes>
@@ -1253,8 +1278,9 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
   constexpr uint32_t kWarpGroups = 32 / kBfsLanes;
   constexpr uint32_t FULL = 0xFFFFFFFFu, GM = (kBfsLanes == 32) ? 0xFFFFFFFFu : ((1u << kBfsLanes) - 1u);
   // the next round's counters (their last readers finished with the last round)
-  if (blockIdx.x == 0 && threadIdx.x < sizeof(Counters) / 4)
-    reinterpret_cast<uint32_t*>(D.ctr + (1u - uint32_t(R.ctr - D.ctr)))[threadIdx.x] = 0u;
+  if (blockIdx.x == 0)
+    for (uint32_t i = threadIdx.x; i < sizeof(Counters) / 4; i += blockDim.x)
+      reinterpret_cast<uint32_t*>(D.ctr + (1u - uint32_t(R.ctr - D.ctr)))[i] = 0u;
   // one block per huge candidate, before the block's share of the starts
   const uint32_t nhuge = min(__ldcg(&R.ctr->huge_used), HUGE_SLOTS);
   for (uint32_t bi = blockIdx.x; bi < nhuge; bi += gridDim.x) expand_big(D, R, bi, sm.huge);
@@ -1271,12 +1297,13 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
   if (threadIdx.x == 0) sm.searches = 0;
   load_start_prefix(D, R, sm.sp);
   const uint32_t nstart = sm.sp[kOrderBuckets + 1];
+  if (blockIdx.x == 0 && threadIdx.x == 0) R.ctr->n_starts = nstart;
   const uint32_t nwarps = gridDim.x * kWarps;
-  // About four fetches per warp, between one start per lane group and one per lane.
-  const uint32_t chunk = min(32u, max(kWarpGroups, nstart / (4u * nwarps)));
+  // About four fetches per warp, between one start per lane group and kStartChunk.
+  const uint32_t chunk = min(kStartChunk, max(kWarpGroups, nstart / (4u * nwarps)));
   // Same-address atomics serialise, so in large rounds a group reserves several
   // cavities' worth of pool at a time (small ones would run out of pool).
-  const uint32_t pool_chunk = chunk == 32u ? kPoolChunk : 0u;
+  const uint32_t pool_chunk = chunk == kStartChunk ? kPoolChunk : 0u;
   unsigned long long searches = 0;
   uint32_t pool_at = 0, pool_end = 0;  // the group's reserved pool words
   const uint32_t lgrp = lane / kBfsLanes;
@@ -2305,9 +2332,7 @@ __device__ __forceinline__ void end_round(const Dev& D, State& S, const Counters
     S.stratum_size = ns.total;
     S.strata += 1;
   }
-  uint32_t starts = 0;
-#pragma unroll
-  for (uint32_t b = 0; b < kOrderBuckets; ++b) starts += __ldcg(&C->sbc[b]);
+  const uint32_t starts = __ldcg(&C->n_starts);
   S.inserted += __ldcg(&C->n_inserted);
   S.starts += starts + min(__ldcg(&C->huge_used), HUGE_SLOTS);
   S.last_starts = starts;
@@ -3017,7 +3042,7 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
   W.bigcand.reserve(HUGE_SLOTS, "bigcand");
   // order-bucket regions: the expected n / kOrderBuckets starts per bucket
   // plus a 25% margin; anything beyond goes to the overflow region
-  const uint64_t start_rc = n / kOrderBuckets + n / 64 + 1024;
+  const uint64_t start_rc = n / kOrderBuckets + n / (4 * kOrderBuckets) + 256;
   const uint64_t start_ovf = start_rc * kOrderBuckets;
   W.starts.reserve(start_ovf + n, "starts");
   // one overflow region per lane group of a k_bfs wave, one edge table per
