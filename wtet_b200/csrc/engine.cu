@@ -199,15 +199,19 @@ struct alignas(16) State {
 // visited tet costs one trip (claim, links and coordinates together) instead
 // of two (ids, then four points), and its words share one DRAM page and one
 // address translation.
+//
+// Sectors (32 bytes) by who reads them together: links, claim and vote (the
+// search, the walks, the candidates); X and Y; Z and ids; the rest.  A tested
+// tet is three sectors.
 struct __align__(128) Tet {
-  uint4 v;
   uint4 n;
   unsigned long long cav;
-  unsigned long long pre;
   unsigned long long vote;
-  unsigned long long pad;
   float4 X, Y, Z;  // .x/.y/.z/.w: vertices 0..3
+  uint4 v;
   uint4 slot;
+  unsigned long long pre;
+  unsigned long long pad;
 };
 static_assert(sizeof(Tet) == 128, "one tet slot is one 128-byte line");
 
@@ -1374,9 +1378,11 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
           head = 0;
           lost = overflow = false;
           running = true;
+          pend = ~0ull;
           if (gl == 0) {
             sq[0] = t_s;
             sn[0] = make_uint4(n0, n1, n2, n3);
+            pend = atomicMin(&D.T[t_s].cav, key);
           }
           // the slot set_add() looks at first holds t0 from the start
 #pragma unroll
@@ -1386,72 +1392,49 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
                 make_uint4(w == h ? t_s : NONE, w + 1u == h ? t_s : NONE, w + 2u == h ? t_s : NONE,
                            w + 3u == h ? t_s : NONE);
           }
-          pend = ~0ull;
         }
         __syncwarp();
       } else if (!busy) {
         break;  // nothing left to hand out
       }
       // ---- one pass: kBfsLanes (queued tet, face) pairs of each group
-      bool add = false, bnd = false, my_lost = false, my_guard = false;
-      uint32_t nt = 0, code = 0, outer = NONE;
-      uint4 nn = make_uint4(NONE, NONE, NONE, NONE);
-      // a search that outgrew its set tells tets apart by its claims alone: all
-      // of them must have arrived
-      if (running && K > kHashTets && pend != ~0ull) {
-        my_lost = pend < key;
-        displaced(D, R, key, pend);
-        pend = ~0ull;
-      }
-      unsigned long long old0 = ~0ull;
-      if (fresh && gl == 0) old0 = atomicMin(&D.T[sq[0]].cav, key);
-      const uint32_t idx = head + gl / 4u;
-      const uint32_t f = gl & 3u;
-      if (running && idx < K) {
-        const uint32_t c = idx < kBfsShared ? sq[idx] : gq[idx];
+      const uint32_t idx = head + gl / 4u, f = gl & 3u;
+      const bool pair = running && idx < K;
+      uint32_t c = 0, outer = NONE;
+      if (pair) {
+        c = idx < kBfsShared ? sq[idx] : gq[idx];
         outer = idx < kBfsShared ? comp(sn[idx], int(f)) : reinterpret_cast<const uint32_t*>(&D.T[c].n)[f];
-        code = (c << 2) | f;
-        nt = outer >> 2;
-        if (outer == NONE) {
+      }
+      const uint32_t code = (c << 2) | f, nt = outer >> 2;
+      bool bnd = pair && outer == NONE, add = false;
+      const bool my_guard = pair && outer != NONE && nt >= D.cap;
+      const bool test = pair && outer != NONE && nt < D.cap;
+      // One round trip: claim, neighbours and coordinates together (lanes with
+      // no pair read slot 0, so that no branch stands between the loads and
+      // what follows).
+      const Tet* T = D.T + (test ? nt : 0u);
+      const unsigned long long cc = __ldcg(&T->cav);
+      const uint4 nn = ld_u4(&T->n);
+      const float4 X = ld_f4(&T->X), Y = ld_f4(&T->Y), Z = ld_f4(&T->Z);
+      // The answers to the last pass's claims, which have had a pass to arrive.
+      // Every lane's are looked at here, before new claims are issued: a
+      // register that a claim in flight is to write makes the whole warp wait.
+      bool my_lost = pend < key;
+      displaced(D, R, key, pend);
+      pend = ~0ull;
+      if (test && cc != key) {
+        if (in_sphere(D, T, X, Y, Z, pq, p) >= 0) {
           bnd = true;
-        } else if (nt >= D.cap) {
-          my_guard = true;
+        } else if (cc < key) {
+          my_lost = true;  // a better claim holds it
+        } else if (K <= kHashTets) {
+          add = set_add(set, nt);
+          if (add) pend = atomicMin(&D.T[nt].cav, key);
         } else {
-          // one round trip: claim, neighbours and coordinates together
-          const Tet* T = D.T + nt;
-          const unsigned long long cc = __ldcg(&T->cav);
-          nn = ld_u4(&T->n);
-          const float4 X = ld_f4(&T->X), Y = ld_f4(&T->Y), Z = ld_f4(&T->Z);
-          // the last pass's claims, and the fresh search's own tet
-          my_lost = my_lost || pend < key || old0 < key;
-          displaced(D, R, key, pend);
-          displaced(D, R, key, old0);
-          pend = old0 = ~0ull;
-          if (cc != key) {
-            if (in_sphere(D, T, X, Y, Z, pq, p) >= 0) {
-              bnd = true;
-            } else if (cc < key) {
-              my_lost = true;  // a better claim holds it
-            } else if (K <= kHashTets) {
-              add = set_add(set, nt);
-              if (add) pend = atomicMin(&D.T[nt].cav, key);
-            } else {
-              unsigned long long old;
-              if (claim(D, R, nt, key, old)) my_lost = true;
-              else add = old != key;
-            }
-          }
+          unsigned long long old;
+          if (claim(D, R, nt, key, old)) my_lost = true;
+          else add = old != key;
         }
-      }
-      // answers not looked at above (no pair in this pass)
-      if (running && !add && pend != ~0ull) {
-        my_lost = my_lost || pend < key;
-        displaced(D, R, key, pend);
-        pend = ~0ull;
-      }
-      if (old0 != ~0ull) {
-        my_lost = my_lost || old0 < key;
-        displaced(D, R, key, old0);
       }
       const uint32_t aball = (__ballot_sync(FULL, add) >> shift) & GM;
       const uint32_t bball = (__ballot_sync(FULL, bnd) >> shift) & GM;
@@ -1485,14 +1468,14 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
         F += __popc(bball);
         running = !lost && !overflow && head < K;
         fin = !running;
-        // a search that ends lost still displaced what its last claims displaced
-        if (fin && pend != ~0ull) {
-          displaced(D, R, key, pend);
-          pend = ~0ull;
-        }
       }
       __syncwarp();
       if (!__any_sync(FULL, fin)) continue;
+      // a search that ends lost still displaced what its last claims displaced
+      if (fin) {
+        displaced(D, R, key, pend);
+        pend = ~0ull;
+      }
       // ---- finished searches: the cavity and its boundary go to the pool
       // Partial claims carry this round's key: the huge path takes it next round.
       if (fin && !lost && overflow && gl == 0) D.bigflag[p] = kPending | 2;
