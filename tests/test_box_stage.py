@@ -130,3 +130,40 @@ def test_bounded_permanent(kind):
             decided += 1
             assert sign(det) == sign(want)
     assert decided > (50 if kind == "lattice" else 400)
+
+
+def rough(p):
+    """insphere_f32's determinant and its bound on the permanent (f32 operations in its order)."""
+    f = np.float32
+    e = p[4]
+    d = [[f(p[i][k] - e[k]) for k in range(3)] for i in range(4)]
+    r = [max(abs(x) for x in q) for q in d]
+    factor = f(f(f(16.0) + f(f(224.0) * f(2.0 ** -24))) * f(2.0 ** -24)) * f(18.0) * f(1.0 + 3.0e-5)
+    bound = f(f(f(f(f(r[0] * r[1]) * f(factor)) * f(r[2] * r[3])) * f(f(r[0] + r[1]) + f(r[2] + r[3]))) + f(1e-33))
+    (ax, ay, az), (bx, by, bz), (cx, cy, cz), (dx, dy, dz) = d
+    m = lambda u, v, w, x: f(f(u * v) - f(w * x))  # noqa: E731
+    ab, bc, cd = m(ax, by, bx, ay), m(bx, cy, cx, by), m(cx, dy, dx, cy)
+    da, ac, bd = m(dx, ay, ax, dy), m(ax, cy, cx, ay), m(bx, dy, dx, by)
+    abc = f(f(f(az * bc) - f(bz * ac)) + f(cz * ab))
+    bcd = f(f(f(bz * cd) - f(cz * bd)) + f(dz * bc))
+    cda = f(f(f(cz * da) + f(dz * ac)) + f(az * cd))
+    dab = f(f(f(dz * ab) + f(az * bd)) + f(bz * da))
+    lift = [f(f(f(x * x) + f(y * y)) + f(z * z)) for x, y, z in d]
+    return f(f(f(lift[3] * abc) - f(lift[2] * dab)) + f(f(lift[1] * cda) - f(lift[0] * bcd))), bound
+
+
+@pytest.mark.parametrize("kind,scale", [("uniform", 1.0), ("super", 1.0), ("tiny", 1e-4), ("tiny", 1e-8), ("tiny", 1e-12)])
+def test_rough_bound(kind, scale):
+    r = np.random.default_rng(13)
+    sup = np.array([[-100, -100, -100], [400, -100, -100], [-100, 400, -100], [-100, -100, 400]], np.float32)
+    decided = 0
+    for _ in range(600):
+        p = (scale * r.random((5, 3))).astype(np.float32)
+        if kind == "super":
+            k = r.integers(1, 4)
+            p[r.choice(4, k, replace=False)] = sup[r.choice(4, k, replace=False)]
+        det, bound = rough(p)
+        want = insphere_value(p)
+        assert abs(Fraction(float(det)) - want) <= Fraction(float(bound))
+        decided += abs(det) > bound
+    assert decided > 500 or scale < 1e-4

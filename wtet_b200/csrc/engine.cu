@@ -534,11 +534,9 @@ __device__ __noinline__ int o4d_sos_call(float4 X, float4 Y, float4 Z, float4 e,
 // Insphere test of p (coordinates pq) against tet T, whose coordinates were
 // loaded with the record; its vertex ids are read only when the FP32 stage
 // cannot decide.
-__device__ __forceinline__ int in_sphere(const Dev& D, const Tet* T, const float4& X, const float4& Y,
-                                         const float4& Z, const float4& pq, uint32_t p) {
-  int s = ex::insphere_f32(corner(X, Y, Z, 0), corner(X, Y, Z, 1), corner(X, Y, Z, 2), corner(X, Y, Z, 3), pq);
-  if (s != 0) return s;
-  s = ex::insphere_mid(X, Y, Z, pq);
+__device__ __forceinline__ int in_sphere_rest(const Dev& D, const Tet* T, const float4& X, const float4& Y,
+                                              const float4& Z, const float4& pq, uint32_t p) {
+  const int s = ex::insphere_mid(X, Y, Z, pq);
   if (s == 1 || s == -1) return s;
   const uint4 V = ld_u4(&T->v);
   if (V.x >= D.nv || V.y >= D.nv || V.z >= D.nv || V.w >= D.nv) {
@@ -546,6 +544,11 @@ __device__ __forceinline__ int in_sphere(const Dev& D, const Tet* T, const float
     return 1;
   }
   return o4d_sos_rest(X, Y, Z, pq, V.x, V.y, V.z, V.w, p, D.sos, &D.tot->err, s);
+}
+__device__ __forceinline__ int in_sphere(const Dev& D, const Tet* T, const float4& X, const float4& Y,
+                                         const float4& Z, const float4& pq, uint32_t p) {
+  const int s = ex::insphere_f32(corner(X, Y, Z, 0), corner(X, Y, Z, 1), corner(X, Y, Z, 2), corner(X, Y, Z, 3), pq);
+  return s != 0 ? s : in_sphere_rest(D, T, X, Y, Z, pq, p);
 }
 
 // Visibility walk from tet t to the tet that contains p, and p's vote there.
@@ -1108,14 +1111,13 @@ __global__ void __launch_bounds__(256) k_cands_learned(Dev D) {
 // start in shared memory and continue in the group's global region; cavities
 // beyond BIG_CAP tets move to the huge path next round.
 //
-// A claim's answer is not waited for: a small set of the cavity's tets in
-// shared memory tells a new tet from one already found, and the answer (a
-// better claim: lost) is looked at in the next pass, after that pass has
-// issued its loads.  Once a cavity outgrows the set, claims are waited for and
-// tell the two apart themselves.
+// A claim's answer (a better claim: lost) is not waited for in its own pass but
+// looked at in the next one, after that pass has issued its record loads.  Only
+// then is the tested tet's claim word loaded -- by now every claim of the search
+// has been performed, so the word tells a tet of the cavity from a new one --
+// and it arrives while the FP32 stage computes.  Two lanes that meet one new
+// tet in the same pass are told apart by a warp match.
 constexpr uint32_t kBulkLanes = 16;  // lanes per search in large rounds; k_rounds has lanes to spare and uses 32
-constexpr uint32_t kHashSlots = 128;
-constexpr uint32_t kHashTets = 64;   // largest cavity at the start of a pass that uses the set (adds at most 32)
 constexpr uint32_t kBfsShared = 48;  // queue entries (tet + neighbour words) per group in shared memory
 constexpr uint32_t kBfsFaces = 48;   // boundary faces per group in shared memory
 // A cavity of K tets joined through at least K - 1 faces has at most 2K + 2 boundary faces.
@@ -1133,7 +1135,6 @@ struct BfsSmem {
   uint4 n[kGroups][kBfsShared];
   uint2 b[kGroups][kBfsFaces];
   uint32_t q[kGroups][kBfsShared];
-  __align__(16) uint32_t set[kGroups][kHashSlots];
   uint32_t sp[kOrderBuckets + 2];
   uint32_t huge[6];
   unsigned long long searches;
@@ -1266,17 +1267,6 @@ __device__ __forceinline__ void expand_big(const Dev& D, const RoundArgs& R, uin
   __syncthreads();
 }
 
-// Adds tet t to a search's set; false when it was there.
-__device__ __forceinline__ bool set_add(uint32_t* set, uint32_t t) {
-  uint32_t h = (t * 0x9E3779B1u) >> 25;  // 128 slots
-  for (;;) {  // ends: at most kHashTets + 32 tets in kHashSlots slots
-    const uint32_t o = atomicCAS(&set[h], NONE, t);
-    if (o == NONE) return true;
-    if (o == t) return false;
-    h = (h + 1) & (kHashSlots - 1);
-  }
-}
-
 template <uint32_t kWarps, uint32_t kBfsLanes>
 __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSmem<kWarps, kBfsLanes>& sm) {
   constexpr uint32_t kWarpGroups = 32 / kBfsLanes;
@@ -1295,7 +1285,6 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
   uint32_t* sq = sm.q[threadIdx.x / kBfsLanes];
   uint4* sn = sm.n[threadIdx.x / kBfsLanes];
   uint2* sb = sm.b[threadIdx.x / kBfsLanes];
-  uint32_t* set = sm.set[threadIdx.x / kBfsLanes];
   uint32_t* gq = D.wscratch + size_t(gid < D.wgroups ? gid : 0) * kScratchWords;
   uint2* gb = reinterpret_cast<uint2*>(gq + BIG_CAP);
   if (threadIdx.x == 0) sm.searches = 0;
@@ -1384,14 +1373,6 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
             sn[0] = make_uint4(n0, n1, n2, n3);
             pend = atomicMin(&D.T[t_s].cav, key);
           }
-          // the slot set_add() looks at first holds t0 from the start
-#pragma unroll
-          for (uint32_t i = 0; i < kHashSlots / 4 / kBfsLanes; ++i) {
-            const uint32_t w = 4u * (gl + i * kBfsLanes), h = (t_s * 0x9E3779B1u) >> 25;
-            reinterpret_cast<uint4*>(set)[w / 4u] =
-                make_uint4(w == h ? t_s : NONE, w + 1u == h ? t_s : NONE, w + 2u == h ? t_s : NONE,
-                           w + 3u == h ? t_s : NONE);
-          }
         }
         __syncwarp();
       } else if (!busy) {
@@ -1406,36 +1387,34 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
         outer = idx < kBfsShared ? comp(sn[idx], int(f)) : reinterpret_cast<const uint32_t*>(&D.T[c].n)[f];
       }
       const uint32_t code = (c << 2) | f, nt = outer >> 2;
-      bool bnd = pair && outer == NONE, add = false;
+      bool bnd = pair && outer == NONE;
       const bool my_guard = pair && outer != NONE && nt >= D.cap;
       const bool test = pair && outer != NONE && nt < D.cap;
-      // One round trip: claim, neighbours and coordinates together (lanes with
-      // no pair read slot 0, so that no branch stands between the loads and
-      // what follows).
+      // One round trip: neighbours and coordinates together (lanes with no pair
+      // read slot 0, so that no branch stands between the loads and their use).
       const Tet* T = D.T + (test ? nt : 0u);
-      const unsigned long long cc = __ldcg(&T->cav);
       const uint4 nn = ld_u4(&T->n);
       const float4 X = ld_f4(&T->X), Y = ld_f4(&T->Y), Z = ld_f4(&T->Z);
-      // The answers to the last pass's claims, which have had a pass to arrive.
-      // Every lane's are looked at here, before new claims are issued: a
+      // The answers to the last pass's claims, before new claims are issued: a
       // register that a claim in flight is to write makes the whole warp wait.
       bool my_lost = pend < key;
       displaced(D, R, key, pend);
       pend = ~0ull;
-      if (test && cc != key) {
-        if (in_sphere(D, T, X, Y, Z, pq, p) >= 0) {
-          bnd = true;
-        } else if (cc < key) {
-          my_lost = true;  // a better claim holds it
-        } else if (K <= kHashTets) {
-          add = set_add(set, nt);
-          if (add) pend = atomicMin(&D.T[nt].cav, key);
-        } else {
-          unsigned long long old;
-          if (claim(D, R, nt, key, old)) my_lost = true;
-          else add = old != key;
-        }
+      __syncwarp();
+      // after every lane's answers (the address depends on this lane's): see above
+      const unsigned long long cc = __ldcg(my_lost ? &D.T[0].cav : &T->cav);
+      int side = ex::insphere_f32(corner(X, Y, Z, 0), corner(X, Y, Z, 1), corner(X, Y, Z, 2), corner(X, Y, Z, 3), pq);
+      const bool open = test && !my_lost && cc != key;  // not a tet of the cavity (yet)
+      if (open && side == 0) side = in_sphere_rest(D, T, X, Y, Z, pq, p);
+      bnd = bnd || (open && side > 0);
+      bool fresh_tet = open && side < 0;
+      if (fresh_tet && cc < key) {
+        my_lost = true;  // a better claim holds it
+        fresh_tet = false;
       }
+      const uint32_t same = __match_any_sync(FULL, fresh_tet ? (nt * kWarpGroups + lgrp) : ~lane);
+      const bool add = fresh_tet && lane == uint32_t(__ffs(int(same))) - 1u;
+      if (add) pend = atomicMin(&D.T[nt].cav, key);
       const uint32_t aball = (__ballot_sync(FULL, add) >> shift) & GM;
       const uint32_t bball = (__ballot_sync(FULL, bnd) >> shift) & GM;
       const uint32_t pos = K + __popc(aball & lt), posb = F + __popc(bball & lt);
@@ -1455,19 +1434,28 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
         else if (posb < kMaxFaces) gb[posb] = make_uint2(code, outer);
         else my_over = true;
       }
-      const uint32_t g_guard = (__ballot_sync(FULL, my_guard) >> shift) & GM;
-      const uint32_t g_lost = (__ballot_sync(FULL, my_lost) >> shift) & GM;
-      const uint32_t g_over = (__ballot_sync(FULL, my_over) >> shift) & GM;
+      const uint32_t bad = __ballot_sync(FULL, my_lost || my_guard || my_over);
       bool fin = false;
       if (running) {
-        if (g_guard && gl == 0) atomicOr(&D.tot->err, kErrGuard);
-        lost = lost || g_lost || g_guard;
-        overflow = overflow || g_over;
         head = min(head + kBfsLanes / 4u, K);
         K += __popc(aball);
         F += __popc(bball);
-        running = !lost && !overflow && head < K;
+        running = head < K;
         fin = !running;
+      }
+      if (bad) {  // warp-uniform
+        const uint32_t g_guard = (__ballot_sync(FULL, my_guard) >> shift) & GM;
+        const uint32_t g_lost = (__ballot_sync(FULL, my_lost) >> shift) & GM;
+        const uint32_t g_over = (__ballot_sync(FULL, my_over) >> shift) & GM;
+        if (running || fin) {
+          if (g_guard && gl == 0) atomicOr(&D.tot->err, kErrGuard);
+          lost = lost || g_lost || g_guard;
+          overflow = overflow || g_over;
+          if (lost || overflow) {
+            running = false;
+            fin = true;
+          }
+        }
       }
       __syncwarp();
       if (!__any_sync(FULL, fin)) continue;

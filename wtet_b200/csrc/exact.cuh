@@ -654,6 +654,7 @@ __device__ __forceinline__ int insphere(const double* pa, const double* pb, cons
 constexpr float kEpsF = 5.9604644775390625e-08f;  // 2^-24
 constexpr float kO3dBoundF = (7.0f + 56.0f * kEpsF) * kEpsF;
 constexpr float kIspBoundF = (16.0f + 224.0f * kEpsF) * kEpsF;
+constexpr float kIspRoughF = kIspBoundF * 18.0f * (1.0f + 3.0e-5f);
 // Permanents below this get no answer (typical permanents of the benchmark
 // clouds are above 1e-16).
 constexpr float kPermMinF = 1.0e-26f;
@@ -711,6 +712,19 @@ __device__ __forceinline__ int insphere_f32(const float4& pa, const float4& pb, 
   const float dlift = __fadd_rn(__fadd_rn(__fmul_rn(dex, dex), __fmul_rn(dey, dey)), __fmul_rn(dez, dez));
   const float det = __fadd_rn(__fsub_rn(__fmul_rn(dlift, abc), __fmul_rn(clift, dab)),
                               __fsub_rn(__fmul_rn(blift, cda), __fmul_rn(alift, bcd)));
+  // First against a bound on the permanent (see insphere_mid): fifteen
+  // operations instead of the permanent's thirty-three decide nearly every test
+  // of points in general position.  Its factor covers the r_i's and its own
+  // rounding; products that underflow are covered by the slack.
+  const float ra = fmaxf(fmaxf(fabsf(aex), fabsf(aey)), fabsf(aez)), rb = fmaxf(fmaxf(fabsf(bex), fabsf(bey)), fabsf(bez));
+  const float rc = fmaxf(fmaxf(fabsf(cex), fabsf(cey)), fabsf(cez)), rd = fmaxf(fmaxf(fabsf(dex), fabsf(dey)), fabsf(dez));
+  const float rough = __fadd_rn(__fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(ra, rb), kIspRoughF), __fmul_rn(rc, rd)),
+                                          __fadd_rn(__fadd_rn(ra, rb), __fadd_rn(rc, rd))),
+                                kUnderflowSlackF);
+  if (rough < 1.0e30f) {
+    if (det > rough) return 1;
+    if (-det > rough) return -1;
+  }
   const float az = fabsf(aez), bz = fabsf(bez), cz = fabsf(cez), dz = fabsf(dez);
   const float p_ab = __fadd_rn(fabsf(aexbey), fabsf(bexaey)), p_bc = __fadd_rn(fabsf(bexcey), fabsf(cexbey));
   const float p_cd = __fadd_rn(fabsf(cexdey), fabsf(dexcey)), p_da = __fadd_rn(fabsf(dexaey), fabsf(aexdey));
