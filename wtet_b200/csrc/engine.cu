@@ -1117,7 +1117,11 @@ __global__ void __launch_bounds__(256) k_cands_learned(Dev D) {
 // has been performed, so the word tells a tet of the cavity from a new one --
 // and it arrives while the FP32 stage computes.  Two lanes that meet one new
 // tet in the same pass are told apart by a warp match.
-constexpr uint32_t kBulkLanes = 16;  // lanes per search in large rounds; k_rounds has lanes to spare and uses 32
+// Lanes per search: a round with searches for every half warp runs two per
+// warp; smaller rounds have lanes to spare (32 in all rounds: 250k sphere 25.0 ms
+// against 27.4 with 16, 8M mixture 178 against 172; 8 lanes: 32.6 and 187).
+constexpr uint32_t kBulkLanes = 16;
+constexpr uint32_t kWideRoundPoints = 65536;  // rounds of at most this many points use 32
 constexpr uint32_t kBfsShared = 48;  // queue entries (tet + neighbour words) per group in shared memory
 constexpr uint32_t kBfsFaces = 48;   // boundary faces per group in shared memory
 // A cavity of K tets joined through at least K - 1 faces has at most 2K + 2 boundary faces.
@@ -1519,8 +1523,12 @@ __device__ __forceinline__ void bfs_body(const Dev& D, const RoundArgs& R, BfsSm
 __global__ void __launch_bounds__(128, WTET_BFS_MINB) k_bfs(Dev D) {
   const RoundArgs R = load_round(D);
   if (!R.live) return;
-  __shared__ BfsSmem<4, kBulkLanes> sm;
-  bfs_body<4, kBulkLanes>(D, R, sm);
+  __shared__ union {
+    BfsSmem<4, kBulkLanes> narrow;
+    BfsSmem<4, 32> wide;
+  } sm;
+  if (R.n_active <= kWideRoundPoints) bfs_body<4, 32>(D, R, sm.wide);
+  else bfs_body<4, kBulkLanes>(D, R, sm.narrow);
 }
 
 __device__ __forceinline__ uint32_t slot_of(const Dev& D, const RoundArgs& R, uint32_t v) {
@@ -1545,7 +1553,7 @@ __device__ __forceinline__ uint32_t edge_hi(const uint4& V, int f, int k) {
 // worse winner p's new tet on f (then either insertion order gives the same
 // tets).  The worse one of a violating pair steps back.  A winner that stays
 // is handed its slots in the same pass.  One lane per boundary face of the
-// list that the search wrote; the loads of up to kChunk winners are issued
+// list that the search wrote; the loads of kCh winners are issued
 // together (records, then faces, then the outer tets' claims), because each
 // of them is one random trip.  cwin: first new slot (virtual), flags, the
 // faces of the first 32 that another cavity of this round touches.
@@ -1558,22 +1566,21 @@ constexpr uint32_t kBigWinners = 4096;
 constexpr uint32_t kBlockFaces = 340;
 constexpr uint32_t kBlockFacesSmall = 64;
 
-template <uint32_t kWarps, uint32_t kBlock>
+template <uint32_t kWarps, uint32_t kBlock, uint32_t kCh>
 __device__ __forceinline__ void shared_body(const Dev& D, const RoundArgs& R) {
   constexpr uint32_t FULL = 0xFFFFFFFFu;
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t ncand = __ldcg(&R.ctr->n_cand);
-  const uint32_t ch = chunk_for(ncand);
   const uint32_t nwarps = gridDim.x * kWarps;
   const uint16_t stamp = uint16_t(R.round);
-  for (uint32_t c0 = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * ch; c0 < ncand;
-       c0 = nwarps * ch + warp_next(&R.ctr->work[1], ch)) {
+  for (uint32_t c0 = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * kCh; c0 < ncand;
+       c0 = nwarps * kCh + warp_next(&R.ctr->work[1], kCh)) {
     // the chunk's records, one per lane; a cavity that lost a tet is out
     uint4 rec_l = make_uint4(0, 0, 0, 0);
     uint32_t bf_l = 0;
     unsigned long long key_l = 0;
     bool alive = false;
-    if (lane < ch && c0 + lane < ncand) {
+    if (lane < kCh && c0 + lane < ncand) {
       rec_l = ld_u4(&D.cand[c0 + lane]);
       bf_l = D.cand_bf[c0 + lane];
       key_l = make_key(D, R, rec_l.x);
@@ -1582,11 +1589,11 @@ __device__ __forceinline__ void shared_body(const Dev& D, const RoundArgs& R) {
     const uint32_t live = __ballot_sync(FULL, alive);
     if (!live) continue;
     // faces, then the claims of the tets beyond them (first 32 of each winner)
-    uint2 e[kChunk];
-    unsigned long long key[kChunk], cc[kChunk];
-    uint32_t F[kChunk];
+    uint2 e[kCh];
+    unsigned long long key[kCh], cc[kCh];
+    uint32_t F[kCh];
 #pragma unroll
-    for (uint32_t j = 0; j < kChunk; ++j) {
+    for (uint32_t j = 0; j < kCh; ++j) {
       F[j] = (live >> j) & 1u ? __shfl_sync(FULL, rec_l.w, int(j)) : 0u;
       key[j] = __shfl_sync(FULL, key_l, int(j));
       const uint32_t bfo = __shfl_sync(FULL, bf_l, int(j));
@@ -1594,12 +1601,12 @@ __device__ __forceinline__ void shared_body(const Dev& D, const RoundArgs& R) {
       if (lane < F[j]) e[j] = reinterpret_cast<const uint2*>(D.pool + bfo)[lane];
     }
 #pragma unroll
-    for (uint32_t j = 0; j < kChunk; ++j) cc[j] = e[j].y != NONE ? __ldcg(&D.T[e[j].y >> 2].cav) : ~0ull;
-    uint32_t touch[kChunk], base[kChunk], fresh[kChunk];
+    for (uint32_t j = 0; j < kCh; ++j) cc[j] = e[j].y != NONE ? __ldcg(&D.T[e[j].y >> 2].cav) : ~0ull;
+    uint32_t touch[kCh], base[kCh], fresh[kCh];
     uint32_t sum = 0;
     bool keep_l = false;  // this lane's winner stays
 #pragma unroll
-    for (uint32_t j = 0; j < kChunk; ++j) {
+    for (uint32_t j = 0; j < kCh; ++j) {
       const uint32_t p = __shfl_sync(FULL, rec_l.x, int(j)), K = __shfl_sync(FULL, rec_l.z, int(j));
       const uint32_t off = __shfl_sync(FULL, rec_l.y, int(j)), bfo = __shfl_sync(FULL, bf_l, int(j));
       bool bad = false, mine = false;
@@ -1645,7 +1652,7 @@ __device__ __forceinline__ void shared_body(const Dev& D, const RoundArgs& R) {
     b0 = __shfl_sync(FULL, b0, 0);
     uint32_t flags_l = 0, base_l = 0, touch_l = 0;
 #pragma unroll
-    for (uint32_t j = 0; j < kChunk; ++j) {
+    for (uint32_t j = 0; j < kCh; ++j) {
       if (!F[j]) continue;  // warp-uniform
       const uint32_t K = __shfl_sync(FULL, rec_l.z, int(j)), off = __shfl_sync(FULL, rec_l.y, int(j));
       const uint32_t bfo = __shfl_sync(FULL, bf_l, int(j));
@@ -1702,7 +1709,8 @@ __device__ __forceinline__ void shared_body(const Dev& D, const RoundArgs& R) {
 __global__ void __launch_bounds__(128, WTET_SHARED_MINB) k_shared(Dev D) {
   const RoundArgs R = load_round(D);
   if (!R.live) return;
-  shared_body<4, kBlockFaces>(D, R);
+  if (chunk_for(__ldcg(&R.ctr->n_cand)) == kChunk) shared_body<4, kBlockFaces, kChunk>(D, R);
+  else shared_body<4, kBlockFaces, 1>(D, R);
 }
 
 // Writes the new tets of every winner.  The three faces through p of a new
@@ -2384,7 +2392,7 @@ __global__ void __launch_bounds__(kRoundThreads, 1) k_rounds(Dev D) {
     cluster_barrier();
     bfs_body<kRoundWarps, 32>(D, R, sm.bfs);
     cluster_barrier();
-    shared_body<kRoundWarps, kBlockFacesSmall>(D, R);
+    shared_body<kRoundWarps, kBlockFacesSmall, 1>(D, R);
     cluster_barrier();
     write_body<kRoundWarps>(D, R, sm.write);
     cluster_barrier();
