@@ -409,13 +409,13 @@ __device__ __forceinline__ uint32_t mix32(uint32_t h) {
 // candidate has priority 1, or with the learned scheduler the priority its
 // network gave it this round (1..1023).
 __device__ __forceinline__ unsigned long long make_key(const Dev& D, const RoundArgs& R, uint32_t p) {
-  const unsigned long long prio = D.bigflag[p] == 2 ? 0u : (D.prio ? D.prio[p] : 1u);
+  const unsigned long long prio = D.bigflag[p] == 2 ? 0u : (R.flags & kLearnedRound ? D.prio[p] : 1u);
   return R.stamp | (prio << 32) | mix32(p ^ (R.round * 0x9E3779B9u));
 }
 
 // The key of a vote winner that is not on the huge path.
 __device__ __forceinline__ unsigned long long start_key(const Dev& D, const RoundArgs& R, uint32_t p) {
-  const unsigned long long prio = D.prio ? D.prio[p] : 1u;
+  const unsigned long long prio = R.flags & kLearnedRound ? D.prio[p] : 1u;
   return R.stamp | (prio << 32) | mix32(p ^ (R.round * 0x9E3779B9u));
 }
 
@@ -439,6 +439,15 @@ __device__ __forceinline__ uint32_t chunk_for(uint32_t items) {
 // (k_write holds one new tet per lane in registers until the warp has read
 // the whole cavity).
 constexpr uint32_t kInPlaceFaces = 32;
+
+// First item of this warp in a loop over items, 32 at a time with the grid's
+// threads as stride.  Large rounds keep a block's warps on neighbouring items;
+// small rounds (kSpread) deal the warps out over the blocks, so that a round of
+// a few hundred points has one warp per SM scheduler instead of one busy SM.
+template <bool kSpread>
+__device__ __forceinline__ uint32_t warp_first() {
+  return kSpread ? ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32u : blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
+}
 
 // Appends `pred` lanes to a list through one atomic per warp.
 __device__ __forceinline__ uint32_t warp_append(uint32_t* ctr, bool pred) {
@@ -1007,11 +1016,11 @@ struct CandSmem {
 // With kLearned, the fused network scores the warp's winners and sets their
 // claim priority; the start list is bucketed by that priority (better first)
 // instead of by the claim hash.
-template <bool kLearned, uint32_t kWarps>
+template <bool kLearned, uint32_t kWarps, bool kSpread>
 __device__ __forceinline__ void cands_body(const Dev& D, const RoundArgs& R, const mlp::Smem* net, CandSmem<kWarps>* sm) {
   const uint32_t lane = threadIdx.x & 31u;
-  for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < R.n_active; i0 += gridDim.x * blockDim.x) {
-    const uint32_t i = i0 + threadIdx.x;
+  for (uint32_t i0 = warp_first<kSpread>(); i0 < R.n_active; i0 += gridDim.x * blockDim.x) {
+    const uint32_t i = i0 + lane;
     bool start = false;
     uint32_t p = 0, t = 0;
     unsigned long long vote = 0;
@@ -1021,7 +1030,9 @@ __device__ __forceinline__ void cands_body(const Dev& D, const RoundArgs& R, con
       t = D.loc[p];
       if (!(tier & kDup) && t < D.cap) vote = D.T[t].vote;
       if (!(tier & kDup) && t < D.cap && uint32_t(vote) == ~p) {
-        if (D.losses && D.losses[p] < 255u) D.losses[p] += 1u;
+        // (the learned scheduler needs the count in the rounds it may serve; a
+        // training log records it in all)
+        if (D.losses && (D.log_x || R.n_active <= D.learned_points) && D.losses[p] < 255u) D.losses[p] += 1u;
         if (tier == 2) {
           uint32_t b = atomicAdd(&R.ctr->huge_used, 1u);
           if (b < HUGE_SLOTS) D.bigcand[b] = p;
@@ -1055,7 +1066,6 @@ __device__ __forceinline__ void cands_body(const Dev& D, const RoundArgs& R, con
         __syncwarp();
       }
     } else {
-      if (start && D.prio) D.prio[p] = 1;
       b = start ? (mix32(p ^ (R.round * 0x9E3779B9u)) >> (32 - kOrderBits)) : 0u;
     }
     if (start && D.prefilter) pre_claim(D, t, start_key(D, R, p));
@@ -1077,23 +1087,20 @@ __device__ __forceinline__ void cands_body(const Dev& D, const RoundArgs& R, con
 
 __global__ void k_cands(Dev D) {
   const RoundArgs R = load_round(D);
-  if (!R.live) return;
-  cands_body<false, 1>(D, R, nullptr, nullptr);
+  if (!R.live || (R.flags & kLearnedRound)) return;
+  cands_body<false, 1, false>(D, R, nullptr, nullptr);
 }
 
-// The learned scheduler's candidate kernel (256-thread blocks).
+// The learned scheduler's candidate kernel (256-thread blocks), in the rounds it
+// serves; the others run k_cands, which keeps more than twice the blocks resident.
 __global__ void __launch_bounds__(256) k_cands_learned(Dev D) {
   const RoundArgs R = load_round(D);
-  if (!R.live) return;
+  if (!R.live || !(R.flags & kLearnedRound) || blockIdx.x * blockDim.x >= R.n_active) return;
   __shared__ __align__(16) mlp::Smem net;
   __shared__ __align__(16) CandSmem<8> sm;
-  if (!(R.flags & kLearnedRound)) {
-    cands_body<false, 1>(D, R, nullptr, nullptr);
-    return;
-  }
   mlp::load_image(net, D.mlp);
   __syncthreads();
-  cands_body<true, 8>(D, R, &net, &sm);
+  cands_body<true, 8, false>(D, R, &net, &sm);
 }
 
 // Cavity growth by groups of kBfsLanes lanes, kWarpGroups at a time per warp:
@@ -2167,12 +2174,13 @@ __device__ __forceinline__ NextStratum next_stratum(const Dev& D, int32_t next_l
 // stride earlier and later on the curve (a point of an earlier stratum: its tet once inserted,
 // else the tet that contains it -- as of this round or, while this very pass
 // relocates it, of the last one; a retired tet forwards to a live one).
+template <bool kSpread>
 __device__ __forceinline__ void relocate_body(const Dev& D, const RoundArgs& R, const NextStratum& ns) {
   uint32_t steps = 0;
   if (ns.total) {
     const uint32_t level = uint32_t(ns.level), nc = D.nc;
     const uint64_t* lvl_off = D.lvl_off + size_t(level) * (nc + 1);
-    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < ns.total; idx += gridDim.x * blockDim.x) {
+    for (uint32_t idx = warp_first<kSpread>() + (threadIdx.x & 31u); idx < ns.total; idx += gridDim.x * blockDim.x) {
       uint32_t lo = 0, hi = nc;
       while (hi - lo > 1) {
         uint32_t mid = (lo + hi) >> 1;
@@ -2215,8 +2223,8 @@ __device__ __forceinline__ void relocate_body(const Dev& D, const RoundArgs& R, 
       D.loc[p] = locate(D, t, p, pq, steps);
     }
   }
-  for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < R.n_active; i0 += gridDim.x * blockDim.x) {
-    uint32_t i = i0 + threadIdx.x;
+  for (uint32_t i0 = warp_first<kSpread>(); i0 < R.n_active; i0 += gridDim.x * blockDim.x) {
+    const uint32_t i = i0 + (threadIdx.x & 31u);
     bool keep = false;
     uint32_t p = 0;
     if (i < R.n_active && (D.bigflag[R.active[i]] & kDup)) {
@@ -2331,7 +2339,7 @@ __global__ void __launch_bounds__(512, WTET_RELOC_MINB) k_relocate(Dev D) {
   if (!R.live) return;
   const NextStratum ns = next_stratum(D, __ldcg(&D.st->next_level), __ldcg(&D.st->stratum_size),
                                       __ldcg(&D.st->overlap_shift), R.n_active, __ldcg(&R.ctr->n_inserted));
-  relocate_body(D, R, ns);
+  relocate_body<false>(D, R, ns);
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0 && atomicAdd(&R.ctr->ticket, 1u) == gridDim.x - 1) {
@@ -2387,8 +2395,8 @@ __global__ void __launch_bounds__(kRoundThreads, 1) k_rounds(Dev D) {
     const RoundArgs R = round_args(D, reinterpret_cast<const uint4*>(&S)[0], reinterpret_cast<const uint4*>(&S)[1]);
     if (!R.live || !(R.flags & kSmallRound)) break;  // the same in every block
     ran = true;
-    if (kLearned && (R.flags & kLearnedRound)) cands_body<kLearned, kRoundWarps>(D, R, net, &sm.cand);
-    else cands_body<false, 1>(D, R, nullptr, nullptr);
+    if (kLearned && (R.flags & kLearnedRound)) cands_body<kLearned, kRoundWarps, true>(D, R, net, &sm.cand);
+    else cands_body<false, 1, true>(D, R, nullptr, nullptr);
     cluster_barrier();
     bfs_body<kRoundWarps, 32>(D, R, sm.bfs);
     cluster_barrier();
@@ -2398,7 +2406,7 @@ __global__ void __launch_bounds__(kRoundThreads, 1) k_rounds(Dev D) {
     cluster_barrier();
     const NextStratum ns =
         next_stratum(D, S.next_level, S.stratum_size, S.overlap_shift, R.n_active, __ldcg(&R.ctr->n_inserted));
-    relocate_body(D, R, ns);
+    relocate_body<true>(D, R, ns);
     // The error flags are read once for all blocks, so that all of them take
     // the same decision (a later flag is seen a round later).
     if (blockIdx.x == 0 && threadIdx.x == 0) R.ctr->err = *reinterpret_cast<volatile uint32_t*>(&D.tot->err);
@@ -3178,10 +3186,10 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
   const uint32_t g_cand = wave(k_cands, TB), g_candl = vmode == 1 ? wave(k_cands_learned, 256) : 0u;
   const uint32_t g_log = wave(k_log_features, TB), g_bfs = wave(k_bfs, 128), g_sh = wave(k_shared, 128);
   const uint32_t g_wr = wave(k_write, 128), g_rel = wave(k_relocate, TB);
-  const uint64_t kernels_per_round = 5 + (vmode == 2 ? 1 : 0);
+  const uint64_t kernels_per_round = 5 + (vmode ? 1 : 0);
   auto enqueue_round = [&]() {
     if (vmode == 1) k_cands_learned<<<g_candl, 256, 0, s>>>(D);
-    else k_cands<<<g_cand, TB, 0, s>>>(D);
+    k_cands<<<g_cand, TB, 0, s>>>(D);
     if (vmode == 2) k_log_features<<<g_log, TB, 0, s>>>(D);
     k_bfs<<<g_bfs, 128, 0, s>>>(D);
     k_shared<<<g_sh, 128, 0, s>>>(D);
@@ -3335,7 +3343,14 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
 
 // ------------------------------------------------------- quality check ----
 
-__global__ void k_check_quality(const float4* pts, uint32_t n, const uint4* tets, const uint4* adj, uint64_t m,
+// SoS keys are the input indices themselves.
+__device__ __noinline__ int quality_exact(float4 X, float4 Y, float4 Z, float4 e, uint4 t, uint32_t vb, uint32_t* err) {
+  const double A[3] = {X.x, Y.x, Z.x}, B[3] = {X.y, Y.y, Z.y}, C[3] = {X.z, Y.z, Z.z}, Dd[3] = {X.w, Y.w, Z.w};
+  const double E[3] = {e.x, e.y, e.z};
+  const int s = ex::insphere(A, B, C, Dd, E, err);
+  return s != 0 ? s : ex::orient4d_sos_degenerate(A, B, C, Dd, E, t.x, t.y, t.z, t.w, vb, err);
+}
+__global__ void __launch_bounds__(128, 8) k_check_quality(const float4* pts, uint32_t n, const uint4* tets, const uint4* adj, uint64_t m,
                                 unsigned long long* out, uint32_t* err) {
   unsigned long long viol = 0, interior = 0;
   for (uint64_t ti = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; ti < m; ti += uint64_t(gridDim.x) * blockDim.x) {
@@ -3356,17 +3371,11 @@ __global__ void k_check_quality(const float4* pts, uint32_t n, const uint4* tets
       uint4 o = tets[oti];
       if (o.x >= n || o.y >= n || o.z >= n || o.w >= n) continue;
       uint32_t vb = comp(o, of);
-      double P[5][3];
-      load_pt(pts, t.x, P[0]);
-      load_pt(pts, t.y, P[1]);
-      load_pt(pts, t.z, P[2]);
-      load_pt(pts, t.w, P[3]);
-      load_pt(pts, vb, P[4]);
-      int s = ex::insphere(P[0], P[1], P[2], P[3], P[4], err);
-      if (s == 0) {
-        // SoS keys are the input indices themselves.
-        s = ex::orient4d_sos_degenerate(P[0], P[1], P[2], P[3], P[4], t.x, t.y, t.z, t.w, vb, err);
-      }
+      const float4 p0 = pts[t.x], p1 = pts[t.y], p2 = pts[t.z], p3 = pts[t.w], e = pts[vb];
+      const float4 X = make_float4(p0.x, p1.x, p2.x, p3.x), Y = make_float4(p0.y, p1.y, p2.y, p3.y);
+      const float4 Z = make_float4(p0.z, p1.z, p2.z, p3.z);
+      int s = ex::insphere_mid(X, Y, Z, e);
+      if (s != 1 && s != -1) s = quality_exact(X, Y, Z, e, t, vb, err);
       if (s < 0) ++viol;
     }
   }

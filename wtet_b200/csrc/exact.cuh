@@ -799,6 +799,26 @@ __device__ __noinline__ int insphere_mid(float4 X, float4 Y, float4 Z, float4 e)
   return bxs && bys && bzs ? 2 : 0;
 }
 
+// Sign of Shewchuk orient3d(a,b,c,d) when certain from f64 arithmetic with the
+// same kind of bound, or 0: each 2x2 minor's permanent is at most 2 r_i r_j, so
+// the permanent is at most 6 r_a r_b r_c.
+__device__ __forceinline__ int orient3d_mid(const float4& a, const float4& b, const float4& c, const float4& d) {
+  const float ra = fmaxf(fmaxf(fabsf(a.x - d.x), fabsf(a.y - d.y)), fabsf(a.z - d.z));
+  const float rb = fmaxf(fmaxf(fabsf(b.x - d.x), fabsf(b.y - d.y)), fabsf(b.z - d.z));
+  const float rc = fmaxf(fmaxf(fabsf(c.x - d.x), fabsf(c.y - d.y)), fabsf(c.z - d.z));
+  const double bound = dmul(dmul(kO3dBoundA * 6.0 * (1.0 + 0x1p-18), double(ra)), dmul(double(rb), double(rc)));
+  const double dx = d.x, dy = d.y, dz = d.z;
+  const double adx = dsub(a.x, dx), ady = dsub(a.y, dy), adz = dsub(a.z, dz);
+  const double bdx = dsub(b.x, dx), bdy = dsub(b.y, dy), bdz = dsub(b.z, dz);
+  const double cdx = dsub(c.x, dx), cdy = dsub(c.y, dy), cdz = dsub(c.z, dz);
+  const double det = dadd(dadd(dmul(adz, dsub(dmul(bdx, cdy), dmul(cdx, bdy))),
+                               dmul(bdz, dsub(dmul(cdx, ady), dmul(adx, cdy)))),
+                          dmul(cdz, dsub(dmul(adx, bdy), dmul(bdx, ady))));
+  if (det > bound) return 1;
+  if (-det > bound) return -1;
+  return 0;
+}
+
 // ---- SoS cascade pieces (src/predicates.rs) ----
 
 // Plain double orient2d on coordinates (u, v): src/predicates.rs:73-75.

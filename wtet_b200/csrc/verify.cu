@@ -42,11 +42,20 @@ __device__ __forceinline__ uint32_t cmp4(const uint4& v, int i) {
   return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w));
 }
 
-__device__ __forceinline__ void ld_pt(const float4* pts, uint32_t v, double* o) {
-  const float4 q = pts[v];
-  o[0] = q.x;
-  o[1] = q.y;
-  o[2] = q.z;
+// The exact tests out of line: the f64 stages with a bounded permanent
+// (orient3d_mid, insphere_mid) answer nearly all of them in the kernel's own
+// registers.  Inlined, the chain needed 168 registers and a 4.6 KB frame per
+// thread, which left 12 warps per SM for a pass of dependent gathers.
+__device__ __noinline__ int orient_exact(float4 a, float4 b, float4 c, float4 d, uint4 t, uint32_t* err) {
+  const double A[3] = {a.x, a.y, a.z}, B[3] = {b.x, b.y, b.z}, C[3] = {c.x, c.y, c.z}, Dd[3] = {d.x, d.y, d.z};
+  const int o = ex::orient3d(A, B, C, Dd, err);
+  return o != 0 ? (o < 0 ? 1 : -1) : ex::orient3d_sos_degenerate(A, B, C, Dd, t.x, t.y, t.z, t.w);
+}
+__device__ __noinline__ int sphere_exact(float4 X, float4 Y, float4 Z, float4 e, uint4 t, uint32_t ve, uint32_t* err) {
+  const double A[3] = {X.x, Y.x, Z.x}, B[3] = {X.y, Y.y, Z.y}, C[3] = {X.z, Y.z, Z.z}, Dd[3] = {X.w, Y.w, Z.w};
+  const double E[3] = {e.x, e.y, e.z};
+  const int s = ex::insphere(A, B, C, Dd, E, err);
+  return s != 0 ? s : ex::orient4d_sos_degenerate(A, B, C, Dd, E, t.x, t.y, t.z, t.w, ve, err);
 }
 
 // Sorted copy of a row (5-comparator network).
@@ -88,7 +97,7 @@ __global__ void k_super_points(float4* pts, uint32_t n) {
   if (k < 4) pts[n + k] = make_float4(S[k][0], S[k][1], S[k][2], 0.f);
 }
 
-__global__ void __launch_bounds__(128) k_verify(const float4* pts, uint32_t n, const uint4* tets, const uint4* adj,
+__global__ void __launch_bounds__(128, 8) k_verify(const float4* pts, uint32_t n, const uint4* tets, const uint4* adj,
                                                 uint64_t m, VerifyCounts* out) {
   const uint32_t inf = n + 4;
   unsigned long long finite = 0, faces = 0, viol = 0, mis = 0, broken = 0, hull = 0, bad = 0;
@@ -100,15 +109,10 @@ __global__ void __launch_bounds__(128) k_verify(const float4* pts, uint32_t n, c
     }
     if (has(t, inf)) continue;
     ++finite;
-    double P[4][3];
-    ld_pt(pts, t.x, P[0]);
-    ld_pt(pts, t.y, P[1]);
-    ld_pt(pts, t.z, P[2]);
-    ld_pt(pts, t.w, P[3]);
+    const float4 p0 = pts[t.x], p1 = pts[t.y], p2 = pts[t.z], p3 = pts[t.w];
     // orient3d_sos == +1 (Shewchuk determinant < 0, src/phase2.rs:404-410)
-    int o = ex::orient3d(P[0], P[1], P[2], P[3], &out->err);
-    o = o != 0 ? (o < 0 ? 1 : -1)
-               : ex::orient3d_sos_degenerate(P[0], P[1], P[2], P[3], t.x, t.y, t.z, t.w);
+    int o = -ex::orient3d_mid(p0, p1, p2, p3);
+    if (o == 0) o = orient_exact(p0, p1, p2, p3, t, &out->err);
     if (o != 1) ++mis;
     const uint4 a = adj[ti];
     const uint4 ts = sorted4(t);
@@ -149,11 +153,10 @@ __global__ void __launch_bounds__(128) k_verify(const float4* pts, uint32_t n, c
       }
       if (ti > oti) continue;  // each face once
       ++faces;
-      double E[3];
-      ld_pt(pts, xb, E);
-      int s = ex::insphere(P[0], P[1], P[2], P[3], E, &out->err);
-      if (s == 0)
-        s = ex::orient4d_sos_degenerate(P[0], P[1], P[2], P[3], E, t.x, t.y, t.z, t.w, xb, &out->err);
+      const float4 X = make_float4(p0.x, p1.x, p2.x, p3.x), Y = make_float4(p0.y, p1.y, p2.y, p3.y);
+      const float4 Z = make_float4(p0.z, p1.z, p2.z, p3.z), e = pts[xb];
+      int s = ex::insphere_mid(X, Y, Z, e);
+      if (s != 1 && s != -1) s = sphere_exact(X, Y, Z, e, t, xb, &out->err);
       if (s < 0) ++viol;
     }
   }
