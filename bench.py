@@ -215,8 +215,8 @@ def bench_config(workload: str, vote: str, world: int):
         "l2": "inputs larger than the 126 MB L2: tets, adjacency and claim arrays of several GB",
     }
     if workload == "batched":
-        cfg["batching"] = "all clouds in one job: insertion rounds over every cloud replayed from CUDA graphs " \
-                          "(graph nodes are the grid-wide barriers; no persistent kernel)"
+        cfg["batching"] = "all clouds in one job: insertion rounds over every cloud, small rounds inside one cluster " \
+                          "kernel, large ones as five launches each"
     return cfg
 
 
@@ -366,8 +366,8 @@ def run_gpu(args):
             "frac": round(achieved / hbm, 5),
             "traffic": TRAFFIC.get(args.workload),
             "traffic_source": TRAFFIC_SOURCE if args.workload in TRAFFIC else None,
-            "basis": "whole triangulation per step (thousands of launches of the round kernels replayed from "
-                     "CUDA graphs, so no single launch is the unit): 12 B/point read + 32 B/tet written over its "
+            "basis": "whole triangulation per step (hundreds of launches of the round kernels in one "
+                     "stream, so no single launch is the unit): 12 B/point read + 32 B/tet written over its "
                      f"device time; peak = {peak_kind} copy bandwidth; traffic = DRAM bytes read + written by all "
                      "launches of one triangulation (ncu)",
         },
@@ -392,17 +392,11 @@ def run_gpu(args):
         dist.destroy_process_group()
 
 
-# DRAM bytes (read + write) of one whole triangulation of the 8M mixture,
-# estimated with ncu: for each round kernel, the DRAM bytes per microsecond of
-# one launch in the most expensive round of the 1M mixture (one kernel, one
-# launch per capture) times that kernel's total time in the time-only launch
-# list of one 8M triangulation.  It describes the kernels it was measured on
-# and must be captured again when they change.
-TRAFFIC: dict = {"mixture8M": 366.7e9}
-TRAFFIC_SOURCE = ("estimate: sum over k_bfs, k_shared, k_write, k_cands, k_relocate, k_activate of "
-                  "(DRAM bytes per us of one bulk-round launch on the 1M mixture, ncu) x (the kernel's total time "
-                  "in the 8M launch list, ncu); early rounds fit in L2, so this over-counts them; two captures of "
-                  "different bulk rounds gave 312 and 367 GB")
+# DRAM bytes (read + write) of one whole triangulation, from ncu.  A figure
+# describes the kernels it was captured on; none has been captured on the
+# current ones.
+TRAFFIC: dict = {}
+TRAFFIC_SOURCE = "ncu"
 
 WORKLOADS = {
     "mixture8M": "8,000,000 points: 60% uniform [0,1]^3, 30% Gaussian ball (0.5, sigma 0.1), "
@@ -538,8 +532,8 @@ def variants(wt, args, golden):
     out["batched"] = {"workload": "batched", "clouds": len(clouds), "points": n, "all_same_as_oracle": same_b,
                       "batched_mpts": round(n / (bm * 1e3), 3), "batched_device_ms": round(bm, 1),
                       "looped_plain_mpts": round(n / (loop_ms * 1e3), 3), "looped_device_ms": round(loop_ms, 1),
-                      "how": "one job over all clouds, insertion rounds replayed from CUDA graphs (no persistent "
-                             "kernel: consecutive graph nodes are the grid-wide barriers)"}
+                      "how": "one job over all clouds; small rounds inside one cluster kernel, large ones as five "
+                             "launches each"}
     return out
 
 

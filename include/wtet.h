@@ -65,13 +65,13 @@ typedef struct wtet_config {
    * for the job's size bucket (wtet_autotune_set_table), else the default.
    * None of them changes the triangulation. */
   uint32_t block_size;             /* threads per block of the per-point kernels: 128, 256 (default), 512 */
-  uint32_t rounds_per_graph;       /* insertion rounds replayed per CUDA-graph launch (default 8, max 64) */
+  uint32_t rounds_per_graph;       /* insertion rounds enqueued per host check (default 8, max 64) */
   uint32_t overlap_shift;          /* next stratum starts when the current one has thinned to
                                       1/2^overlap_shift of its size (default 3) */
   uint32_t candidate_filter;       /* neighbourhood pre-claim before cavity growth: 1 = on (default),
                                       2 = off */
   uint32_t pool_factor;            /* cavity-pool entries per point (default 24, 4..64) */
-  uint32_t learned_gate;           /* learned scheduler: rounds whose graph may see at most
+  uint32_t learned_gate;           /* learned scheduler: rounds that may see at most
                                       learned_gate x 1024 uninserted points take the network's claim
                                       priority, larger rounds the hashed one; 0 = default (2048) */
   uint32_t initial_capacity;       /* initial tet slots per point, in eighths; 0 = default (58, i.e. 7.25
@@ -93,7 +93,7 @@ typedef struct wtet_stats {
   uint64_t num_tets;          /* output tets (incl. super and infinity tets) */
   uint64_t walk_steps;        /* point-location steps */
   uint64_t num_failed;        /* points left out as exact duplicates */
-  uint64_t kernel_launches;   /* CUDA kernels executed by the call (graph nodes included) */
+  uint64_t kernel_launches;   /* CUDA kernels launched by the call */
   double device_ms;           /* device time of the call, CUDA events */
   uint64_t vote_winners;      /* points that won their tet's vote (insertion attempts) */
   uint64_t capacity_grows;    /* times the tet arrays grew during the run */

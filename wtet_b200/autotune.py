@@ -4,7 +4,7 @@ are left at 0 (``Config`` defaults).
 
 Knobs (none changes the triangulation, which the tuner verifies):
   block_size        threads per block of the per-point kernels (128/256/512)
-  rounds_per_graph  insertion rounds per CUDA-graph launch (4..32)
+  rounds_per_graph  insertion rounds enqueued per host check (4..32)
   overlap_shift     when the next stratum starts (the current one thinned to 1/2^k)
   candidate_filter  neighbourhood pre-claim before cavity growth (1 on, 2 off)
   pool_factor       cavity-pool entries per point (the round's candidate queue)
@@ -152,7 +152,7 @@ def tune_bucket(clouds, repeats: int = 3, verbose: bool = True) -> dict:
     """Coordinate descent over KNOBS from the defaults; every choice must give
     the same tet set as the defaults."""
     best = dict(DEFAULTS)
-    _measure(clouds, best, 1)  # warm-up (allocations, graph capture)
+    _measure(clouds, best, 1)  # warm-up (allocations)
     best_ms, ref = _measure(clouds, best, repeats)
     for k in KNOBS:
         for v in CHOICES[k]:

@@ -12,26 +12,20 @@
 // equivalent to some sequential order.  The result is therefore the unique
 // SoS Delaunay triangulation, with no flip failures and nothing left to repair.
 //
-// Round structure (one insertion round over all clouds of a job; 9 kernels
-// replayed from a CUDA graph):
-//   k_activate    locate the new stratum's points (walk from the curve
-//                 predecessor's tet)
-//   (votes)       each uninserted point votes for its tet (64-bit atomicMax
-//                 of score | ~point, src/shaders/vote.wgsl semantics) when it
-//                 is located (k_activate) or relocated (k_relocate); a tet's
-//                 vote stays valid until the tet is retired
-//   k_cands       the winner of each tet becomes a candidate and pre-claims
-//                 its tet's neighbourhood with its claim key (with the
-//                 learned scheduler, k_cands_learned: the fused BF16 MLP sets
-//                 the winners' claim priority in the rounds of the first
-//                 strata)
+// Round structure (one insertion round over all clouds of a job; a large round
+// is five kernels, rounds of a few thousand points run the same five passes
+// inside k_rounds):
+//   k_cands       the winner of each tet's vote (64-bit atomicMax of score |
+//                 ~point, src/shaders/vote.wgsl semantics) becomes a candidate
+//                 and pre-claims its tet's neighbourhood with its claim key
+//                 (with the learned scheduler, k_cands_learned: the fused BF16
+//                 MLP sets the winners' claim priority in the rounds it serves)
 //   k_bfs         candidates whose pre-claims all hold grow their cavities by
-//                 breadth-first search with exact insphere (16 lanes per
-//                 candidate), claiming cavity tets by 64-bit atomicMin of a
-//                 round-stamped key; k_expand_big grows the huge ones, one
-//                 block each
-//   k_resolve     a candidate wins when it holds the minimum claim on all its
-//                 cavity tets
+//                 breadth-first search with exact insphere (16 or 32 lanes per
+//                 candidate, a block for a huge one), claiming cavity tets by
+//                 64-bit atomicMin of a round-stamped key and listing the
+//                 boundary faces; a completed cavity that no better claim
+//                 displaced has won
 //   k_shared      two winners whose cavities share a face both stay only if
 //                 that face remains Delaunay (exact insphere); else the worse
 //                 one steps back -- this exact test replaces a blanket
@@ -41,17 +35,21 @@
 //                 (rotation around boundary edges for the very largest
 //                 cavities), cavity retired
 //   k_relocate    points whose tet was retired walk (exact orient3d) from a
-//                 tet of the inserting point; the rest keep their tet; the
-//                 uninserted list is compacted with warp-aggregated appends;
-//                 unused recycled slots carry over
-//   k_end         list swap, stop conditions, and the next round's start:
-//                 the next stratum once the current one has thinned
+//                 tet of the inserting point and vote for the tet they reach
+//                 (a tet's vote stays valid until the tet is retired); the next
+//                 stratum, when due, is located by walks from the neighbours on
+//                 the curve; the uninserted list is compacted with
+//                 warp-aggregated appends; unused recycled slots carry over;
+//                 the last block ends the round (list swap, stop conditions,
+//                 the next round's start)
+// What bounds a round is latency: every pass is a chain of dependent gathers
+// (issue slots ~30% busy, DRAM ~20% of its rate in the largest rounds), so the
+// design counts trips, keeps many short chains in flight and avoids launches.
 // The cavity search, shared-face test and tet writing take their work items
 // dynamically (atomic cursors): cavity sizes vary by orders of magnitude.
 // Strata: points are bucketed per cloud along a Morton (or Hilbert) curve
 // (counting sort) and inserted in the reference's stratified stride order
-// (src/gpu/mod.rs:533-600), each new stratum located by a walk from its
-// predecessor on the curve.
+// (src/gpu/mod.rs:533-600).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -163,7 +161,7 @@ constexpr uint32_t kSmallRound = 1u;
 constexpr uint32_t kLearnedRound = 2u;
 
 // Round-loop state kept on the device, so that a round is a fixed kernel
-// sequence that can be replayed from a CUDA graph without host round trips.
+// sequence that needs no host round trip.
 struct alignas(16) State {
   // read by every round kernel: the first 32 bytes, two vector loads
   uint32_t round;         // rounds executed
@@ -2967,8 +2965,8 @@ void launch_small_rounds(const Dev& D, bool learned, cudaStream_t s) {
 JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t capacity) {
   reserve_stack_once();
   Workspace& W = ws();
-  // The legacy default stream cannot be captured into a graph; the workspace's
-  // own (blocking) stream orders with it implicitly.
+  // The workspace's own (blocking) stream orders with the legacy default stream
+  // implicitly.
   cudaStream_t s = job.stream ? job.stream : W.stream;
   const uint32_t nc = uint32_t(job.offsets.size() - 1);
   const uint64_t n = job.offsets.back();
@@ -3081,7 +3079,7 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
     ck(cudaMemsetAsync(W.log_pslot.p, 0xFF, nv * 4, s), "memset");
   }
   if (vmode == 1) W.prio.reserve(nv, "claim priorities");
-  // Rounds whose graph may see at most this many uninserted points use the
+  // Rounds that may see at most this many uninserted points use the
   // learned scheduler (its training log records the same rounds).
   const char* tr = getenv("WTET_TRACE");
   const int trace = tr ? atoi(tr) : 0;
@@ -3169,7 +3167,7 @@ JobResult run_job(const Job& job, uint32_t* d_out_t, uint32_t* d_out_a, uint64_t
       uint64_t(std::max<uint32_t>(job.cfg.max_insert_iterations, 1u)) * (maxtop + 1), 65000ull));
   const uint32_t TB = (cfg.block_size == 128 || cfg.block_size == 512) ? cfg.block_size : 256u;
 
-  // ---- the round loop, driven from device state and replayed from a graph ----
+  // ---- the round loop, driven from device state ----
   std::vector<uint32_t> lt(maxtop + 1);
   for (uint32_t L = 0; L <= maxtop; ++L) lt[L] = lvl_total[L];
   ck(cudaMemcpyAsync(W.lvl_total.p, lt.data(), (maxtop + 1) * 4, cudaMemcpyHostToDevice, s), "h2d");
